@@ -416,14 +416,16 @@ void Engine::build_blocks(const std::vector<const HostBlock*>& blocks, const std
 		if (need_ls) f32_.lsw.upload(tof(lsw));
 		f32_.vol.upload(tof(vol));
 	}
-	// reductions: chunks of 4096 cells, never straddling a block
-	chunk_ = 4096;
+	// reductions: chunks of TAIL_CHUNK cells, never straddling a block
 	max_chunks_ = 1;
-	for (int b = 0; b < nb_; b++) max_chunks_ = std::max(max_chunks_, (roff_[b + 1] - roff_[b] + chunk_ - 1) / chunk_);
-	partial_.alloc((size_t)nb_ * max_chunks_ * 5);
+	for (int b = 0; b < nb_; b++)
+		max_chunks_ = std::max(max_chunks_, (roff_[b + 1] - roff_[b] + TAIL_CHUNK - 1) / TAIL_CHUNK);
+	partial_.alloc((size_t)TAIL_SLOTS * nb_ * max_chunks_ * 5);
 	hist_d_.alloc(opt_.hist_capacity * (size_t)nb_ * 10);
 	fd_hist_.alloc((size_t)nb_ * 10);
-	wall_terms_.alloc(5 * std::max<size_t>(1, wall_face_.n));
+	wall_terms_.alloc(TAIL_SLOTS * 5 * std::max<size_t>(1, wall_face_.n));
+	pend_d_.alloc(2);
+	cuda_ok(cudaMemset(pend_d_.p, 0, 2 * sizeof(int)), "memset");
 	iter_d_.alloc(1);
 	bad_d_.alloc(1);
 	zero_d_.alloc(1);
@@ -492,7 +494,7 @@ void Engine::count_device_bytes() {
 	                &wall_face_, &roff_d_, &xsend_, &xrecv_})
 		bytes += b->n * sizeof(int);
 	for (auto* b : {&S_, &nhat_, &area_, &rl_, &rr_, &fc_, &vol64_, &lsw64_, &W0_, &srad_, &grad_, &lim_, &partial_,
-	                &hist_d_})
+	                &hist_d_, &wall_terms_})
 		bytes += b->n * sizeof(double);
 	for (auto* b : {&f64_.P0, &f64_.P1, &f64_.FS, &f64_.Rc, &f64_.Rd, &f64_.dt, &f64_.sgeo, &f64_.sS, &f64_.srv,
 	                &f64_.lsw, &f64_.vol})
@@ -653,44 +655,49 @@ void Engine::halo() {
 	started_ = true;
 }
 
-static ReduceArgs make_reduce(int NR, int NA, int nb, const int* roff, int chunk, int max_chunks, double* partial,
-                              const int* woff, const int* wface, int n_wall, double* wall_terms, const int* flr,
-                              const double* S, const double* fc, double denom, double* hist, const int* d_iter,
-                              int* d_bad) {
+ReduceArgs Engine::reduce_args(double* hist, int* d_iter, bool with_halo) const {
 	ReduceArgs a{};
-	a.NR = NR;
-	a.NA = NA;
-	a.nblocks = nb;
-	a.roff = roff;
-	a.chunk = chunk;
-	a.max_chunks = max_chunks;
-	a.partial = partial;
-	a.wall_off = woff;
-	a.wall_face = wface;
-	a.n_wall = n_wall;
-	a.wall_terms = wall_terms;
-	a.face_lr = flr;
-	a.S = S;
-	a.fc = fc;
-	a.denom = denom;
-	a.wall_denom = nullptr;
+	a.NR = NR_;
+	a.NA = NA_;
+	a.nblocks = nb_;
+	a.roff = roff_d_.p;
+	a.max_chunks = max_chunks_;
+	a.partial = partial_.p;
+	a.wall_off = wall_off_.p;
+	a.wall_face = wall_face_.p;
+	a.n_wall = (int)wall_face_.n;
+	a.wall_terms = wall_terms_.p;
+	a.face_lr = face_lr_.p;
+	a.S = S_.p;
+	a.fc = fc_.p;
+	a.denom = denom_;
+	a.wall_denom = wall_denom_d_.p;
+	a.n_halo = with_halo ? (int)halo_dst_.n : 0;
+	a.halo_dst = halo_dst_.p;
+	a.halo_src = halo_src_.p;
 	a.hist = hist;
-	a.stride = nb * 10;
+	a.stride = nb_ * 10;
 	a.d_iter = d_iter;
-	a.d_bad = d_bad;
+	a.d_bad = bad_d_.p;
+	a.pend = pend_d_.p;
+	a.ticket = reinterpret_cast<unsigned*>(pend_d_.p + 1);
 	return a;
+}
+
+// the per-block sums of the iterations whose tails have run since the last call
+void Engine::flush_tail() {
+	launch_tail_sums(reduce_args(hist_d_.p, iter_d_.p, false), pend_, true, st_);
+	pend_ = 0;
 }
 
 void Engine::flow_data(std::vector<double>& out) {
 	require_not_delta("flow_data");
-	ReduceArgs a = make_reduce(NR_, NA_, nb_, roff_d_.p, chunk_, max_chunks_, partial_.p, wall_off_.p, wall_face_.p,
-	                           (int)wall_face_.n, wall_terms_.p, face_lr_.p, S_.p, fc_.p, denom_, fd_hist_.p, zero_d_.p,
-	                           bad_d_.p);
-	a.wall_denom = wall_denom_d_.p;
+	const ReduceArgs a = reduce_args(fd_hist_.p, zero_d_.p, false);
 	if (opt_.precision == PREC_FP64)
-		launch_reduce<double>(a, f64_.Rc.p, f64_.Rd.p, cur_ ? f64_.P1.p : f64_.P0.p, st_);
+		launch_tail<double>(a, f64_.Rc.p, f64_.Rd.p, cur_ ? f64_.P1.p : f64_.P0.p, nullptr, st_);
 	else
-		launch_reduce<float>(a, f32_.Rc.p, f32_.Rd.p, cur_ ? f32_.P1.p : f32_.P0.p, st_);
+		launch_tail<float>(a, f32_.Rc.p, f32_.Rd.p, cur_ ? f32_.P1.p : f32_.P0.p, nullptr, st_);
+	launch_tail_sums(a, 1, false, st_);
 	check("flow_data");
 	out.resize((size_t)nb_ * 10);
 	cuda_ok(cudaMemcpyAsync(out.data(), fd_hist_.p, out.size() * sizeof(double), cudaMemcpyDeviceToHost, st_), "d2h");
@@ -721,13 +728,7 @@ void Engine::smoothed_iteration_body() {
 	}
 	double* prim = cur_ ? f64_.P1.p : f64_.P0.p;
 	double* other = cur_ ? f64_.P0.p : f64_.P1.p;
-	ReduceArgs a = make_reduce(NR_, NA_, nb_, roff_d_.p, chunk_, max_chunks_, partial_.p, wall_off_.p, wall_face_.p,
-	                           (int)wall_face_.n, wall_terms_.p, face_lr_.p, S_.p, fc_.p, denom_, hist_d_.p, iter_d_.p,
-	                           bad_d_.p);
-	a.wall_denom = wall_denom_d_.p;
-	launch_reduce<double>(a, f64_.Rc.p, f64_.Rd.p, prim, st_);
-	launch_halo<double>((int)halo_dst_.n, halo_dst_.p, halo_src_.p, NA_, prim, other, st_);
-	launch_iter_advance(iter_d_.p, st_);
+	launch_tail<double>(reduce_args(hist_d_.p, iter_d_.p, true), f64_.Rc.p, f64_.Rd.p, prim, other, st_);
 }
 
 template <class T>
@@ -775,47 +776,52 @@ void Engine::iteration_body(Fused<T>& f, int parity, std::vector<cudaEvent_t>* m
 		mark();
 		p ^= 1;
 	}
-	ReduceArgs a = make_reduce(NR_, NA_, nb_, roff_d_.p, chunk_, max_chunks_, partial_.p, wall_off_.p, wall_face_.p,
-	                           (int)wall_face_.n, wall_terms_.p, face_lr_.p, S_.p, fc_.p, denom_, hist_d_.p, iter_d_.p,
-	                           bad_d_.p);
-	a.wall_denom = wall_denom_d_.p;
-	launch_reduce<T>(a, f.Rc.p, f.Rd.p, p ? f.P1.p : f.P0.p, st_);
-	launch_halo<T>((int)halo_dst_.n, halo_dst_.p, halo_src_.p, NA_, p ? f.P1.p : f.P0.p, p ? f.P0.p : f.P1.p, st_);
-	launch_iter_advance(iter_d_.p, st_);
+	launch_tail<T>(reduce_args(hist_d_.p, iter_d_.p, true), f.Rc.p, f.Rd.p, p ? f.P1.p : f.P0.p, p ? f.P0.p : f.P1.p,
+	               st_);
+	if (marks) {
+		pend_ = 1;
+		flush_tail();
+	}
 	mark();
 }
 
 int Engine::launches_per_iteration() const {
 	const int stages = (int)alpha_.size();
-	if (deck_.smoothing)  // W0, spectral radius, time step; per stage (grad, lim,) conv, diss, 2 smoothing, update, BC
-		return 3 + stages * ((order_ == 2 ? 2 : 0) + 6) + 3 + (halo_dst_.n ? 1 : 0) + 1;
-	return (order_ == 2 ? 2 * stages : stages + 1) + 3 /*reduce*/ + (halo_dst_.n ? 1 : 0) + 1 /*advance*/;
+	if (deck_.smoothing)  // W0, spectral radius, time step; per stage (grad, lim,) conv, diss, 2 smoothing, update, BC; tail
+		return 3 + stages * ((order_ == 2 ? 2 : 0) + 6) + 1;
+	return (order_ == 2 ? 2 * stages : stages + 1) + 1 /*tail; its sums once per TAIL_SLOTS iterations*/;
+}
+
+// Launches one outer iteration (its captured graph, or eagerly); the tail's
+// sums follow once per TAIL_SLOTS iterations and before the caller reads them.
+template <class T>
+void Engine::step(Fused<T>& f) {
+	if (opt_.use_graph) {
+		if (!graph_[cur_]) {
+			cudaGraph_t g;
+			cuda_ok(cudaStreamBeginCapture(st_, cudaStreamCaptureModeThreadLocal), "capture");
+			iteration_body<T>(f, cur_, nullptr);
+			cuda_ok(cudaStreamEndCapture(st_, &g), "capture");
+			cuda_ok(cudaGraphInstantiate(&graph_[cur_], g, 0), "graph instantiate");
+			cudaGraphDestroy(g);
+		}
+		cuda_ok(cudaGraphLaunch(graph_[cur_], st_), "graph launch");
+	} else {
+		iteration_body<T>(f, cur_, nullptr);
+		check("iteration");
+	}
+	cur_ ^= deck_.smoothing ? 0 : ((int)alpha_.size() & 1);
+	if (++pend_ == TAIL_SLOTS) flush_tail();
 }
 
 template <class T>
 void Engine::run_iterations(Fused<T>& f, int n) {
-	const int stages = (int)alpha_.size();
 	while (n > 0) {
 		if (dev_iter_ == (int)opt_.hist_capacity) collect_history(total_iter_, dev_iter_);
 		const int room = (int)opt_.hist_capacity - dev_iter_;
 		const int m = std::min(n, room);
-		for (int i = 0; i < m; i++) {
-			if (opt_.use_graph) {
-				if (!graph_[cur_]) {
-					cudaGraph_t g;
-					cuda_ok(cudaStreamBeginCapture(st_, cudaStreamCaptureModeThreadLocal), "capture");
-					iteration_body<T>(f, cur_, nullptr);
-					cuda_ok(cudaStreamEndCapture(st_, &g), "capture");
-					cuda_ok(cudaGraphInstantiate(&graph_[cur_], g, 0), "graph instantiate");
-					cudaGraphDestroy(g);
-				}
-				cuda_ok(cudaGraphLaunch(graph_[cur_], st_), "graph launch");
-			} else {
-				iteration_body<T>(f, cur_, nullptr);
-				check("iteration");
-			}
-			cur_ ^= deck_.smoothing ? 0 : (stages & 1);
-		}
+		for (int i = 0; i < m; i++) step(f);
+		flush_tail();
 		dev_iter_ += m;
 		n -= m;
 		// a shard's records need every rank's norms: kept on the device until taken
@@ -852,26 +858,11 @@ double Engine::iterate_timed(int n) {
 	cuda_ok(cudaEventCreate(&e0), "event");
 	cuda_ok(cudaEventCreate(&e1), "event");
 	cuda_ok(cudaEventRecord(e0, st_), "event");
-	const int stages = (int)alpha_.size();
 	for (int i = 0; i < n; i++) {
-		if (opt_.use_graph) {
-			if (!graph_[cur_]) {
-				cudaGraph_t g;
-				cuda_ok(cudaStreamBeginCapture(st_, cudaStreamCaptureModeThreadLocal), "capture");
-				if (opt_.precision == PREC_FP64) iteration_body<double>(f64_, cur_, nullptr);
-				else iteration_body<float>(f32_, cur_, nullptr);
-				cuda_ok(cudaStreamEndCapture(st_, &g), "capture");
-				cuda_ok(cudaGraphInstantiate(&graph_[cur_], g, 0), "graph instantiate");
-				cudaGraphDestroy(g);
-			}
-			cuda_ok(cudaGraphLaunch(graph_[cur_], st_), "graph launch");
-		} else {
-			if (opt_.precision == PREC_FP64) iteration_body<double>(f64_, cur_, nullptr);
-			else iteration_body<float>(f32_, cur_, nullptr);
-			check("iteration");
-		}
-		cur_ ^= deck_.smoothing ? 0 : (stages & 1);
+		if (opt_.precision == PREC_FP64) step(f64_);
+		else step(f32_);
 	}
+	flush_tail();
 	cuda_ok(cudaEventRecord(e1, st_), "event");
 	cuda_ok(cudaEventSynchronize(e1), "event sync");
 	float ms = 0.f;

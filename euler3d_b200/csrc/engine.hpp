@@ -269,7 +269,13 @@ private:
 	DevBuf<double> partial_, hist_d_, fd_hist_, wall_terms_;
 	DevBuf<int> iter_d_, bad_d_, zero_d_;
 	bool started_ = false;
-	int chunk_ = 0, max_chunks_ = 0;
+	int max_chunks_ = 0;
+	DevBuf<int> pend_d_;  // iterations in the tail ring, block counter of the running tail launch
+	int pend_ = 0;        // the same count on the host
+	ReduceArgs reduce_args(double* hist, int* d_iter, bool with_halo) const;
+	void flush_tail();
+	template <class T>
+	void step(Fused<T>& f);
 	int dev_iter_ = 0;  // iterations recorded on the device since the last collect
 	int total_iter_ = 0;
 	std::vector<char> have_rms0_;

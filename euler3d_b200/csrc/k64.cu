@@ -57,7 +57,9 @@ void launch_update(const GeoView& g, const StateView& s, const Physics& ph, doub
 void launch_bc(const GeoView& g, const StateView& s, const Physics& ph, int g0, int g1, cudaStream_t st) {
 	if (g1 > g0) k_bc<<<blocks_for(g1 - g0, TPB), TPB, 0, st>>>(g, s, ph, g0, g1);
 }
-void launch_iter_advance(int* d_iter, cudaStream_t st) { k_iter_advance<<<1, 1, 0, st>>>(d_iter); }
+void launch_tail_sums(const ReduceArgs& a, int n, bool advance, cudaStream_t st) {
+	if (n > 0) k_tail_sums<<<dim3(a.nblocks, n), 160, 0, st>>>(a, advance ? 1 : 0);
+}
 void launch_smooth(const GeoView& g, const StateView& s, double* j1, int r0, int r1, cudaStream_t st) {
 	if (r1 <= r0) return;
 	k_irs_start<<<blocks_for(r1 - r0, TPB), TPB, 0, st>>>(g, s, j1, r0, r1);
@@ -67,7 +69,7 @@ void launch_smooth(const GeoView& g, const StateView& s, double* j1, int r0, int
 template void launch_halo<double>(int, const int*, const int*, int, double*, double*, cudaStream_t);
 template void launch_halo_pack<double>(int, const int*, int, const double*, double*, cudaStream_t);
 template void launch_halo_unpack<double>(int, const int*, int, const double*, double*, double*, cudaStream_t);
-template void launch_reduce<double>(const ReduceArgs&, const double*, const double*, const double*, cudaStream_t);
+template void launch_tail<double>(const ReduceArgs&, const double*, const double*, double*, double*, cudaStream_t);
 template void launch_recon<double>(const FusedView<double>&, const Physics&, int, int, bool, int, cudaStream_t);
 template void launch_start<double>(const FusedView<double>&, const Physics&, int, cudaStream_t);
 template void launch_flux_update<double>(const FusedView<double>&, const Physics&, int, bool, double, double, int, int,

@@ -33,30 +33,12 @@ void launch_halo_pack(int n, const int* src, int NA, const T* P, T* buf, cudaStr
 template <class T>
 void launch_halo_unpack(int n, const int* dst, int NA, const T* buf, T* b0, T* b1, cudaStream_t);
 
-// Per-block reductions written into hist[iter*stride + b*10 + (0..4 norms, 5..9 forces)],
-// iter read from *d_iter (the device iteration counter).
-struct ReduceArgs {
-	int NR, NA, nblocks;
-	const int* roff;       // nblocks+1 real-cell offsets
-	int chunk, max_chunks;
-	double* partial;       // nblocks*max_chunks*5
-	const int* wall_off;   // nblocks+1
-	const int* wall_face;
-	int n_wall;
-	double* wall_terms;    // 5*n_wall
-	const int* face_lr;
-	const double* S;
-	const double* fc;
-	double denom;          // 0.5*gamma*M*M*cmac
-	const double* wall_denom;  // per wall face (cases of a batch differ in Mach), or null
-	double* hist;
-	int stride;
-	const int* d_iter;
-	int* d_bad;
-};
+// end of an iteration (k_tail), then the sums of the iterations in its ring (k_tail_sums);
+// P: current primitives, P2: the other buffer (halo ghosts are written to both)
 template <class T>
-void launch_reduce(const ReduceArgs&, const T* Rc, const T* Rd, const T* P, cudaStream_t);
-void launch_iter_advance(int* d_iter, cudaStream_t);
+void launch_tail(const ReduceArgs&, const T* Rc, const T* Rd, T* P, T* P2, cudaStream_t);
+// n: pending iterations; advance: move *d_iter on by n
+void launch_tail_sums(const ReduceArgs&, int n, bool advance, cudaStream_t);
 
 // ---- fused stage kernels ----
 template <class T>

@@ -21,16 +21,10 @@ void launch_halo_unpack(int n, const int* dst, int NA, const T* buf, T* b0, T* b
 }
 
 template <class T>
-void launch_reduce(const ReduceArgs& a, const T* Rc, const T* Rd, const T* P, cudaStream_t st) {
-	constexpr int THREADS = 256;
-	dim3 grid(a.max_chunks, a.nblocks);
-	k_norm_partial<T, THREADS><<<grid, THREADS, 0, st>>>(Rc, Rd, a.NR, a.roff, a.chunk, a.max_chunks, a.partial);
-	k_norm_final<<<(a.nblocks * 5 + 127) / 128, 128, 0, st>>>(a.partial, a.nblocks, a.max_chunks, a.hist, a.stride,
-	                                                         a.d_iter, a.d_bad);
-	if (a.n_wall > 0)
-		k_wall_terms<T><<<(a.n_wall + 127) / 128, 128, 0, st>>>(P, a.NA, a.n_wall, a.wall_face, a.face_lr, a.S, a.fc,
-		                                                     a.denom, a.wall_denom, a.wall_terms);
-	k_wall_sums<<<a.nblocks, 128, 0, st>>>(a.wall_terms, a.n_wall, a.wall_off, a.hist, a.stride, a.d_iter);
+void launch_tail(const ReduceArgs& a, const T* Rc, const T* Rd, T* P, T* P2, cudaStream_t st) {
+	const auto blocks = [](int n) { return (n + TAIL_TPB - 1) / TAIL_TPB; };
+	const int grid = a.nblocks * a.max_chunks + blocks(a.n_wall) + blocks(a.n_halo);
+	k_tail<T><<<grid, TAIL_TPB, 0, st>>>(a, Rc, Rd, P, P2);
 }
 
 // FP64 later stages on tetrahedra: one lane per (cell, variable)

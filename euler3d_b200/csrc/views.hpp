@@ -89,6 +89,37 @@ struct FusedView {
 	const double* nhat64;     // 3*NF
 };
 
+// End of an iteration (k_tail, k_tail_sums): norm chunks, wall terms and halo
+// of one iteration into ring slot *pend, then the per-block sums of all pending
+// iterations into hist[(*d_iter + i)*stride + b*10 + (0..4 norms, 5..9 forces)].
+constexpr int TAIL_TPB = 256;     // threads per block of k_tail
+constexpr int TAIL_CHUNK = 1024;  // cells per norm chunk: 48 blocks at 48k cells, 3,000 at 3.07M
+constexpr int TAIL_SLOTS = 32;    // iterations the ring holds
+struct ReduceArgs {
+	int NR, NA, nblocks;
+	const int* roff;       // nblocks+1 real-cell offsets
+	int max_chunks;        // TAIL_CHUNK-cell chunks of the largest block
+	double* partial;       // TAIL_SLOTS*nblocks*5*max_chunks
+	const int* wall_off;   // nblocks+1
+	const int* wall_face;
+	int n_wall;
+	double* wall_terms;    // TAIL_SLOTS*5*n_wall
+	const int* face_lr;
+	const double* S;
+	const double* fc;
+	double denom;          // 0.5*gamma*M*M*cmac
+	const double* wall_denom;  // per wall face (cases of a batch differ in Mach), or null
+	int n_halo;
+	const int* halo_dst;
+	const int* halo_src;
+	double* hist;
+	int stride;
+	int* d_iter;
+	int* d_bad;
+	int* pend;             // iterations in the ring
+	unsigned* ticket;      // blocks of the running launch that are done
+};
+
 // One launch of the persistent batch kernel: several outer iterations over the
 // work list (tiles of real cells of the active cases).
 struct PersistArgs {
