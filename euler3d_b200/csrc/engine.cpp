@@ -269,6 +269,7 @@ void Engine::build_blocks(const std::vector<const HostBlock*>& blocks, const std
 	tet4_ = 1;
 	for (int c = 0; c < NR_ && tet4_; c++)
 		if (slot_ptr[c] != 4 * c || slot_ptr[c + 1] != 4 * c + 4) tet4_ = 0;
+	if (tet4_ && NS_ != 4 * NR_ + NG_) throw Error(E3D_ERR_MESH, "internal: ghost cell without exactly one face");
 	std::vector<int> slot_face(NS_), slot_nbr(NS_), slot_mate(NS_);
 	std::vector<double> lsw(3 * (size_t)NS_, 0.0);
 	std::vector<int> face_lr(2 * (size_t)NF_);

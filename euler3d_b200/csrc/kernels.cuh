@@ -873,43 +873,54 @@ __global__ void __launch_bounds__(128) k_start(FusedView<T> v, Physics ph, int c
 // the dissipative flux (its guard is always true) but Rd*(1-0) + sum(D*0) equals
 // Rd for finite fluxes, so the flux and the Rd store are skipped.  Rc is stored
 // only at the last stage, the one the norms (and callers) read.
+//
+// One face at a time (FP64: the slot loop stays rolled).  Holding all four
+// slots' mates, normals and neighbours live took the FP64 Roe pass to 128
+// registers and 23 % resident warps, with instruction-cache misses from four
+// copies of the flux; one copy needs 96.  Neighbours of a tetrahedron follow
+// from the mate slot (real slot 4c+k, ghost g's only slot 4 NR + g), so
+// slot_nbr is not read, and beta = 1 drops Rd unread.  B200, us a launch with /
+// without dissipation: 663k tets FP64 Roe 136 / 100 -> 121 / 88; 3.07M FP32
+// Roe 184 / 147 -> 175 / 144 (FP32 keeps the loop unrolled: 178 / 156 rolled).
 template <class T, int SCHEME, bool ORDER1, int NSL, bool DISS>
 __device__ __forceinline__ void flux_update_cell(const FusedView<T>& v, const Physics& ph, T alpha, T beta, int last,
                                                  int carry_w0, int c) {
+	constexpr int UNROLL = NSL == 4 && sizeof(T) == 4 ? 4 : 1;
+	const int NR = v.NR;
 	const SlotRange<T, NSL> sr(v, c);
 	const T g = T(ph.gamma), gr = T(ph.gr), gm1 = T(ph.gm1);
-	int mate[MAXSL];
-	load_int<T, NSL>(v.slot_mate, sr, mate);
+	const T keep = T(1.0) - beta;
 	T ac[5], ad[5];
 	for (int q = 0; q < 5; q++) {
 		ac[q] = T(0.0);
-		ad[q] = DISS ? v.Rd[q * v.NR + c] * (T(1.0) - beta) : v.Rd[q * v.NR + c];
+		ad[q] = (!DISS || keep != T(0.0)) ? v.Rd[q * (size_t)NR + c] : T(0.0);
+		if (DISS) ad[q] *= keep;
 	}
 	Q5<T> qc;
-	int nb[MAXSL];
-	if (ORDER1) {
-		qc = ld5(v.Pin, v.NA, c);
-		load_int<T, NSL>(v.slot_nbr, sr, nb);
-	}
+	if (ORDER1) qc = ld5(v.Pin, v.NA, c);
 #ifdef E3D_SHARED_SIDES
 	constexpr bool shared_sides = ORDER1 && SCHEME == FLUX_AUSM;
 	AusmSide<T> own;
 	if constexpr (shared_sides) own = ausm_side(qc, g, gr);
 #endif
-	T geo[MAXSL][4];
-	load_geo<T, NSL>(v.sgeo, sr, geo);
-#pragma unroll
-	E3D_SLOTS(k, sr) {
-		const bool left = mate[k] >= 0;
-		const int m = left ? mate[k] : ~mate[k];
+	unsigned ghosts = 0;  // slots with a ghost neighbour
+#pragma unroll UNROLL
+	for (int k = 0; k < (NSL == 4 ? 4 : sr.n); k++) {
+		const int s = sr.s0 + k;
+		const int mt = v.slot_mate[s];
+		const bool left = mt >= 0;
+		const int m = left ? mt : ~mt;
+		const int nb = NSL == 4 ? (m < 4 * NR ? m >> 2 : m - 3 * NR) : v.slot_nbr[s];
+		if (nb >= NR) ghosts |= 1u << k;
 		Q5<T> qo, qn;
 		if (ORDER1) {
 			qo = qc;
-			qn = ld5(v.Pin, v.NA, nb[k]);
+			qn = ld5(v.Pin, v.NA, nb);
 		} else {
-			qo = ld5(v.FS, v.NS, sr.s0 + k);
+			qo = ld5(v.FS, v.NS, s);
 			qn = ld5(v.FS, v.NS, m);
 		}
+		const typename Vec4<T>::type geo = reinterpret_cast<const typename Vec4<T>::type*>(v.sgeo)[s];
 		Q5<T> L, R;
 		for (int q = 0; q < 5; q++) {
 			qv(L, q) = left ? qv(qo, q) : qv(qn, q);
@@ -921,68 +932,184 @@ __device__ __forceinline__ void flux_update_cell(const FusedView<T>& v, const Ph
 			const AusmSide<T> nbr = ausm_side(qn, g, gr);
 			// sides selected by value: a branch on the orientation would run the
 			// face arithmetic twice in warps whose cells differ
-			ausm_face_sides<T, DISS>(left ? own : nbr, left ? nbr : own, geo[k][0], geo[k][1], geo[k][2], geo[k][3],
-			                         fc, fd);
+			ausm_face_sides<T, DISS>(left ? own : nbr, left ? nbr : own, geo.x, geo.y, geo.z, geo.w, fc, fd);
 		} else
 #endif
 		if (SCHEME == FLUX_ROE) {
-			flux_central(L, R, geo[k][0], geo[k][1], geo[k][2], geo[k][3], gr, fc);
-			if (DISS) flux_roe_diss(L, R, geo[k][0], geo[k][1], geo[k][2], geo[k][3], gr, gm1, fd);
+			flux_central(L, R, geo.x, geo.y, geo.z, geo.w, gr, fc);
+			if (DISS) flux_roe_diss(L, R, geo.x, geo.y, geo.z, geo.w, gr, gm1, fd);
 		} else {
-			flux_ausm_conv(L, R, geo[k][0], geo[k][1], geo[k][2], geo[k][3], g, gr, fc);
-			if (DISS) flux_ausm_diss(L, R, geo[k][0], geo[k][1], geo[k][2], geo[k][3], g, gr, fd);
+			flux_ausm_conv(L, R, geo.x, geo.y, geo.z, geo.w, g, gr, fc);
+			if (DISS) flux_ausm_diss(L, R, geo.x, geo.y, geo.z, geo.w, g, gr, fd);
 		}
-		if (left) {
-			for (int q = 0; q < 5; q++) {
-				ac[q] += fc[q];
-				if (DISS) ad[q] += fd[q] * beta;
-			}
-		} else {
-			for (int q = 0; q < 5; q++) {
-				ac[q] -= fc[q];
-				if (DISS) ad[q] -= fd[q] * beta;
-			}
+		for (int q = 0; q < 5; q++) {
+			ac[q] += left ? fc[q] : -fc[q];
+			if (DISS) ad[q] += (left ? fd[q] : -fd[q]) * beta;
 		}
 	}
 	double w0[5], wn[5];
 	for (int q = 0; q < 5; q++) {
-		if (last) v.Rc[q * v.NR + c] = ac[q];
-		if (DISS) v.Rd[q * v.NR + c] = ad[q];
-		w0[q] = v.W0[q * v.NR + c];
+		if (last) v.Rc[q * (size_t)NR + c] = ac[q];
+		if (DISS) v.Rd[q * (size_t)NR + c] = ad[q];
+		w0[q] = v.W0[q * (size_t)NR + c];
 	}
 	const T coef = alpha * v.dt[c] / v.vol[c];
 	const Q5<T> qnew = conservative_update<T>(w0, coef, ac, ad, gm1, wn);
 	st5(v.Pout, v.NA, c, qnew);
 	if (last && carry_w0)
-		for (int q = 0; q < 5; q++) v.W0[q * v.NR + c] = wn[q];
-	if (!ORDER1) load_int<T, NSL>(v.slot_nbr, sr, nb);
+		for (int q = 0; q < 5; q++) v.W0[q * (size_t)NR + c] = wn[q];
+	while (ghosts) {
+		const int s = sr.s0 + __ffs(ghosts) - 1;
+		ghosts &= ghosts - 1;
+		int nb;
+		if (NSL == 4) {
+			const int mt = v.slot_mate[s];
+			nb = (mt >= 0 ? mt : ~mt) - 3 * NR;
+		} else {
+			nb = v.slot_nbr[s];
+		}
+		const int kind = v.gkind[nb - NR];
+		if (kind == GK_NONE) continue;
+		// freestream of the ghost's case (batched cases differ in Mach and alpha)
+		const double* f = v.case_free ? v.case_free + 5 * v.gcase[nb - NR] : ph.free;
+		const Q5<T> fr{T(f[0]), T(f[1]), T(f[2]), T(f[3]), T(f[4])};
+		const T* n = v.sgeo + 4 * (size_t)s;
+		st5(v.Pout, v.NA, nb, ghost_state(kind, qnew, fr, n[0], n[1], n[2], g));
+	}
+}
+
+// resident blocks per SM the FP64 flux pass is compiled for (5: 96 registers;
+// 663k tets, Roe: 121 us at 5, 128 at 6, 138 at 7)
+#ifndef E3D_FLUX64_MIN_BLOCKS
+#define E3D_FLUX64_MIN_BLOCKS 5
+#endif
+template <class T, int SCHEME, bool ORDER1, int NSL, bool DISS>
+__global__ void __launch_bounds__(128, sizeof(T) == 4 ? 8 : E3D_FLUX64_MIN_BLOCKS) k_flux_update(FusedView<T> v, Physics ph, T alpha, T beta, int last, int carry_w0) {
+	const int c = blockIdx.x * blockDim.x + threadIdx.x;
+	if (c < v.NR) flux_update_cell<T, SCHEME, ORDER1, NSL, DISS>(v, ph, alpha, beta, last, carry_w0, c);
+}
+
+// FP64 pass 2 with one lane per slot, LPC lanes per cell (4: tetrahedra; 8: up to
+// 6 slots).  flux_update_cell runs a cell's face fluxes one after the other in
+// one thread, a dependent chain of ~2,000 FP64 operations (Roe): on a small mesh
+// a launch is that latency (3k cells: 19 us, here 11).  Here each lane
+// forms one face's flux, then the cell's lanes exchange them through shared
+// memory and lane k adds up variable k over the slots in ascending face id
+// (the reference's order, so FP64 results are the same bits) and updates it;
+// lane 0 has the energy too.
+template <int SCHEME, bool ORDER1, int LPC, bool DISS>
+__device__ __forceinline__ void flux_update_slots(const FusedView<double>& v, const Physics& ph, double alpha, double beta, int last,
+                                                  int carry_w0, int c, bool in_range, double (*sm)[33]) {
+	constexpr unsigned FULL = 0xffffffffu;
+	const int lane = threadIdx.x & 31, k = lane & (LPC - 1), first = lane - k;
+	const int NR = v.NR;
+	const double g = ph.gamma, gr = ph.gr, gm1 = ph.gm1;
+	int s0 = LPC * c, n = LPC;
+	if (LPC != 4) {
+		s0 = v.slot_ptr[c];
+		n = v.slot_ptr[c + 1] - s0;
+	}
+	const bool on = in_range && k < n;
+	const int s = s0 + (k < n ? k : 0);
+	const int mt = v.slot_mate[s];
+	const bool left = mt >= 0;
+	const int m = left ? mt : ~mt;
+	const int nb = LPC == 4 ? (m < 4 * NR ? m >> 2 : m - 3 * NR) : v.slot_nbr[s];
+	const Q5<double> qo = ORDER1 ? ld5(v.Pin, v.NA, c) : ld5(v.FS, v.NS, s);
+	const Q5<double> qn = ORDER1 ? ld5(v.Pin, v.NA, nb) : ld5(v.FS, v.NS, m);
+	const typename Vec4<double>::type geo = reinterpret_cast<const typename Vec4<double>::type*>(v.sgeo)[s];
+	// this lane's share of the cell: variable k, and variable 4 on lane 0
+	const int qk = k < 4 ? k : 0;
+	const double keep = 1.0 - beta;
+	double rd = 0.0, rd4 = 0.0;
+	if (!DISS || keep != 0.0) {  // beta = 1 (the first stage) drops the old value
+		rd = v.Rd[(size_t)qk * NR + c];
+		if (k == 0) rd4 = v.Rd[4 * (size_t)NR + c];
+	}
+	const double w0 = v.W0[(size_t)qk * NR + c];
+	const double w04 = k == 0 ? v.W0[4 * (size_t)NR + c] : 0.0;
+	const double coef = alpha * v.dt[c] / v.vol[c];
+	{
+		Q5<double> L, R;
+		for (int q = 0; q < 5; q++) {
+			qv(L, q) = left ? qv(qo, q) : qv(qn, q);
+			qv(R, q) = left ? qv(qn, q) : qv(qo, q);
+		}
+		double fc[5], fd[5];
+		if (SCHEME == FLUX_ROE) {
+			flux_central(L, R, geo.x, geo.y, geo.z, geo.w, gr, fc);
+			if (DISS) flux_roe_diss(L, R, geo.x, geo.y, geo.z, geo.w, gr, gm1, fd);
+		} else {
+			flux_ausm_conv(L, R, geo.x, geo.y, geo.z, geo.w, g, gr, fc);
+			if (DISS) flux_ausm_diss(L, R, geo.x, geo.y, geo.z, geo.w, g, gr, fd);
+		}
 #pragma unroll
-	E3D_SLOTS(k, sr) {
-		if (nb[k] >= v.NR) {
-			const int gi = nb[k] - v.NR;
-			const int kind = v.gkind[gi];
-			if (kind != GK_NONE) {
-				// freestream of the ghost's case (batched cases differ in Mach and alpha)
-				const double* f = v.case_free ? v.case_free + 5 * v.gcase[gi] : ph.free;
-				Q5<T> fr;
-				fr.r = T(f[0]);
-				fr.u = T(f[1]);
-				fr.v = T(f[2]);
-				fr.w = T(f[3]);
-				fr.p = T(f[4]);
-				// the face normal is read again here (boundary slots only) so that the
-				// slots' geometry need not stay live through the update
-				const T* n = v.sgeo + 4 * (size_t)(sr.s0 + k);
-				st5(v.Pout, v.NA, nb[k], ghost_state(kind, qnew, fr, n[0], n[1], n[2], g));
-			}
+		for (int q = 0; q < 5; q++) {
+			sm[q][lane] = left ? fc[q] : -fc[q];
+			if (DISS) sm[5 + q][lane] = left ? fd[q] : -fd[q];
+		}
+	}
+	__syncwarp();
+	double ac = 0.0, ad = DISS ? rd * keep : rd, ac4 = 0.0, ad4 = DISS ? rd4 * keep : rd4;
+#pragma unroll
+	for (int i = 0; i < (LPC == 4 ? 4 : MAXSL); i++) {
+		if (LPC != 4 && i >= n) break;
+		ac += sm[qk][first + i];
+		if (DISS) ad += sm[5 + qk][first + i] * beta;
+		if (k == 0) {
+			ac4 += sm[4][first + i];
+			if (DISS) ad4 += sm[9][first + i] * beta;
+		}
+	}
+	const double wn = w0 - coef * (ac - ad);
+	const double wn4 = w04 - coef * (ac4 - ad4);
+	const double r = __shfl_sync(FULL, wn, first);
+	const double mx = __shfl_sync(FULL, wn, first + 1), my = __shfl_sync(FULL, wn, first + 2),
+	             mz = __shfl_sync(FULL, wn, first + 3);
+	// one division per lane: the velocity component, on lane 0 the kinetic energy
+	const double x = (k == 0 ? 0.5 * (mx * mx + my * my + mz * mz) : wn) / r;
+	const double qnew = k == 0 ? r : x;
+	const double pnew = (gm1 * (wn4 - x));
+	if (in_range && k < 4) {
+		if (last) v.Rc[(size_t)k * NR + c] = ac;
+		if (DISS) v.Rd[(size_t)k * NR + c] = ad;
+		v.Pout[4 * (size_t)c + k] = qnew;
+		if (last && carry_w0) v.W0[(size_t)k * NR + c] = wn;
+		if (k == 0) {
+			if (last) v.Rc[4 * (size_t)NR + c] = ac4;
+			if (DISS) v.Rd[4 * (size_t)NR + c] = ad4;
+			v.Pout[4 * (size_t)v.NA + c] = pnew;
+			if (last && carry_w0) v.W0[4 * (size_t)NR + c] = wn4;
+		}
+	}
+	// boundary conditions of the cell's ghost cells
+	const bool ghost = on && nb >= NR;
+	if (__any_sync(FULL, ghost)) {
+		Q5<double> q;
+		q.r = __shfl_sync(FULL, qnew, first);
+		q.u = __shfl_sync(FULL, qnew, first + 1);
+		q.v = __shfl_sync(FULL, qnew, first + 2);
+		q.w = __shfl_sync(FULL, qnew, first + 3);
+		q.p = __shfl_sync(FULL, pnew, first);
+		const int kind = ghost ? v.gkind[nb - NR] : (int)GK_NONE;
+		if (kind != GK_NONE) {
+			// freestream of the ghost's case (batched cases differ in Mach and alpha)
+			const double* f = v.case_free ? v.case_free + 5 * v.gcase[nb - NR] : ph.free;
+			const Q5<double> fr{f[0], f[1], f[2], f[3], f[4]};
+			st5(v.Pout, v.NA, nb, ghost_state(kind, q, fr, geo.x, geo.y, geo.z, g));
 		}
 	}
 }
 
-template <class T, int SCHEME, bool ORDER1, int NSL, bool DISS>
-__global__ void __launch_bounds__(128, sizeof(T) == 4 ? 8 : E3D_FP64_MIN_BLOCKS) k_flux_update(FusedView<T> v, Physics ph, T alpha, T beta, int last, int carry_w0) {
-	const int c = blockIdx.x * blockDim.x + threadIdx.x;
-	if (c < v.NR) flux_update_cell<T, SCHEME, ORDER1, NSL, DISS>(v, ph, alpha, beta, last, carry_w0, c);
+template <int SCHEME, bool ORDER1, int LPC, bool DISS>
+__global__ void __launch_bounds__(128, 4)
+    k_flux_slots(FusedView<double> v, Physics ph, double alpha, double beta, int last, int carry_w0) {
+	__shared__ double sm[4][DISS ? 10 : 5][33];
+	const int c = (blockIdx.x * 128 + threadIdx.x) / LPC;
+	const bool in_range = c < v.NR;
+	if (__any_sync(0xffffffffu, in_range))
+		flux_update_slots<SCHEME, ORDER1, LPC, DISS>(v, ph, alpha, beta, last, carry_w0, in_range ? c : v.NR - 1,
+		                                                in_range, sm[threadIdx.x >> 5]);
 }
 
 // ===================================================================== reductions

@@ -73,21 +73,38 @@ void launch_start(const FusedView<T>& v, const Physics& ph, int carry, cudaStrea
 	else k_start<T, 0><<<(v.NR + 127) / 128, 128, 0, st>>>(v, ph, carry);
 }
 
+// Largest mesh (tetrahedra; half of it for 8 lanes per cell) whose FP64 flux
+// pass runs one lane per slot.  Below it a launch is latency: four times the
+// threads, each with a quarter of the chain.  Above it the exchange through shared
+// memory costs more than it hides.  B200, us a launch with dissipation, per cell /
+// per slot: Roe 3k 19 / 11, 48k 25 / 20, 132k 40 / 34, 216k 53 / 50 (second order
+// 57 / 55), 384k 80 / 88; AUSM 3k 16 / 10, 48k 18 / 16, 83k 20 / 21, 216k 33 / 39.
+// FP32 gains little (3k 10 / 8, 48k 10.5 / 10.6) and keeps one form, so that the
+// batch kernels and this path round alike.
+constexpr int slot_pass_cells(int scheme) { return scheme == FLUX_ROE ? 220000 : 80000; }
+
 template <class T>
 void launch_flux_update(const FusedView<T>& v, const Physics& ph, int scheme, bool order1, double alpha, double beta,
                         int last, int carry, cudaStream_t st) {
 	if (v.NR <= 0) return;
-	const int grid = (v.NR + 127) / 128;
+	const int grid = (v.NR + 127) / 128, g4 = (v.NR + 31) / 32, g8 = (v.NR + 15) / 16;
+	const bool slots = sizeof(T) == 8 && v.NR <= slot_pass_cells(scheme) / (v.tet4 ? 1 : 2);
 	const T a = T(alpha), b = T(beta);
-#define E3D_FLUX(S, O)                                                                                  \
-	do {                                                                                                \
-		if (beta != 0.0) {                                                                              \
-			if (v.tet4) k_flux_update<T, S, O, 4, true><<<grid, 128, 0, st>>>(v, ph, a, b, last, carry);  \
-			else k_flux_update<T, S, O, 0, true><<<grid, 128, 0, st>>>(v, ph, a, b, last, carry);         \
-		} else {                                                                                        \
-			if (v.tet4) k_flux_update<T, S, O, 4, false><<<grid, 128, 0, st>>>(v, ph, a, b, last, carry); \
-			else k_flux_update<T, S, O, 0, false><<<grid, 128, 0, st>>>(v, ph, a, b, last, carry);        \
-		}                                                                                               \
+#define E3D_FLUX_D(S, O, D)                                                                                \
+	do {                                                                                                   \
+		if constexpr (sizeof(T) == 8)                                                                      \
+			if (slots) {                                                                                   \
+				if (v.tet4) k_flux_slots<S, O, 4, D><<<g4, 128, 0, st>>>(v, ph, a, b, last, carry);        \
+				else k_flux_slots<S, O, 8, D><<<g8, 128, 0, st>>>(v, ph, a, b, last, carry);               \
+				break;                                                                                     \
+			}                                                                                              \
+		if (v.tet4) k_flux_update<T, S, O, 4, D><<<grid, 128, 0, st>>>(v, ph, a, b, last, carry);          \
+		else k_flux_update<T, S, O, 0, D><<<grid, 128, 0, st>>>(v, ph, a, b, last, carry);                 \
+	} while (0)
+#define E3D_FLUX(S, O)                                                                                     \
+	do {                                                                                                   \
+		if (beta != 0.0) E3D_FLUX_D(S, O, true);                                                           \
+		else E3D_FLUX_D(S, O, false);                                                                      \
 	} while (0)
 	if (scheme == FLUX_AUSM) {
 		if (order1) E3D_FLUX(FLUX_AUSM, true);
@@ -97,6 +114,7 @@ void launch_flux_update(const FusedView<T>& v, const Physics& ph, int scheme, bo
 		else E3D_FLUX(FLUX_ROE, false);
 	}
 #undef E3D_FLUX
+#undef E3D_FLUX_D
 }
 
 }  // namespace e3d
