@@ -790,7 +790,7 @@ int Engine::launches_per_iteration() const {
 	const int stages = (int)alpha_.size();
 	if (deck_.smoothing)  // W0, spectral radius, time step; per stage (grad, lim,) conv, diss, 2 smoothing, update, BC; tail
 		return 3 + stages * ((order_ == 2 ? 2 : 0) + 6) + 1;
-	return (order_ == 2 ? 2 * stages : stages + 1) + 1 /*tail; its sums once per TAIL_SLOTS iterations*/;
+	return (order_ == 2 ? 2 * stages + (tet4_ ? 0 : 1) : stages + 1) + 1 /*tail; its sums once per TAIL_SLOTS iterations*/;
 }
 
 // Launches one outer iteration (its captured graph, or eagerly); the tail's

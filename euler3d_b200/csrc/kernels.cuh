@@ -179,11 +179,11 @@ __global__ void k_limiter(GeoView g, StateView s, Physics ph, int r0, int r1, in
 			if (qv(qn, v) < qv(mn, v)) qv(mn, v) = qv(qn, v);
 		}
 	}
-	double dmax[5], dmin[5], phi[5], gr[5][3];
+	double dmax[5], dmin[5], gr[5][3];
+	CellLimiter<double, LIM> phi[5];
 	for (int v = 0; v < 5; v++) {
 		dmax[v] = qv(mx, v) - qv(q0, v);
 		dmin[v] = qv(mn, v) - qv(q0, v);
-		phi[v] = INFINITY;
 		for (int d = 0; d < 3; d++) gr[v][d] = s.grad[(v * 3 + d) * g.NA + c];
 	}
 	const double eps2 = ph.k3 * g.vol[c];
@@ -193,12 +193,10 @@ __global__ void k_limiter(GeoView g, StateView s, Physics ph, int r0, int r1, in
 		for (int v = 0; v < 5; v++) {
 			double d2 = 0.0;
 			for (int d = 0; d < 3; d++) d2 += gr[v][d] * r[d];
-			const double lf = (LIM == LIM_BARTH_JESPERSEN) ? limiter_bj_face(d2, dmax[v], dmin[v], ph.omega)
-			                                               : limiter_venkat_face(d2, dmax[v], dmin[v], eps2);
-			if (lf < phi[v]) phi[v] = lf;
+			phi[v].face(d2, dmax[v], dmin[v], ph.omega, eps2);
 		}
 	}
-	for (int v = 0; v < 5; v++) s.lim[v * g.NA + c] = phi[v];
+	for (int v = 0; v < 5; v++) s.lim[v * g.NA + c] = phi[v].value(dmax[v], dmin[v]);
 }
 
 // Left/right states of face f reconstructed from gradients and limiters.
@@ -633,16 +631,16 @@ __device__ __forceinline__ void recon_cell(const FusedView<T>& v, const Physics&
 		Q5<T> fs[4];
 		for (int q = 0; q < 5; q++) {
 			const T dmax = qv(mx, q) - qv(q0, q), dmin = qv(mn, q) - qv(q0, q);
-			T d2[4], phi = T(INFINITY);
+			T d2[4];
+			CellLimiter<T, LIM> lim;
 #pragma unroll
 			for (int k = 0; k < 4; k++) {
 				d2[k] = gr[q][0] * rv[k][0];
 				d2[k] += gr[q][1] * rv[k][1];
 				d2[k] += gr[q][2] * rv[k][2];
-				const T lf = (LIM == LIM_BARTH_JESPERSEN) ? limiter_bj_face(d2[k], dmax, dmin, T(ph.omega))
-				                                          : limiter_venkat_face(d2[k], dmax, dmin, eps2);
-				if (lf < phi) phi = lf;
+				lim.face(d2[k], dmax, dmin, T(ph.omega), eps2);
 			}
+			const T phi = lim.value(dmax, dmin);
 #pragma unroll
 			for (int k = 0; k < 4; k++) qv(fs[k], q) = qv(q0, q) + phi * d2[k];
 		}
@@ -653,17 +651,16 @@ __device__ __forceinline__ void recon_cell(const FusedView<T>& v, const Physics&
 		T phi[5];
 		for (int q = 0; q < 5; q++) {
 			const T dmax = qv(mx, q) - qv(q0, q), dmin = qv(mn, q) - qv(q0, q);
-			phi[q] = T(INFINITY);
+			CellLimiter<T, LIM> lim;
 #pragma unroll
 			E3D_SLOTS(k, sr) {
 				T d2 = T(0.0);
 				d2 += gr[q][0] * rv[k][0];
 				d2 += gr[q][1] * rv[k][1];
 				d2 += gr[q][2] * rv[k][2];
-				const T lf = (LIM == LIM_BARTH_JESPERSEN) ? limiter_bj_face(d2, dmax, dmin, T(ph.omega))
-				                                          : limiter_venkat_face(d2, dmax, dmin, eps2);
-				if (lf < phi[q]) phi[q] = lf;
+				lim.face(d2, dmax, dmin, T(ph.omega), eps2);
 			}
+			phi[q] = lim.value(dmax, dmin);
 		}
 #pragma unroll
 		E3D_SLOTS(k, sr) {
@@ -729,106 +726,111 @@ __global__ void __launch_bounds__(128, sizeof(T) == 4 ? E3D_RECON_MIN_BLOCKS : E
 	if (c < v.NR) recon_cell<T, GRAD, LIM, FIRST, NSL>(v, ph, carry_w0, c);
 }
 
-// FP64 reconstruction of the later stages with one lane per (cell, variable),
-// all-tetrahedron meshes.  Gradient, limiter and face states of one variable
-// depend on that variable alone, so five lanes per cell run the same
-// per-variable arithmetic as recon_cell's FP64 branch, in the same order (bit
-// for bit), with a fifth of its gradient/limiter state and the slot weights
-// read per slot: 64 registers instead of 128, 30 resident warps per SM instead
-// of 16.  A block covers RV_CELLS cells (5 * RV_CELLS threads, cell-major: the
-// four lanes of a cell's (rho, u, v, w) read and write one 32-byte vector
-// together).  Measured on B200 (3.07M tets, second order): 2.61 TB/s against
-// 2.44 for the one-thread-per-cell pass.  The first stage keeps recon_cell: its
-// time step and W0 need the whole cell, and one lane of five doing them made
-// that pass slower (2.82 against 2.89 TB/s).
+// Reconstruction with one lane per (cell, variable): FP64 later stages on
+// tetrahedra, every stage and both precisions on other cells.  Gradient, limiter
+// and face states of one variable depend on that variable alone, so five lanes
+// per cell run the same per-variable arithmetic as recon_cell, in the same order
+// (FP64: bit for bit), with a fifth of its gradient/limiter state and the slot
+// weights read per slot: 48 registers instead of 128, 40 resident warps per SM
+// instead of 16 (663k tets FP64: 118 us at 6 blocks of 64 registers, 115 at 8).  A block covers RV_CELLS cells (5 * RV_CELLS threads,
+// cell-major: the four lanes of a cell's (rho, u, v, w) read and write one
+// 32-byte vector together).  Measured on B200 (3.07M tets, FP64 second order):
+// 2.61 TB/s against 2.44 for the one-thread-per-cell pass.  On tetrahedra the
+// first stage keeps recon_cell: its time step and W0 need the whole cell, and
+// one lane of five doing them made that pass slower (2.82 against 2.89 TB/s).
+// With slot counts known only at run time, one thread per cell kept its slot
+// arrays in local memory: 65k hexahedra FP64 40 us a launch, 25 here (the
+// first stage with W0 and the time step in k_start).
 constexpr int RV_CELLS = 32;
 #ifndef E3D_RV_MIN_BLOCKS
-#define E3D_RV_MIN_BLOCKS 6
+#define E3D_RV_MIN_BLOCKS 8
 #endif
 
-__device__ __forceinline__ double ldq(const double* __restrict__ P, int n, int c, int q) {
+template <class T>
+__device__ __forceinline__ T ldq(const T* __restrict__ P, int n, int c, int q) {
 	return q < 4 ? P[4 * (size_t)c + q] : P[4 * (size_t)n + c];
 }
-__device__ __forceinline__ void stq(double* __restrict__ P, int n, int c, int q, double x) {
+template <class T>
+__device__ __forceinline__ void stq(T* __restrict__ P, int n, int c, int q, T x) {
 	if (q < 4) P[4 * (size_t)c + q] = x;
 	else P[4 * (size_t)n + c] = x;
 }
 
-template <int GRAD, int LIM>
-__global__ void __launch_bounds__(5 * RV_CELLS, E3D_RV_MIN_BLOCKS) k_recon_var(FusedView<double> v, Physics ph) {
+template <class T, int GRAD, int LIM, int NSL>
+__global__ void __launch_bounds__(5 * RV_CELLS, E3D_RV_MIN_BLOCKS) k_recon_var(FusedView<T> v, Physics ph) {
 	const int c = blockIdx.x * RV_CELLS + threadIdx.x / 5, q = threadIdx.x % 5;
 	if (c >= v.NR) return;
-	const SlotRange<double, 4> sr(v, c);
-	const double q0 = ldq(v.Pin, v.NA, c, q);
-	int nb[4];
-	load_int<double, 4>(v.slot_nbr, sr, nb);
-	double gr[3] = {0.0, 0.0, 0.0};
-	double mx = q0, mn = q0;
+	const SlotRange<T, NSL> sr(v, c);
+	const T q0 = ldq(v.Pin, v.NA, c, q);
+	int nb[MAXSL];
+	if (NSL == 4) load_int<T, NSL>(v.slot_nbr, sr, nb);
+	T gr[3] = {T(0.0), T(0.0), T(0.0)};
+	T mx = q0, mn = q0;
 	{
-		const double* __restrict__ wa = (GRAD == GRAD_GREEN_GAUSS ? v.sS : v.lsw) + 3 * (size_t)sr.s0;
+		const T* __restrict__ wa = (GRAD == GRAD_GREEN_GAUSS ? v.sS : v.lsw) + 3 * (size_t)sr.s0;
 #pragma unroll
-		for (int k = 0; k < 4; k++) {
-			const double w[1][3] = {{__ldg(wa + 3 * k), __ldg(wa + 3 * k + 1), __ldg(wa + 3 * k + 2)}};
-			const double qn = ldq(v.Pin, v.NA, nb[k], q);
+		E3D_SLOTS(k, sr) {
+			if (NSL != 4) nb[k] = __ldg(v.slot_nbr + sr.s0 + k);
+			const T w[3] = {__ldg(wa + 3 * k), __ldg(wa + 3 * k + 1), __ldg(wa + 3 * k + 2)};
+			const T qn = ldq(v.Pin, v.NA, nb[k], q);
 			if (GRAD == GRAD_GREEN_GAUSS) {
-				const double a = 0.5 * (q0 + qn);
-				gr[0] += a * w[0][0];
-				gr[1] += a * w[0][1];
-				gr[2] += a * w[0][2];
+				const T a = T(0.5) * (q0 + qn);
+				gr[0] += a * w[0];
+				gr[1] += a * w[1];
+				gr[2] += a * w[2];
 			} else {
-				const double dq = qn - q0;
-				gr[0] += w[0][0] * dq;
-				gr[1] += w[0][1] * dq;
-				gr[2] += w[0][2] * dq;
+				const T dq = qn - q0;
+				gr[0] += w[0] * dq;
+				gr[1] += w[1] * dq;
+				gr[2] += w[2] * dq;
 			}
 			if (qn > mx) mx = qn;
 			if (qn < mn) mn = qn;
 		}
 	}
-	const double V = v.vol[c];
+	const T V = v.vol[c];
 	if (GRAD == GRAD_GREEN_GAUSS)
 		for (int d = 0; d < 3; d++) gr[d] /= V;
-	const double* __restrict__ ra = v.srv + 3 * (size_t)sr.s0;
-	const double eps2 = ph.k3 * V;
-	const double dmax = mx - q0, dmin = mn - q0;
-	double phi = INFINITY;
+	const T* __restrict__ ra = v.srv + 3 * (size_t)sr.s0;
+	const T eps2 = T(ph.k3) * V;
+	const T dmax = mx - q0, dmin = mn - q0;
+	CellLimiter<T, LIM> lim;
 #pragma unroll
-	for (int k = 0; k < 4; k++) {
-		double d2 = 0.0;
+	E3D_SLOTS(k, sr) {
+		T d2 = T(0.0);
 		d2 += gr[0] * __ldg(ra + 3 * k);
 		d2 += gr[1] * __ldg(ra + 3 * k + 1);
 		d2 += gr[2] * __ldg(ra + 3 * k + 2);
-		const double lf = (LIM == LIM_BARTH_JESPERSEN) ? limiter_bj_face(d2, dmax, dmin, ph.omega)
-		                                               : limiter_venkat_face(d2, dmax, dmin, eps2);
-		if (lf < phi) phi = lf;
+		lim.face(d2, dmax, dmin, T(ph.omega), eps2);
 	}
+	const T phi = lim.value(dmax, dmin);
 #pragma unroll
-	for (int k = 0; k < 4; k++)
-		stq(v.FS, v.NS, sr.s0 + k, q,
-		    recon(q0, phi, gr[0], gr[1], gr[2], __ldg(ra + 3 * k), __ldg(ra + 3 * k + 1), __ldg(ra + 3 * k + 2)));
+	E3D_SLOTS(k, sr)
+	stq(v.FS, v.NS, sr.s0 + k, q,
+	    recon(q0, phi, gr[0], gr[1], gr[2], __ldg(ra + 3 * k), __ldg(ra + 3 * k + 1), __ldg(ra + 3 * k + 2)));
 	// ghost cells of this cell's boundary faces (recon_cell's tail, one variable)
 #pragma unroll
-	for (int k = 0; k < 4; k++) {
+	E3D_SLOTS(k, sr) {
 		if (nb[k] < v.NR) continue;
 		const int g = nb[k];
 		int ms = v.slot_mate[sr.s0 + k];
 		ms = ms >= 0 ? ms : ~ms;
-		const double qg = ldq(v.Pin, v.NA, g, q);
-		const double* n = v.sgeo + 4 * (size_t)(sr.s0 + k);
-		const double g0 = v.srv[3 * (size_t)ms], g1 = v.srv[3 * (size_t)ms + 1], g2 = v.srv[3 * (size_t)ms + 2];
-		double gg[3] = {0.0, 0.0, 0.0};
+		const T qg = ldq(v.Pin, v.NA, g, q);
+		const T* n = v.sgeo + 4 * (size_t)(sr.s0 + k);
+		const T g0 = v.srv[3 * (size_t)ms], g1 = v.srv[3 * (size_t)ms + 1], g2 = v.srv[3 * (size_t)ms + 2];
+		T gg[3] = {T(0.0), T(0.0), T(0.0)};
 		if (v.grefl[g - v.NR] != 0) reflect_grad(gr, n[0], n[1], n[2], gg);
-		double gmx = qg, gmn = qg;
+		T gmx = qg, gmn = qg;
 		if (q0 > gmx) gmx = q0;
 		if (q0 < gmn) gmn = q0;
-		double d2 = 0.0;
+		T d2 = T(0.0);
 		d2 += gg[0] * g0;
 		d2 += gg[1] * g1;
 		d2 += gg[2] * g2;
-		const double dmx = gmx - qg, dmn = gmn - qg;
-		const double lf = (LIM == LIM_BARTH_JESPERSEN) ? limiter_bj_face(d2, dmx, dmn, ph.omega)
-		                                               : limiter_venkat_face(d2, dmx, dmn, ph.k3 * v.vol[g]);
-		double pg = INFINITY;
+		const T dmx = gmx - qg, dmn = gmn - qg;
+		const T lf = (LIM == LIM_BARTH_JESPERSEN) ? limiter_bj_face(d2, dmx, dmn, T(ph.omega))
+		                                          : limiter_venkat_face(d2, dmx, dmn, T(ph.k3) * v.vol[g]);
+		T pg = T(INFINITY);
 		if (lf < pg) pg = lf;
 		stq(v.FS, v.NS, ms, q, recon(qg, pg, gg[0], gg[1], gg[2], g0, g1, g2));
 	}

@@ -27,27 +27,25 @@ void launch_tail(const ReduceArgs& a, const T* Rc, const T* Rd, T* P, T* P2, cud
 	k_tail<T><<<grid, TAIL_TPB, 0, st>>>(a, Rc, Rd, P, P2);
 }
 
-// FP64 later stages on tetrahedra: one lane per (cell, variable)
-// (k_recon_var); build with -DE3D_FP64_RECON_VAR=0 for the one-thread-per-cell pass
-#ifndef E3D_FP64_RECON_VAR
-#define E3D_FP64_RECON_VAR 1
-#endif
+template <class T>
+void launch_start(const FusedView<T>& v, const Physics& ph, int carry, cudaStream_t st) {
+	if (v.NR <= 0) return;
+	if (v.tet4) k_start<T, 4><<<(v.NR + 127) / 128, 128, 0, st>>>(v, ph, carry);
+	else k_start<T, 0><<<(v.NR + 127) / 128, 128, 0, st>>>(v, ph, carry);
+}
+
+// Which pass reconstructs: see k_recon_var.
 template <class T, int GRAD, int LIM>
 void recon_dispatch_first(const FusedView<T>& v, const Physics& ph, bool first, int carry, cudaStream_t st) {
-	const int grid = (v.NR + 127) / 128;
-	if constexpr (sizeof(T) == 8 && E3D_FP64_RECON_VAR) {
-		if (v.tet4 && !first) {
-			k_recon_var<GRAD, LIM><<<(v.NR + RV_CELLS - 1) / RV_CELLS, 5 * RV_CELLS, 0, st>>>(v, ph);
-			return;
-		}
+	const int grid = (v.NR + 127) / 128, gv = (v.NR + RV_CELLS - 1) / RV_CELLS;
+	if (!v.tet4) {
+		if (first) launch_start<T>(v, ph, carry, st);
+		k_recon_var<T, GRAD, LIM, 0><<<gv, 5 * RV_CELLS, 0, st>>>(v, ph);
+		return;
 	}
-	if (v.tet4) {
-		if (first) k_recon<T, GRAD, LIM, true, 4><<<grid, 128, 0, st>>>(v, ph, carry);
-		else k_recon<T, GRAD, LIM, false, 4><<<grid, 128, 0, st>>>(v, ph, carry);
-	} else {
-		if (first) k_recon<T, GRAD, LIM, true, 0><<<grid, 128, 0, st>>>(v, ph, carry);
-		else k_recon<T, GRAD, LIM, false, 0><<<grid, 128, 0, st>>>(v, ph, carry);
-	}
+	if (first) k_recon<T, GRAD, LIM, true, 4><<<grid, 128, 0, st>>>(v, ph, carry);
+	else if constexpr (sizeof(T) == 8) k_recon_var<T, GRAD, LIM, 4><<<gv, 5 * RV_CELLS, 0, st>>>(v, ph);
+	else k_recon<T, GRAD, LIM, false, 4><<<grid, 128, 0, st>>>(v, ph, carry);
 }
 
 template <class T>
@@ -64,13 +62,6 @@ void launch_recon(const FusedView<T>& v, const Physics& ph, int grad, int lim, b
 		else
 			recon_dispatch_first<T, GRAD_GREEN_GAUSS, LIM_BARTH_JESPERSEN>(v, ph, first, carry, st);
 	}
-}
-
-template <class T>
-void launch_start(const FusedView<T>& v, const Physics& ph, int carry, cudaStream_t st) {
-	if (v.NR <= 0) return;
-	if (v.tet4) k_start<T, 4><<<(v.NR + 127) / 128, 128, 0, st>>>(v, ph, carry);
-	else k_start<T, 0><<<(v.NR + 127) / 128, 128, 0, st>>>(v, ph, carry);
 }
 
 // Largest mesh (tetrahedra; half of it for 8 lanes per cell) whose FP64 flux

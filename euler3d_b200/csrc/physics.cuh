@@ -206,12 +206,45 @@ __device__ __forceinline__ T limiter_bj_face(T d2, T dmax, T dmin, T omega) {
 	return T(1.0);
 }
 
+template <class T>
+__device__ __forceinline__ T limiter_venkat_face(T d2, T dmax, T dmin, T eps2);
+template <>
+__device__ __forceinline__ float limiter_venkat_face<float>(float d2, float dmax, float dmin, float eps2);
+template <>
+__device__ __forceinline__ double limiter_venkat_face<double>(double d2, double dmax, double dmin, double eps2);
+
+// The smallest face limiter of a cell with one or two divisions instead of one
+// per face.  Barth-Jespersen: a face's value is min(1, dmax/d2) for d2 > 0 and
+// min(1, dmin/d2) for d2 < 0, with dmax >= 0 >= dmin.  Division rounds
+// monotonically, so the smallest value is the one of the largest d2 or of the
+// most negative one, bit for bit in IEEE arithmetic (a NaN d2 counts as 1, as
+// in the branches above).  Venkatakrishnan's values are compared one by one.
+template <class T, int LIM>
+struct CellLimiter {
+	T pos = T(0.0), neg = T(0.0), phi = LIM == 0 ? T(1.0) : T(INFINITY);
+	__device__ __forceinline__ void face(T d2, T dmax, T dmin, T omega, T eps2) {
+		if (LIM == 0) {
+			d2 = (tcopysign(T(1.0), d2)) * (tabs(d2) + omega);
+			if (d2 > pos) pos = d2;
+			if (d2 < neg) neg = d2;
+		} else {
+			const T lf = limiter_venkat_face(d2, dmax, dmin, eps2);
+			if (lf < phi) phi = lf;
+		}
+	}
+	__device__ __forceinline__ T value(T dmax, T dmin) const {
+		if (LIM != 0) return phi;
+		T x = T(1.0);
+		if (pos > T(0.0)) x = tmin(x, dmax / pos);
+		if (neg < T(0.0)) x = tmin(x, dmin / neg);
+		return x;
+	}
+};
+
 // Venkatakrishnan face limiter, eps2 = K^3 * V (Venkatakrishnan.cpp:92,227-238).
 // The double version keeps the reference's expression (two divisions); the
 // float version uses the same function with d2 cancelled from numerator and
 // denominator, (D^2+eps2+2 d2 D) / (D^2+eps2 + d2 (2 d2 + D)), one division.
-template <class T>
-__device__ __forceinline__ T limiter_venkat_face(T d2, T dmax, T dmin, T eps2);
 template <>
 __device__ __forceinline__ float limiter_venkat_face<float>(float d2, float dmax, float dmin, float eps2) {
 	if (!(d2 > 0.0f) && !(d2 < 0.0f)) return 1.0f;  // zero or NaN, as the reference's branches

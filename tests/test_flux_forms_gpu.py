@@ -1,4 +1,4 @@
-"""The flux pass's two forms (one lane per slot, one thread per cell) on both sides of the size where they change."""
+"""Stage passes against the oracle at the sizes where their forms change and where their last blocks are partly filled."""
 import os
 
 import numpy as np
@@ -19,8 +19,21 @@ pytestmark = pytest.mark.gpu
 def test_matches_oracle(mesh, n, nz, flux, order, tmp_path):
     deck = mg.Deck(topology="", mach=0.7, aoa_deg=2.0, flux=flux, order=order)
     path = mg.write_hex_case(str(tmp_path), n, nz, deck=deck) if mesh == "hex" else mg.write_case(str(tmp_path), n, deck=deck)
+    _check(path, deck, str(tmp_path))
+
+
+# hexahedra, one lane per (cell, variable): 32 cells fill a block exactly, 99 leave the fourth with 3
+@pytest.mark.parametrize("n,nz", [(4, 2), (3, 11)])
+@pytest.mark.parametrize("gradient", ["greengauss", "leastsquares"])
+@pytest.mark.parametrize("limiter", ["barthjespersen", "venkatakrishnan"])
+def test_hex_reconstruction(n, nz, gradient, limiter, tmp_path):
+    deck = mg.Deck(topology="", mach=0.7, aoa_deg=2.0, flux="ausm", order=2, gradient=gradient, limiter=limiter)
+    _check(mg.write_hex_case(str(tmp_path), n, nz, deck=deck), deck, str(tmp_path))
+
+
+def _check(path, deck, directory):
     case = api.Case(path)
-    ref = case_oracle(case, os.path.join(str(tmp_path), deck.topology))
+    ref = case_oracle(case, os.path.join(directory, deck.topology))
     s = api.Solver(case)
     ref.iterate(2)
     s.iterate(2)
