@@ -1,12 +1,20 @@
 // Warm-start surrogate: training and inference kernels (see surrogate.hpp).
 //
-// The 128-wide layers run as one templated tensor-core GEMM, C = A * B^T
-// with BF16 operands staged in shared memory and FP32 accumulators
-// (mma.sync m16n8k16), and a per-use epilogue: bias + GELU (forward), times
-// GELU'(z) (backward data), or an FP32 partial of a split-K slice (weight
-// gradients, summed over slices in a fixed order).  The 5-wide output layer
-// runs on the CUDA cores.  No floating-point atomics anywhere: every sum is
-// a fixed-order loop or tree, so a training run is reproducible bit for bit.
+// A training step is three launches.  k_mlp takes tiles of 64 rows through the
+// whole network and back: the weights stay in shared memory, the activations
+// of a tile never leave the SM between layers, GELU'(z) stays in registers from
+// the forward to the backward pass (one erf for both), and only the BF16
+// activations and gradients that the weight gradients need are written out.
+// k_wgrad forms dW = g^T a over slices of rows, k_update adds up the partials in
+// a fixed order and applies Adam.  Inference is k_mlp's forward half alone.
+// All GEMMs are mma.sync m16n8k16 with BF16 operands and FP32 accumulators, k
+// ascending.  Per row the step is 0.2 MFLOP of GEMM but 384 erf and 384 exp, so
+// the CUDA cores, not the tensor cores, bound it.  No floating-point atomics
+// anywhere: every sum is a fixed-order loop or tree, so a training run is
+// reproducible bit for bit.
+// B200: a 16,384-row step took 334 us as 25 launches with every activation in
+// global memory; 65 us in this form.  A 384k-row forward pass: 940 us in 5
+// launches; 335 us in one.
 #include <cuda_bf16.h>
 
 #include <algorithm>
@@ -30,11 +38,6 @@ __device__ __forceinline__ uint16_t f2bf(float x) {
 }
 __device__ __forceinline__ float bf2f(uint16_t u) { return __uint_as_float(((uint32_t)u) << 16); }
 
-__device__ __forceinline__ float gelu(float z) { return 0.5f * z * (1.f + erff(z * 0.70710678118654752f)); }
-__device__ __forceinline__ float gelu_d(float z) {
-	return 0.5f * (1.f + erff(z * 0.70710678118654752f)) + z * 0.39894228040143268f * expf(-0.5f * z * z);
-}
-
 __host__ __device__ __forceinline__ uint64_t mix64(uint64_t x) {
 	// splitmix64 finaliser
 	x += 0x9E3779B97F4A7C15ull;
@@ -56,273 +59,453 @@ __device__ __forceinline__ void wfree(float mach, float aoa_deg, float gamma, fl
 	w[4] = 0.5f * (u * u + v * v) + 1.f / (gamma - 1.f);
 }
 
-// ------------------------------------------------------------------ GEMM
-enum { L_ROW = 0, L_COL = 1 };
-enum { EPI_FWD_GELU = 0, EPI_BWD_GELU = 1, EPI_PARTIAL = 2 };
-
-struct Epi {
-	const float* bias;  // EPI_FWD_GELU
-	float* zout;        // EPI_FWD_GELU: pre-activation [M][ldo]
-	uint16_t* hout;     // EPI_FWD_GELU: GELU(z) BF16; EPI_BWD_GELU: g BF16 [M][ldo]
-	const float* zin;   // EPI_BWD_GELU: pre-activation of the layer below [M][ldo]
-	float* part;        // EPI_PARTIAL: [slices][M][N]
-	int ldo;
-};
-
-constexpr int BM = 64, BN = 64, BK = 32, SPAD = 8;
-
-__device__ __forceinline__ uint32_t ld32(const uint16_t* p) { return *reinterpret_cast<const uint32_t*>(p); }
-
-__device__ __forceinline__ void mma_bf16(float c[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
-                                         uint32_t b1) {
+// ------------------------------------------------------------------ tensor-core fragments
+__device__ __forceinline__ void mma_bf16(float c[4], const uint32_t a[4], uint32_t b0, uint32_t b1) {
 	asm volatile(
 	    "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
 	    "{%0,%1,%2,%3};\n"
 	    : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-	    : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+	    : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+template <bool TRANS>
+__device__ __forceinline__ void ldsm4(uint32_t r[4], const uint16_t* p) {
+	const uint32_t a = (uint32_t)__cvta_generic_to_shared(p);
+	if (TRANS)
+		asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n"
+		             : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+		             : "r"(a));
+	else
+		asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];\n"
+		             : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+		             : "r"(a));
 }
 
-// C[m][n] = sum_k A(m,k) B(n,k);  A(m,k) = A[m*lda+k] (L_ROW) or A[k*lda+m] (L_COL),
-// B(n,k) = B[n*ldb+k] (L_ROW) or B[k*ldb+n] (L_COL).  blockIdx.z = split-K slice.
-template <int AL, int BL, int EPI>
-__global__ void __launch_bounds__(128) k_gemm(int M, int N, int K, const uint16_t* __restrict__ A, int lda,
-                                              const uint16_t* __restrict__ B, int ldb, int k_slice, Epi ep) {
-	__shared__ __align__(16) uint16_t As[BM][BK + SPAD];
-	__shared__ __align__(16) uint16_t Bs[BN][BK + SPAD];
-	const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-	const int g = lane >> 2, t = lane & 3;
-	const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
-	const int kb = blockIdx.z * k_slice, ke = min(K, kb + k_slice);
-	const int wm = (warp >> 1) * 32, wn = (warp & 1) * 32;
-	float acc[2][4][4];
-#pragma unroll
-	for (int i = 0; i < 2; i++)
-#pragma unroll
-		for (int j = 0; j < 4; j++)
-#pragma unroll
-			for (int r = 0; r < 4; r++) acc[i][j][r] = 0.f;
+constexpr int TR = 64;         // rows of a tile
+constexpr int MLP_TPB = 512;   // 16 warps: 4 (16 rows) x 4 (32 columns) of a 64 x 128 layer
+constexpr int LDH = H + 8;     // shared rows of 128 BF16 values, padded: 8 rows of a matrix hit 32 banks
+constexpr int LDX = S::IN + 8;
+// per-block sums of the output layer and the biases: W4, b4, b3, b2, b1
+constexpr int PA_B4 = S::OUT * H, PA_B3 = PA_B4 + S::OUT, PA_B2 = PA_B3 + H, PA_B1 = PA_B2 + H, PA_N = PA_B1 + H;
 
-	for (int k0 = kb; k0 < ke; k0 += BK) {
-#pragma unroll 4
-		for (int e = 0; e < (BM * BK) / 128; e++) {
-			const int idx = e * 128 + tid;
-			int m, k;
-			if (AL == L_ROW) {
-				m = idx / BK;
-				k = idx % BK;
-			} else {
-				m = idx % BM;
-				k = idx / BM;
-			}
-			const int gm = m0 + m, gk = k0 + k;
-			uint16_t v = 0;
-			if (gm < M && gk < ke) v = AL == L_ROW ? A[(size_t)gm * lda + gk] : A[(size_t)gk * lda + gm];
-			As[m][k] = v;
-		}
-#pragma unroll 4
-		for (int e = 0; e < (BN * BK) / 128; e++) {
-			const int idx = e * 128 + tid;
-			int n, k;
-			if (BL == L_ROW) {
-				n = idx / BK;
-				k = idx % BK;
-			} else {
-				n = idx % BN;
-				k = idx / BN;
-			}
-			const int gn = n0 + n, gk = k0 + k;
-			uint16_t v = 0;
-			if (gn < N && gk < ke) v = BL == L_ROW ? B[(size_t)gn * ldb + gk] : B[(size_t)gk * ldb + gn];
-			Bs[n][k] = v;
-		}
-		__syncthreads();
+struct MlpShared {
+	uint16_t w1[H][LDX], w2[H][LDH], w3[H][LDH];
+	uint16_t x[TR][LDX], a1[TR][LDH], a2[TR][LDH], a3[TR][LDH], g2[TR][LDH];
+	float w4[H][12];  // W4 transposed: the 5 outputs' weights of one input, padded against bank conflicts
+	float b1[H], b2[H], b3[H], b4[S::OUT], norm[S::N_NORM];
+	float t[TR][S::OUT], d4[TR][S::OUT];  // targets (inference: freestream state), dL/dy
+	float red[PA_N];
+	float loss[MLP_TPB / 32];
+};
+
+// One warp's 16 x 32 part of (64 x K) * (K x 128); B row-major [n][k] or, BT, [k][n].
+template <int K, int LDA, int LDB, bool BT>
+__device__ __forceinline__ void warp_gemm(float acc[4][4], const uint16_t (*A)[LDA], const uint16_t (*B)[LDB], int m0,
+                                          int n0) {
+	const int lane = threadIdx.x & 31, r = lane & 7, id = lane >> 3;
 #pragma unroll
-		for (int ks = 0; ks < BK; ks += 16) {
-			uint32_t a[2][4], b[4][2];
+	for (int j = 0; j < 4; j++)
 #pragma unroll
-			for (int i = 0; i < 2; i++) {
-				const int r = wm + 16 * i + g;
-				a[i][0] = ld32(&As[r][ks + 2 * t]);
-				a[i][1] = ld32(&As[r + 8][ks + 2 * t]);
-				a[i][2] = ld32(&As[r][ks + 2 * t + 8]);
-				a[i][3] = ld32(&As[r + 8][ks + 2 * t + 8]);
-			}
+		for (int i = 0; i < 4; i++) acc[j][i] = 0.f;
 #pragma unroll
-			for (int j = 0; j < 4; j++) {
-				const int c = wn + 8 * j + g;
-				b[j][0] = ld32(&Bs[c][ks + 2 * t]);
-				b[j][1] = ld32(&Bs[c][ks + 2 * t + 8]);
-			}
+	for (int k0 = 0; k0 < K; k0 += 16) {
+		uint32_t a[4], b[2][4];
+		ldsm4<false>(a, &A[m0 + r + (id & 1) * 8][k0 + (id >> 1) * 8]);
 #pragma unroll
-			for (int i = 0; i < 2; i++)
+		for (int h = 0; h < 2; h++)
+			if (BT) ldsm4<true>(b[h], &B[k0 + r + (id & 1) * 8][n0 + 16 * h + (id >> 1) * 8]);
+			else ldsm4<false>(b[h], &B[n0 + 16 * h + r + (id >> 1) * 8][k0 + (id & 1) * 8]);
 #pragma unroll
-				for (int j = 0; j < 4; j++) mma_bf16(acc[i][j], a[i][0], a[i][1], a[i][2], a[i][3], b[j][0], b[j][1]);
-		}
-		__syncthreads();
+		for (int j = 0; j < 4; j++) mma_bf16(acc[j], a, b[j >> 1][2 * (j & 1)], b[j >> 1][2 * (j & 1) + 1]);
 	}
-	// epilogue: acc[i][j] = rows (g, g+8) x cols (2t, 2t+1) of the 16x8 tile
+}
+__device__ __forceinline__ uint32_t pack2(float a, float b) { return (uint32_t)f2bf(a) | ((uint32_t)f2bf(b) << 16); }
+
+// z = acc + bias, h = GELU(z) to shared memory; gd = GELU'(z) kept by the thread
+template <bool TRAIN>
+__device__ __forceinline__ void gelu_layer(const float acc[4][4], const float* bias, uint16_t (*out)[LDH], float gd[4][4],
+                                           int m0, int n0) {
+	const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
 #pragma unroll
-	for (int i = 0; i < 2; i++)
+	for (int j = 0; j < 4; j++) {
+		const int n = n0 + 8 * j + 2 * t;
+		float h[4];
 #pragma unroll
-		for (int j = 0; j < 4; j++)
+		for (int i = 0; i < 4; i++) {
+			const float z = acc[j][i] + bias[n + (i & 1)];
+			const float e = 1.f + erff(z * 0.70710678118654752f);
+			h[i] = 0.5f * z * e;
+			if (TRAIN) gd[j][i] = 0.5f * e + z * 0.39894228040143268f * expf(-0.5f * z * z);
+		}
+		*reinterpret_cast<uint32_t*>(&out[m0 + g][n]) = pack2(h[0], h[1]);
+		*reinterpret_cast<uint32_t*>(&out[m0 + g + 8][n]) = pack2(h[2], h[3]);
+	}
+}
+__device__ __forceinline__ void store_grad(const float acc[4][4], const float gd[4][4], uint16_t (*out)[LDH], int m0, int n0) {
+	const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
 #pragma unroll
-			for (int r = 0; r < 4; r++) {
-				const int m = m0 + wm + 16 * i + g + (r >= 2 ? 8 : 0);
-				const int n = n0 + wn + 8 * j + 2 * t + (r & 1);
-				if (m >= M || n >= N) continue;
-				const float v = acc[i][j][r];
-				if (EPI == EPI_FWD_GELU) {
-					const float z = v + ep.bias[n];
-					ep.zout[(size_t)m * ep.ldo + n] = z;
-					ep.hout[(size_t)m * ep.ldo + n] = f2bf(gelu(z));
-				} else if (EPI == EPI_BWD_GELU) {
-					ep.hout[(size_t)m * ep.ldo + n] = f2bf(v * gelu_d(ep.zin[(size_t)m * ep.ldo + n]));
-				} else {
-					ep.part[((size_t)blockIdx.z * M + m) * N + n] = v;
+	for (int j = 0; j < 4; j++) {
+		const int n = n0 + 8 * j + 2 * t;
+		*reinterpret_cast<uint32_t*>(&out[m0 + g][n]) = pack2(acc[j][0] * gd[j][0], acc[j][1] * gd[j][1]);
+		*reinterpret_cast<uint32_t*>(&out[m0 + g + 8][n]) = pack2(acc[j][2] * gd[j][2], acc[j][3] * gd[j][3]);
+	}
+}
+// a tile's first `rows` rows of 128 values to global memory
+__device__ __forceinline__ void copy_rows(const uint16_t (*src)[LDH], uint16_t* __restrict__ dst, int rows) {
+	for (int i = threadIdx.x; i < TR * (H / 8); i += MLP_TPB) {
+		const int r = i / (H / 8), c = i % (H / 8);
+		if (r < rows) reinterpret_cast<uint4*>(dst)[(size_t)r * (H / 8) + c] = *reinterpret_cast<const uint4*>(&src[r][8 * c]);
+	}
+}
+// 5 values of a 16-byte-aligned row
+__device__ __forceinline__ void load5(const float* p, float o[S::N_OUT]) {
+	const float4 v = *reinterpret_cast<const float4*>(p);
+	o[0] = v.x;
+	o[1] = v.y;
+	o[2] = v.z;
+	o[3] = v.w;
+	o[4] = p[4];
+}
+__device__ __forceinline__ float colsum16(const uint16_t (*g)[LDH], int r0, int j) {
+	float s = 0.f;
+#pragma unroll
+	for (int r = 0; r < 16; r++) s += bf2f(g[r0 + r][j]);
+	return s;
+}
+
+struct MlpArgs {
+	int n;                // rows
+	const float* feat;    // [.][8] raw features
+	const float* state;   // [.][8] conservative states (training)
+	long long n_store;    // > 0: row i is a hashed draw from n_store samples; 0: row i
+	uint64_t seed;
+	long long step;
+	const float* norm;
+	float gamma;
+	const float* master;  // FP32 parameters (biases)
+	const uint16_t* wb;   // BF16 weights
+	uint16_t *x, *a1, *a2, *g1, *g2, *g3;  // training: operands of the weight gradients
+	float* part;          // training: [block][PA_N]
+	float* lossp;         // training: [block] squared-error sums
+	float* out;           // inference: [n][8] conservative states
+};
+
+// The network forward, and with TRAIN back to the first layer, over tiles of TR
+// rows.  One block per SM (163 KB of shared memory), weights loaded once.
+template <bool TRAIN>
+__global__ void __launch_bounds__(MLP_TPB, 1) k_mlp(MlpArgs p) {
+	extern __shared__ __align__(16) unsigned char dyn[];
+	MlpShared& s = *reinterpret_cast<MlpShared*>(dyn);
+	const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+	const int m0 = (warp & 3) * 16, n0 = (warp >> 2) * 32;
+	for (int i = t; i < H * S::IN / 8; i += MLP_TPB)
+		*reinterpret_cast<uint4*>(&s.w1[i / 2][8 * (i % 2)]) = reinterpret_cast<const uint4*>(p.wb + S::OFF_W1)[i];
+	for (int i = t; i < H * H / 8; i += MLP_TPB) {
+		*reinterpret_cast<uint4*>(&s.w2[i / 16][8 * (i % 16)]) = reinterpret_cast<const uint4*>(p.wb + S::OFF_W2)[i];
+		*reinterpret_cast<uint4*>(&s.w3[i / 16][8 * (i % 16)]) = reinterpret_cast<const uint4*>(p.wb + S::OFF_W3)[i];
+	}
+	for (int i = t; i < S::N_OUT * H; i += MLP_TPB) s.w4[i % H][i / H] = bf2f(p.wb[S::OFF_W4 + i]);
+	if (t < H) {
+		s.b1[t] = p.master[S::OFF_B1 + t];
+		s.b2[t] = p.master[S::OFF_B2 + t];
+		s.b3[t] = p.master[S::OFF_B3 + t];
+	}
+	if (t < S::OUT) s.b4[t] = p.master[S::OFF_B4 + t];
+	if (t < S::N_NORM) s.norm[t] = p.norm[t];
+	__syncthreads();
+	const int row8 = t >> 3, j8 = t & 7;          // 8 lanes per row: inputs, outputs
+	const int col = t & (H - 1), r16 = (t >> 7) * 16;  // 16 rows of one column: sums over rows
+	float se = 0.f, w4sum[S::N_OUT] = {0.f, 0.f, 0.f, 0.f, 0.f}, b4sum = 0.f, b3sum = 0.f, b2sum = 0.f, b1sum = 0.f;
+	const int n_tiles = (p.n + TR - 1) / TR;
+	for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
+		const int i0 = tile * TR, rows = min(TR, p.n - i0);
+		const bool valid = row8 < rows;
+		{  // standardised features, scaled targets
+			const long long i = i0 + (valid ? row8 : 0);
+			long long src = i;
+			if (p.n_store > 0)
+				src = (long long)(mix64(p.seed ^ mix64((uint64_t)p.step * 0x100000001B3ull + (uint64_t)i)) %
+				                  (uint64_t)p.n_store);
+			const float f = p.feat[(size_t)src * 8 + j8];
+			const uint16_t xv = valid && j8 < S::N_IN ? f2bf((f - s.norm[j8]) / s.norm[8 + j8]) : (uint16_t)0;
+			s.x[row8][j8] = xv;
+			s.x[row8][8 + j8] = 0;
+			const float mach = __shfl_sync(0xffffffffu, f, (lane & 24) + 4), aoa = __shfl_sync(0xffffffffu, f, (lane & 24) + 5);
+			float wf[5];
+			wfree(mach, aoa, p.gamma, wf);
+			const float w = j8 == 0 ? wf[0] : j8 == 1 ? wf[1] : j8 == 2 ? wf[2] : j8 == 3 ? wf[3] : wf[4];
+			if (TRAIN) {
+				if (valid) {
+					p.x[(size_t)i * S::IN + j8] = xv;
+					p.x[(size_t)i * S::IN + 8 + j8] = 0;
 				}
+				s.t[row8][j8] = j8 < S::N_OUT ? (p.state[(size_t)src * 8 + j8] - w) / s.norm[16 + j8] : 0.f;
+			} else {
+				s.t[row8][j8] = w;
 			}
-}
-
-template <int AL, int BL, int EPI>
-void gemm(int M, int N, int K, const uint16_t* A, int lda, const uint16_t* B, int ldb, int slices, const Epi& ep,
-          cudaStream_t st) {
-	const int ks = ((K + slices - 1) / slices + BK - 1) / BK * BK;
-	const int sl = (K + ks - 1) / ks;
-	dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM, sl);
-	k_gemm<AL, BL, EPI><<<grid, 128, 0, st>>>(M, N, K, A, lda, B, ldb, ks, ep);
-}
-
-// ------------------------------------------------------------------ small kernels
-// minibatch rows: standardised features (BF16, [n][IN]) and scaled targets ([n][OUT])
-__global__ void k_prepare(int n, const float* __restrict__ feat, int ldf, const float* __restrict__ state, int lds,
-                          long long n_store, uint64_t seed, long long step, const float* __restrict__ norm, float gamma,
-                          uint16_t* __restrict__ x, float* __restrict__ tgt) {
-	const int i = blockIdx.x * blockDim.x + threadIdx.x;
-	if (i >= n) return;
-	long long src = i;
-	if (n_store > 0) src = (long long)(mix64(seed ^ mix64((uint64_t)step * 0x100000001B3ull + (uint64_t)i)) %
-	                                   (uint64_t)n_store);
-	const float* f = feat + (size_t)src * ldf;
-	for (int j = 0; j < S::IN; j++)
-		x[(size_t)i * S::IN + j] = j < S::N_IN ? f2bf((f[j] - norm[j]) / norm[8 + j]) : (uint16_t)0;
-	if (tgt) {
-		float wf[5];
-		wfree(f[4], f[5], gamma, wf);
-		const float* s = state + (size_t)src * lds;
-		for (int q = 0; q < S::OUT; q++) tgt[(size_t)i * S::OUT + q] = q < S::N_OUT ? (s[q] - wf[q]) / norm[16 + q] : 0.f;
-	}
-}
-
-// output layer on the CUDA cores: y[b][q] = b4[q] + sum_j W4[q][j] a3[b][j]
-__global__ void k_out_layer(int n, const uint16_t* __restrict__ a3, const uint16_t* __restrict__ w4,
-                            const float* __restrict__ b4, float* __restrict__ y) {
-	__shared__ float w[S::N_OUT][H];
-	for (int i = threadIdx.x; i < S::N_OUT * H; i += blockDim.x) w[i / H][i % H] = bf2f(w4[i]);
-	__syncthreads();
-	const int b = blockIdx.x * blockDim.x + threadIdx.x;
-	if (b >= n) return;
-	float acc[S::N_OUT];
-	for (int q = 0; q < S::N_OUT; q++) acc[q] = 0.f;
-	const uint16_t* a = a3 + (size_t)b * H;
-	for (int j = 0; j < H; j += 2) {
-		const uint32_t p = *reinterpret_cast<const uint32_t*>(a + j);
-		const float x0 = bf2f((uint16_t)(p & 0xFFFFu)), x1 = bf2f((uint16_t)(p >> 16));
-		for (int q = 0; q < S::N_OUT; q++) acc[q] += w[q][j] * x0 + w[q][j + 1] * x1;
-	}
-	for (int q = 0; q < S::OUT; q++) y[(size_t)b * S::OUT + q] = q < S::N_OUT ? acc[q] + b4[q] : 0.f;
-}
-
-// d4 = dL/dy for L = mean over rows and the 5 outputs of (y - t)^2; per-block squared-error sums
-__global__ void k_loss(int n, const float* __restrict__ y, const float* __restrict__ t, float* __restrict__ d4,
-                       float* __restrict__ lossp) {
-	__shared__ float red[256];
-	const int b = blockIdx.x * blockDim.x + threadIdx.x;
-	float se = 0.f;
-	if (b < n)
-		for (int q = 0; q < S::OUT; q++) {
-			const float e = q < S::N_OUT ? y[(size_t)b * S::OUT + q] - t[(size_t)b * S::OUT + q] : 0.f;
-			d4[(size_t)b * S::OUT + q] = 2.f * e / (float)(n * S::N_OUT);
-			se += e * e;
 		}
-	red[threadIdx.x] = se;
+		__syncthreads();
+		float acc[4][4], gd1[4][4], gd2[4][4], gd3[4][4];
+		warp_gemm<S::IN, LDX, LDX, false>(acc, s.x, s.w1, m0, n0);
+		gelu_layer<TRAIN>(acc, s.b1, s.a1, gd1, m0, n0);
+		__syncthreads();
+		warp_gemm<H, LDH, LDH, false>(acc, s.a1, s.w2, m0, n0);
+		gelu_layer<TRAIN>(acc, s.b2, s.a2, gd2, m0, n0);
+		__syncthreads();
+		warp_gemm<H, LDH, LDH, false>(acc, s.a2, s.w3, m0, n0);
+		gelu_layer<TRAIN>(acc, s.b3, s.a3, gd3, m0, n0);
+		__syncthreads();
+		{  // output layer: each of a row's 8 lanes takes 16 of the 128 inputs
+			float y[S::N_OUT] = {0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+			for (int k = 0; k < 16; k += 2) {
+				const int j = 16 * j8 + ((k + 2 * j8) & 15);  // staggered: the lanes' reads spread over the banks
+				const uint32_t v = *reinterpret_cast<const uint32_t*>(&s.a3[row8][j]);
+				const float x0 = bf2f((uint16_t)(v & 0xFFFFu)), x1 = bf2f((uint16_t)(v >> 16));
+				float wa[S::N_OUT], wc[S::N_OUT];
+				load5(s.w4[j], wa);
+				load5(s.w4[j + 1], wc);
+#pragma unroll
+				for (int q = 0; q < S::N_OUT; q++) y[q] += wa[q] * x0 + wc[q] * x1;
+			}
+#pragma unroll
+			for (int q = 0; q < S::N_OUT; q++)
+				for (int h = 4; h > 0; h >>= 1) y[q] += __shfl_xor_sync(0xffffffffu, y[q], h);
+			const float yq = (j8 == 0 ? y[0] : j8 == 1 ? y[1] : j8 == 2 ? y[2] : j8 == 3 ? y[3] : y[4]) + s.b4[j8];
+			if (TRAIN) {
+				const float e = valid && j8 < S::N_OUT ? yq - s.t[row8][j8] : 0.f;
+				s.d4[row8][j8] = 2.f * e / (float)(p.n * S::N_OUT);
+				se += e * e;
+			} else if (valid) {
+				p.out[(size_t)(i0 + row8) * 8 + j8] = j8 < S::N_OUT ? s.t[row8][j8] + s.norm[16 + j8] * yq : 0.f;
+			}
+		}
+		if (!TRAIN) continue;  // the next tile's first write to a3 is behind three barriers
+		__syncthreads();
+#pragma unroll
+		for (int r = 0; r < 16; r++) {
+			const float a = bf2f(s.a3[r16 + r][col]);
+			float d[S::N_OUT];
+			load5(s.d4[r16 + r], d);
+#pragma unroll
+			for (int q = 0; q < S::N_OUT; q++) w4sum[q] += d[q] * a;
+			if (col < S::OUT) b4sum += s.d4[r16 + r][col];
+		}
+		{  // g3 = GELU'(z3) * (d4 W4)
+			const int g = lane >> 2, c2 = 2 * (lane & 3);
+			float da[S::N_OUT], db[S::N_OUT];
+			load5(s.d4[m0 + g], da);
+			load5(s.d4[m0 + g + 8], db);
+#pragma unroll
+			for (int j = 0; j < 4; j++)
+#pragma unroll
+				for (int i = 0; i < 2; i++) {
+					float w[S::N_OUT], u = 0.f, v = 0.f;
+					load5(s.w4[n0 + 8 * j + c2 + i], w);
+#pragma unroll
+					for (int q = 0; q < S::N_OUT; q++) {
+						u += da[q] * w[q];
+						v += db[q] * w[q];
+					}
+					acc[j][i] = u;
+					acc[j][2 + i] = v;
+				}
+		}
+		__syncthreads();
+		store_grad(acc, gd3, s.a3, m0, n0);  // a3 is read no more: it holds g3 from here
+		__syncthreads();
+		copy_rows(s.a3, p.g3 + (size_t)i0 * H, rows);
+		b3sum += colsum16(s.a3, r16, col);
+		warp_gemm<H, LDH, LDH, true>(acc, s.a3, s.w3, m0, n0);
+		store_grad(acc, gd2, s.g2, m0, n0);
+		__syncthreads();
+		copy_rows(s.g2, p.g2 + (size_t)i0 * H, rows);
+		b2sum += colsum16(s.g2, r16, col);
+		warp_gemm<H, LDH, LDH, true>(acc, s.g2, s.w2, m0, n0);
+		store_grad(acc, gd1, s.a3, m0, n0);  // g1
+		__syncthreads();
+		copy_rows(s.a3, p.g1 + (size_t)i0 * H, rows);
+		copy_rows(s.a1, p.a1 + (size_t)i0 * H, rows);
+		copy_rows(s.a2, p.a2 + (size_t)i0 * H, rows);
+		b1sum += colsum16(s.a3, r16, col);
+	}
+	if (!TRAIN) return;
+	// the four row groups' sums in order, then the block's squared error
+	for (int grp = 0; grp < 4; grp++) {
+		__syncthreads();
+		if ((t >> 7) == grp) {
+			const bool z = grp == 0;
+#pragma unroll
+			for (int q = 0; q < S::OUT; q++) {
+				float& r = s.red[q * H + col];
+				const float v = q < S::N_OUT ? w4sum[q < S::N_OUT ? q : 0] : 0.f;
+				r = z ? v : r + v;
+			}
+			if (col < S::OUT) s.red[PA_B4 + col] = z ? b4sum : s.red[PA_B4 + col] + b4sum;
+			s.red[PA_B3 + col] = z ? b3sum : s.red[PA_B3 + col] + b3sum;
+			s.red[PA_B2 + col] = z ? b2sum : s.red[PA_B2 + col] + b2sum;
+			s.red[PA_B1 + col] = z ? b1sum : s.red[PA_B1 + col] + b1sum;
+		}
+	}
+	for (int h = 16; h > 0; h >>= 1) se += __shfl_down_sync(0xffffffffu, se, h);
+	if (lane == 0) s.loss[warp] = se;
 	__syncthreads();
-	for (int h = blockDim.x / 2; h > 0; h >>= 1) {
-		if (threadIdx.x < h) red[threadIdx.x] += red[threadIdx.x + h];
+	for (int i = t; i < PA_N; i += MLP_TPB) p.part[(size_t)blockIdx.x * PA_N + i] = s.red[i];
+	if (t == 0) {
+		float l = 0.f;
+		for (int w = 0; w < MLP_TPB / 32; w++) l += s.loss[w];
+		p.lossp[blockIdx.x] = l;
+	}
+}
+
+// Weight gradients dW[o][i] = sum_rows g[row][o] a[row][i] of one slice of rows
+// (blockIdx.x) of layer 3, 2 or 1 (blockIdx.y), tiles of 64 rows in two buffers:
+// the next one loads while this one is multiplied.  part: [slice][2 H H + H IN].
+constexpr int WG_TPB = 256;
+constexpr int WG_N = 2 * H * H + H * S::IN;
+struct WgShared {
+	uint16_t g[2][TR][LDH], a[2][TR][LDH];
+};
+__device__ __forceinline__ void cp16(void* dst, const void* src, bool on) {
+	const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
+	const int n = on ? 16 : 0;
+	asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(d), "l"(src), "r"(n));
+}
+// rows [r0, r0 + TR) of a [.][COLS] matrix, rows at or past `end` as zeros
+template <int COLS>
+__device__ __forceinline__ void load_tile(uint16_t (*dst)[LDH], const uint16_t* __restrict__ src, int r0, int end) {
+	for (int i = threadIdx.x; i < TR * (COLS / 8); i += WG_TPB) {
+		const int r = i / (COLS / 8), c = i % (COLS / 8);
+		const bool on = r0 + r < end;
+		cp16(&dst[r][8 * c], src + (size_t)(on ? r0 + r : 0) * COLS + 8 * c, on);
+	}
+}
+
+template <int IN>  // columns of a: 128, or 16 for the first layer
+__device__ __forceinline__ void wgrad_slice(WgShared& s, const uint16_t* __restrict__ g, const uint16_t* __restrict__ a,
+                                            int r0, int r1, float* __restrict__ out) {
+	// 8 warps: 2 (64 outputs) x 4 (32 inputs); 8 (16 outputs) x 1 (16 inputs)
+	constexpr int MT = IN == H ? 4 : 1, NT = IN == H ? 4 : 2;
+	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, r = lane & 7, id = lane >> 3;
+	const int m0 = IN == H ? (warp & 1) * 64 : warp * 16, n0 = IN == H ? (warp >> 1) * 32 : 0;
+	float acc[MT][NT][4];
+#pragma unroll
+	for (int i = 0; i < MT; i++)
+#pragma unroll
+		for (int j = 0; j < NT; j++)
+#pragma unroll
+			for (int k = 0; k < 4; k++) acc[i][j][k] = 0.f;
+	load_tile<H>(s.g[0], g, r0, r1);
+	load_tile<IN>(s.a[0], a, r0, r1);
+	asm volatile("cp.async.commit_group;\n");
+	int buf = 0;
+	for (int b = r0; b < r1; b += TR, buf ^= 1) {
+		if (b + TR < r1) {
+			load_tile<H>(s.g[buf ^ 1], g, b + TR, r1);
+			load_tile<IN>(s.a[buf ^ 1], a, b + TR, r1);
+		}
+		asm volatile("cp.async.commit_group;\n");
+		asm volatile("cp.async.wait_group 1;\n");
+		__syncthreads();
+#pragma unroll
+		for (int k0 = 0; k0 < TR; k0 += 16) {
+			uint32_t fa[MT][4], fb[NT / 2][4];
+#pragma unroll
+			for (int i = 0; i < MT; i++)
+				ldsm4<true>(fa[i], &s.g[buf][k0 + r + (id >> 1) * 8][m0 + 16 * i + (id & 1) * 8]);
+#pragma unroll
+			for (int j = 0; j < NT / 2; j++)
+				ldsm4<true>(fb[j], &s.a[buf][k0 + r + (id & 1) * 8][n0 + 16 * j + (id >> 1) * 8]);
+#pragma unroll
+			for (int i = 0; i < MT; i++)
+#pragma unroll
+				for (int j = 0; j < NT; j++) mma_bf16(acc[i][j], fa[i], fb[j >> 1][2 * (j & 1)], fb[j >> 1][2 * (j & 1) + 1]);
+		}
 		__syncthreads();
 	}
-	if (threadIdx.x == 0) lossp[blockIdx.x] = red[0];
-}
-
-__global__ void k_loss_final(int nparts, const float* __restrict__ lossp, int n, double* __restrict__ out) {
-	if (threadIdx.x != 0 || blockIdx.x != 0) return;
-	double s = 0.0;
-	for (int i = 0; i < nparts; i++) s += (double)lossp[i];
-	*out = s / ((double)n * S::N_OUT);
-}
-
-// g3[b][j] = gelu'(z3[b][j]) * sum_q d4[b][q] W4[q][j]  (BF16 out)
-__global__ void k_out_back(int n, const float* __restrict__ d4, const uint16_t* __restrict__ w4,
-                           const float* __restrict__ z3, uint16_t* __restrict__ g3) {
-	const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-	if (i >= (long long)n * H) return;
-	const int b = (int)(i / H), j = (int)(i % H);
-	float s = 0.f;
-	for (int q = 0; q < S::N_OUT; q++) s += d4[(size_t)b * S::OUT + q] * bf2f(w4[q * H + j]);
-	g3[i] = f2bf(s * gelu_d(z3[i]));
-}
-
-// per-slice partial sums over rows: dW4[q][j] = sum_b d4[b][q] a3[b][j] and db4[q] = sum_b d4[b][q]
-// part layout [slice][OUT*H + OUT]
-__global__ void k_out_wgrad(int n, int rows, const float* __restrict__ d4, const uint16_t* __restrict__ a3,
-                            float* __restrict__ part) {
-	const int j = threadIdx.x;  // H threads
-	const int r0 = blockIdx.x * rows, r1 = min(n, r0 + rows);
-	float acc[S::N_OUT], bacc[S::N_OUT];
-	for (int q = 0; q < S::N_OUT; q++) acc[q] = bacc[q] = 0.f;
-	for (int b = r0; b < r1; b++) {
-		const float a = bf2f(a3[(size_t)b * H + j]);
-		for (int q = 0; q < S::N_OUT; q++) {
-			const float d = d4[(size_t)b * S::OUT + q];
-			acc[q] += d * a;
-			bacc[q] += d;
+	const int gg = lane >> 2, t2 = 2 * (lane & 3);
+#pragma unroll
+	for (int i = 0; i < MT; i++)
+#pragma unroll
+		for (int j = 0; j < NT; j++) {
+			const int o = m0 + 16 * i + gg, n = n0 + 8 * j + t2;
+			*reinterpret_cast<float2*>(&out[(size_t)o * IN + n]) = make_float2(acc[i][j][0], acc[i][j][1]);
+			*reinterpret_cast<float2*>(&out[(size_t)(o + 8) * IN + n]) = make_float2(acc[i][j][2], acc[i][j][3]);
 		}
+}
+
+__global__ void __launch_bounds__(WG_TPB) k_wgrad(MlpArgs p, int rows, float* __restrict__ part) {
+	extern __shared__ __align__(16) unsigned char dyn[];
+	WgShared& s = *reinterpret_cast<WgShared*>(dyn);
+	const int r0 = blockIdx.x * rows, r1 = min(p.n, r0 + rows);
+	float* out = part + (size_t)blockIdx.x * WG_N;
+	if (blockIdx.y == 0) wgrad_slice<H>(s, p.g3, p.a2, r0, r1, out);
+	else if (blockIdx.y == 1) wgrad_slice<H>(s, p.g2, p.a1, r0, r1, out + H * H);
+	else wgrad_slice<S::IN>(s, p.g1, p.x, r0, r1, out + 2 * H * H);
+}
+
+struct AdamArgs {
+	float *w, *m, *v;
+	uint16_t* wb;
+	float lr, b1, b2, eps, c1, c2;
+};
+// Gradient of parameter i: its partials in four interleaved runs, each in block or
+// slice order, then the runs' sums in order; Adam with UPDATE.  A thread per run:
+// one thread per parameter, 64 dependent adds over loads 145 KB apart, took 17 us.
+// The last block adds up the loss.
+constexpr int UP_RUNS = 4, UP_PARAMS = 256 / UP_RUNS;
+template <bool UPDATE>
+__global__ void __launch_bounds__(256) k_update(int blocks_a, const float* __restrict__ pa, int slices,
+                                                const float* __restrict__ pw, float* __restrict__ grad, AdamArgs a,
+                                                const float* __restrict__ lossp, int n, double* __restrict__ loss) {
+	if (blockIdx.x == gridDim.x - 1) {
+		if (threadIdx.x == 0) {
+			double l = 0.0;
+#pragma unroll 8
+			for (int i = 0; i < blocks_a; i++) l += (double)lossp[i];
+			*loss = l / ((double)n * S::N_OUT);
+		}
+		return;
 	}
-	float* p = part + (size_t)blockIdx.x * (S::OUT * H + S::OUT);
-	for (int q = 0; q < S::OUT; q++) p[q * H + j] = q < S::N_OUT ? acc[q] : 0.f;
-	if (j < S::OUT) p[S::OUT * H + j] = j < S::N_OUT ? bacc[j] : 0.f;
-}
-
-// per-slice column sums of a BF16 [n][H] matrix (bias gradients); part [slice][H]
-__global__ void k_colsum(int n, int rows, const uint16_t* __restrict__ g, float* __restrict__ part) {
-	const int j = threadIdx.x;
-	const int r0 = blockIdx.x * rows, r1 = min(n, r0 + rows);
-	float s = 0.f;
-	for (int b = r0; b < r1; b++) s += bf2f(g[(size_t)b * H + j]);
-	part[(size_t)blockIdx.x * H + j] = s;
-}
-
-// out[i] = sum over slices s (in order) of part[s*len + i]
-__global__ void k_reduce_slices(int slices, int len, const float* __restrict__ part, float* __restrict__ out) {
-	const int i = blockIdx.x * blockDim.x + threadIdx.x;
-	if (i >= len) return;
-	float s = 0.f;
-	for (int k = 0; k < slices; k++) s += part[(size_t)k * len + i];
-	out[i] = s;
-}
-
-__global__ void k_adam(int n, float* __restrict__ w, float* __restrict__ m, float* __restrict__ v,
-                       const float* __restrict__ g, uint16_t* __restrict__ wb, float lr, float b1, float b2, float eps,
-                       float c1, float c2) {
-	const int i = blockIdx.x * blockDim.x + threadIdx.x;
-	if (i >= n) return;
-	const float gi = g[i];
-	const float mi = b1 * m[i] + (1.f - b1) * gi;
-	const float vi = b2 * v[i] + (1.f - b2) * gi * gi;
-	m[i] = mi;
-	v[i] = vi;
-	const float wi = w[i] - lr * (mi / c1) / (sqrtf(vi / c2) + eps);
-	w[i] = wi;
-	wb[i] = f2bf(wi);
+	const int lp = threadIdx.x % UP_PARAMS, run = threadIdx.x / UP_PARAMS;
+	const int i = min(blockIdx.x * UP_PARAMS + lp, S::N_PARAM - 1);
+	const float* src;
+	int count, stride;
+	const auto from_slices = [&](int off) {
+		src = pw + off;
+		count = slices;
+		stride = WG_N;
+	};
+	const auto from_blocks = [&](int off) {
+		src = pa + off;
+		count = blocks_a;
+		stride = PA_N;
+	};
+	if (i < S::OFF_B1) from_slices(2 * H * H + i);
+	else if (i < S::OFF_W2) from_blocks(PA_B1 + i - S::OFF_B1);
+	else if (i < S::OFF_B2) from_slices(H * H + i - S::OFF_W2);
+	else if (i < S::OFF_W3) from_blocks(PA_B2 + i - S::OFF_B2);
+	else if (i < S::OFF_B3) from_slices(i - S::OFF_W3);
+	else if (i < S::OFF_W4) from_blocks(PA_B3 + i - S::OFF_B3);
+	else from_blocks(i - S::OFF_W4);  // W4, b4
+	float g = 0.f;
+#pragma unroll 8
+	for (int k = run; k < count; k += UP_RUNS) g += src[(size_t)k * stride];
+	__shared__ float sums[UP_RUNS][UP_PARAMS];
+	sums[run][lp] = g;
+	__syncthreads();
+	if (run != 0 || blockIdx.x * UP_PARAMS + lp >= S::N_PARAM) return;
+	for (int r = 1; r < UP_RUNS; r++) g += sums[r][lp];
+	if (!UPDATE) {
+		grad[i] = g;
+		return;
+	}
+	const float mi = a.b1 * a.m[i] + (1.f - a.b1) * g;
+	const float vi = a.b2 * a.v[i] + (1.f - a.b2) * g * g;
+	a.m[i] = mi;
+	a.v[i] = vi;
+	const float wi = a.w[i] - a.lr * (mi / a.c1) / (sqrtf(vi / a.c2) + a.eps);
+	a.w[i] = wi;
+	a.wb[i] = f2bf(wi);
 }
 
 __global__ void k_to_bf16(int n, const float* __restrict__ w, uint16_t* __restrict__ wb) {
@@ -330,39 +513,37 @@ __global__ void k_to_bf16(int n, const float* __restrict__ w, uint16_t* __restri
 	if (i < n) wb[i] = f2bf(w[i]);
 }
 
-// conservative state from the network output
-__global__ void k_denormalise(int n, const float* __restrict__ y, const float* __restrict__ feat, int ldf,
-                              const float* __restrict__ norm, float gamma, float* __restrict__ out, int ldo) {
-	const int b = blockIdx.x * blockDim.x + threadIdx.x;
-	if (b >= n) return;
-	const float* f = feat + (size_t)b * ldf;
-	float wf[5];
-	wfree(f[4], f[5], gamma, wf);
-	for (int q = 0; q < S::N_OUT; q++) out[(size_t)b * ldo + q] = wf[q] + norm[16 + q] * y[(size_t)b * S::OUT + q];
-	for (int q = S::N_OUT; q < ldo; q++) out[(size_t)b * ldo + q] = 0.f;
-}
-
-// feature statistics: per-block partial sums of x and x^2 (double), fixed order
-__global__ void k_feat_stats(long long n, const float* __restrict__ feat, const float* __restrict__ state, float gamma,
-                             long long rows, double* __restrict__ part) {
-	const int j = threadIdx.x;  // 16 threads: 0..5 features, 8..12 target deviations
-	const long long r0 = (long long)blockIdx.x * rows, r1 = min(n, r0 + rows);
+// feature statistics: per-block sums of x and x^2 (double) over STAT_ROWS rows,
+// 16 threads a row group (0..5 features, 8..12 target deviations), fixed order
+constexpr int STAT_ROWS = 2048;
+__global__ void __launch_bounds__(256) k_feat_stats(long long n, const float* __restrict__ feat,
+                                                    const float* __restrict__ state, float gamma,
+                                                    double* __restrict__ part) {
+	const int j = threadIdx.x & 15, grp = threadIdx.x >> 4;
+	const long long r0 = (long long)blockIdx.x * STAT_ROWS, r1 = min(n, r0 + STAT_ROWS);
 	double s = 0.0, s2 = 0.0;
-	for (long long b = r0; b < r1; b++) {
-		double x;
+	for (long long b = r0 + grp; b < r1; b += 16) {
+		double x = 0.0;
 		if (j < 8) {
-			x = j < S::N_IN ? (double)feat[b * 8 + j] : 0.0;
-		} else {
+			if (j < S::N_IN) x = (double)feat[b * 8 + j];
+		} else if (j - 8 < S::N_OUT) {
 			float wf[5];
 			wfree(feat[b * 8 + 4], feat[b * 8 + 5], gamma, wf);
 			const int q = j - 8;
-			x = q < S::N_OUT ? (double)state[b * 8 + q] - (double)wf[q] : 0.0;
+			x = (double)state[b * 8 + q] - (double)(q == 0 ? wf[0] : q == 1 ? wf[1] : q == 2 ? wf[2] : q == 3 ? wf[3] : wf[4]);
 		}
 		s += x;
 		s2 += x * x;
 	}
-	part[(size_t)blockIdx.x * 32 + j] = s;
-	part[(size_t)blockIdx.x * 32 + 16 + j] = s2;
+	__shared__ double red[16][32];
+	red[grp][j] = s;
+	red[grp][16 + j] = s2;
+	__syncthreads();
+	if (threadIdx.x < 32) {
+		double v = 0.0;
+		for (int k = 0; k < 16; k++) v += red[k][threadIdx.x];
+		part[(size_t)blockIdx.x * 32 + threadIdx.x] = v;
+	}
 }
 
 inline void ok(cudaError_t e, const char* what) {
@@ -376,6 +557,13 @@ inline int blocks(long long n, int t) { return (int)((n + t - 1) / t); }
 Surrogate::Surrogate(int device, uint64_t seed, double gamma) : device_(device), gamma_(gamma), seed_(seed) {
 	if (device_ >= 0) ok(cudaSetDevice(device_), "cudaSetDevice");
 	ok(cudaStreamCreateWithFlags(&st_, cudaStreamNonBlocking), "cudaStreamCreate");
+	int dev = 0;
+	ok(cudaGetDevice(&dev), "cudaGetDevice");
+	ok(cudaDeviceGetAttribute(&sms_, cudaDevAttrMultiProcessorCount, dev), "SM count");
+	const auto smem = cudaFuncAttributeMaxDynamicSharedMemorySize;
+	ok(cudaFuncSetAttribute(k_mlp<true>, smem, (int)sizeof(MlpShared)), "shared memory");
+	ok(cudaFuncSetAttribute(k_mlp<false>, smem, (int)sizeof(MlpShared)), "shared memory");
+	ok(cudaFuncSetAttribute(k_wgrad, smem, (int)sizeof(WgShared)), "shared memory");
 	// Kaiming-uniform initialisation from a seeded generator (host), padding entries zero
 	std::vector<float> w(S::N_PARAM, 0.f);
 	std::mt19937_64 rng(seed);
@@ -474,11 +662,10 @@ void Surrogate::clear_samples() {
 
 void Surrogate::fit_normalisation() {
 	if (n_samples_ < 2) throw Error(E3D_ERR_STATE, "surrogate: no training samples");
-	const long long rows = 65536;
-	const int nb = (int)((n_samples_ + rows - 1) / rows);
+	const int nb = (int)((n_samples_ + STAT_ROWS - 1) / STAT_ROWS);
 	DevBuf<double> part;
 	part.alloc((size_t)nb * 32);
-	k_feat_stats<<<nb, 16, 0, st_>>>(n_samples_, feat_.p, state_.p, (float)gamma_, rows, part.p);
+	k_feat_stats<<<nb, 256, 0, st_>>>(n_samples_, feat_.p, state_.p, (float)gamma_, part.p);
 	ok(cudaGetLastError(), "feat_stats");
 	std::vector<double> h((size_t)nb * 32);
 	ok(cudaMemcpyAsync(h.data(), part.p, h.size() * sizeof(double), cudaMemcpyDeviceToHost, st_), "stats");
@@ -505,76 +692,47 @@ void Surrogate::ensure_work(int n) {
 	if (n <= work_n_) return;
 	work_n_ = n;
 	x_.alloc((size_t)n * S::IN);
-	for (auto* b : {&a1_, &a2_, &a3_, &g1_, &g2_, &g3_}) b->alloc((size_t)n * H);
-	for (auto* b : {&z1_, &z2_, &z3_}) b->alloc((size_t)n * H);
-	y_.alloc((size_t)n * S::OUT);
-	t_.alloc((size_t)n * S::OUT);
-	lossp_.alloc((size_t)blocks(n, 256));
-	// split-K partials: up to 64 slices of the largest weight block (+ output layer)
-	part_.alloc((size_t)64 * (H * H + S::OUT * H + S::OUT));
+	for (auto* b : {&a1_, &a2_, &g1_, &g2_, &g3_}) b->alloc((size_t)n * H);
+	lossp_.alloc((size_t)sms_);
+	part_.alloc((size_t)sms_ * PA_N);
+	wpart_.alloc((size_t)kSlices * WG_N);
 }
 
-// forward of n prepared rows (x_ filled): z1..z3, a1..a3, y
-void Surrogate::forward(int n) {
-	Epi e{};
-	e.ldo = H;
-	e.bias = master_.p + S::OFF_B1;
-	e.zout = z1_.p;
-	e.hout = a1_.p;
-	gemm<L_ROW, L_ROW, EPI_FWD_GELU>(n, H, S::IN, x_.p, S::IN, wb_.p + S::OFF_W1, S::IN, 1, e, st_);
-	e.bias = master_.p + S::OFF_B2;
-	e.zout = z2_.p;
-	e.hout = a2_.p;
-	gemm<L_ROW, L_ROW, EPI_FWD_GELU>(n, H, H, a1_.p, H, wb_.p + S::OFF_W2, H, 1, e, st_);
-	e.bias = master_.p + S::OFF_B3;
-	e.zout = z3_.p;
-	e.hout = a3_.p;
-	gemm<L_ROW, L_ROW, EPI_FWD_GELU>(n, H, H, a2_.p, H, wb_.p + S::OFF_W3, H, 1, e, st_);
-	k_out_layer<<<blocks(n, 128), 128, 0, st_>>>(n, a3_.p, wb_.p + S::OFF_W4, master_.p + S::OFF_B4, y_.p);
-	ok(cudaGetLastError(), "forward");
-}
-
-// backward of the rows of the last forward against the targets in t_: loss and grad_ (all parameters)
-void Surrogate::backward(int n, double* loss_out) {
-	float* d4 = reinterpret_cast<float*>(g1_.p);  // reuse: d4 [n][OUT] floats fit in g1 ([n][H] BF16)
-	const int lb = blocks(n, 256);
-	k_loss<<<lb, 256, 0, st_>>>(n, y_.p, t_.p, d4, lossp_.p);
-	k_loss_final<<<1, 1, 0, st_>>>(lb, lossp_.p, n, loss_d_.p);
-	// output layer gradients
-	const int rows = std::max(64, (n + 63) / 64);
-	const int sl = (n + rows - 1) / rows;
-	const int lo = S::OUT * H + S::OUT;
-	k_out_wgrad<<<sl, H, 0, st_>>>(n, rows, d4, a3_.p, part_.p);
-	k_reduce_slices<<<blocks(lo, 256), 256, 0, st_>>>(sl, lo, part_.p, grad_.p + S::OFF_W4);  // W4 then b4
-	k_out_back<<<blocks((long long)n * H, 256), 256, 0, st_>>>(n, d4, wb_.p + S::OFF_W4, z3_.p, g3_.p);
-	ok(cudaGetLastError(), "backward out");
-	const int slices = std::min(64, std::max(1, n / 256));
-	auto wgrad = [&](const uint16_t* g, const uint16_t* a, int in, int off_w, int off_b) {
-		Epi e{};
-		e.part = part_.p;
-		gemm<L_COL, L_COL, EPI_PARTIAL>(H, in, n, g, H, a, in, slices, e, st_);
-		const int ks = ((n + slices - 1) / slices + BK - 1) / BK * BK;
-		const int s_used = (n + ks - 1) / ks;
-		k_reduce_slices<<<blocks(H * in, 256), 256, 0, st_>>>(s_used, H * in, part_.p, grad_.p + off_w);
-		k_colsum<<<sl, H, 0, st_>>>(n, rows, g, part_.p);
-		k_reduce_slices<<<1, H, 0, st_>>>(sl, H, part_.p, grad_.p + off_b);
-	};
-	wgrad(g3_.p, a2_.p, H, S::OFF_W3, S::OFF_B3);
-	Epi e{};
-	e.ldo = H;
-	e.zin = z2_.p;
-	e.hout = g2_.p;
-	gemm<L_ROW, L_COL, EPI_BWD_GELU>(n, H, H, g3_.p, H, wb_.p + S::OFF_W3, H, 1, e, st_);
-	wgrad(g2_.p, a1_.p, H, S::OFF_W2, S::OFF_B2);
-	e.zin = z1_.p;
-	e.hout = g1_.p;  // d4 is dead by now
-	gemm<L_ROW, L_COL, EPI_BWD_GELU>(n, H, H, g2_.p, H, wb_.p + S::OFF_W2, H, 1, e, st_);
-	wgrad(g1_.p, x_.p, S::IN, S::OFF_W1, S::OFF_B1);
-	ok(cudaGetLastError(), "backward");
-	if (loss_out) {
-		ok(cudaMemcpyAsync(loss_out, loss_d_.p, sizeof(double), cudaMemcpyDeviceToHost, st_), "loss");
-		ok(cudaStreamSynchronize(st_), "sync");
-	}
+// Loss and gradient partials of n rows (part_, wpart_, lossp_); `grad`: gradient
+// into grad_ and the loss into *loss, else one Adam step as well.
+void Surrogate::step_rows(int n, const float* feat, const float* state, long long n_store, const AdamStep* adam,
+                          double* loss) {
+	MlpArgs p{};
+	p.n = n;
+	p.feat = feat;
+	p.state = state;
+	p.n_store = n_store;
+	p.seed = seed_;
+	p.step = step_;
+	p.norm = norm_.p;
+	p.gamma = (float)gamma_;
+	p.master = master_.p;
+	p.wb = wb_.p;
+	p.x = x_.p;
+	p.a1 = a1_.p;
+	p.a2 = a2_.p;
+	p.g1 = g1_.p;
+	p.g2 = g2_.p;
+	p.g3 = g3_.p;
+	p.part = part_.p;
+	p.lossp = lossp_.p;
+	const int grid = std::min(sms_, blocks(n, TR));
+	k_mlp<true><<<grid, MLP_TPB, sizeof(MlpShared), st_>>>(p);
+	// slices of whole tiles, at most kSlices of them
+	const int rows = blocks(blocks(n, TR), kSlices) * TR, slices = blocks(n, rows);
+	k_wgrad<<<dim3(slices, 3), WG_TPB, sizeof(WgShared), st_>>>(p, rows, wpart_.p);
+	AdamArgs a{};
+	if (adam)
+		a = AdamArgs{master_.p, m1_.p, m2_.p, wb_.p, adam->lr, adam->b1, adam->b2, adam->eps, adam->c1, adam->c2};
+	const int ug = blocks(S::N_PARAM, UP_PARAMS) + 1;
+	if (adam) k_update<true><<<ug, 256, 0, st_>>>(grid, part_.p, slices, wpart_.p, grad_.p, a, lossp_.p, n, loss);
+	else k_update<false><<<ug, 256, 0, st_>>>(grid, part_.p, slices, wpart_.p, grad_.p, a, lossp_.p, n, loss);
+	ok(cudaGetLastError(), "training step");
 }
 
 double Surrogate::train(int steps, int batch, double lr, std::vector<float>* loss_per_step) {
@@ -583,26 +741,20 @@ double Surrogate::train(int steps, int batch, double lr, std::vector<float>* los
 	if (n_samples_ < 2) throw Error(E3D_ERR_STATE, "surrogate: no training samples");
 	if (!normalised_) fit_normalisation();
 	ensure_work(batch);
-	DevBuf<double> hist;
-	hist.alloc((size_t)steps);
-	const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
+	if (hist_.n < (size_t)steps) hist_.alloc((size_t)steps);
+	AdamStep ad{0.f, 0.9f, 0.999f, 1e-8f, 1.f, 1.f};
 	for (int s = 0; s < steps; s++) {
-		k_prepare<<<blocks(batch, 256), 256, 0, st_>>>(batch, feat_.p, 8, state_.p, 8, n_samples_, seed_, step_,
-		                                               norm_.p, (float)gamma_, x_.p, t_.p);
-		forward(batch);
-		backward(batch, nullptr);
-		ok(cudaMemcpyAsync(hist.p + s, loss_d_.p, sizeof(double), cudaMemcpyDeviceToDevice, st_), "loss");
-		step_++;
 		// cosine decay to 5% of lr over this call
 		const double frac = steps > 1 ? (double)s / (steps - 1) : 1.0;
-		const float lr_s = (float)(lr * (0.05 + 0.95 * 0.5 * (1.0 + std::cos(3.14159265358979 * frac))));
-		const float c1 = 1.f - std::pow(b1, (float)step_), c2 = 1.f - std::pow(b2, (float)step_);
-		k_adam<<<blocks(S::N_PARAM, 256), 256, 0, st_>>>(S::N_PARAM, master_.p, m1_.p, m2_.p, grad_.p, wb_.p, lr_s,
-		                                                 b1, b2, eps, c1, c2);
+		ad.lr = (float)(lr * (0.05 + 0.95 * 0.5 * (1.0 + std::cos(3.14159265358979 * frac))));
+		ad.c1 = 1.f - std::pow(ad.b1, (float)(step_ + 1));
+		ad.c2 = 1.f - std::pow(ad.b2, (float)(step_ + 1));
+		step_rows(batch, feat_.p, state_.p, n_samples_, &ad, hist_.p + s);
+		step_++;
 	}
 	ok(cudaGetLastError(), "train");
 	std::vector<double> h(steps);
-	ok(cudaMemcpyAsync(h.data(), hist.p, steps * sizeof(double), cudaMemcpyDeviceToHost, st_), "loss history");
+	ok(cudaMemcpyAsync(h.data(), hist_.p, steps * sizeof(double), cudaMemcpyDeviceToHost, st_), "loss history");
 	ok(cudaStreamSynchronize(st_), "sync");
 	if (loss_per_step) loss_per_step->assign(h.begin(), h.end());
 	const int k = std::min(steps, 50);
@@ -622,10 +774,9 @@ double Surrogate::gradient(const float* feat6, const float* state5, int n, std::
 	fd.upload(f);
 	sd.upload(s);
 	ensure_work(n);
-	k_prepare<<<blocks(n, 256), 256, 0, st_>>>(n, fd.p, 8, sd.p, 8, 0, 0, 0, norm_.p, (float)gamma_, x_.p, t_.p);
-	forward(n);
+	step_rows(n, fd.p, sd.p, 0, nullptr, loss_d_.p);
 	double loss = 0.0;
-	backward(n, &loss);
+	ok(cudaMemcpyAsync(&loss, loss_d_.p, sizeof(double), cudaMemcpyDeviceToHost, st_), "loss");
 	grad.resize(S::N_PARAM);
 	ok(cudaMemcpyAsync(grad.data(), grad_.p, S::N_PARAM * sizeof(float), cudaMemcpyDeviceToHost, st_), "grad");
 	ok(cudaStreamSynchronize(st_), "sync");
@@ -634,15 +785,17 @@ double Surrogate::gradient(const float* feat6, const float* state5, int n, std::
 
 void Surrogate::predict_device(const float* feat, long long n, float* state, cudaStream_t consumer) {
 	if (consumer) ok(cudaStreamSynchronize(consumer), "sync");
-	const int chunk = 1 << 20;
-	ensure_work((int)std::min<long long>(n, chunk));
+	const long long chunk = 1 << 30;  // rows of a launch fit an int
 	for (long long b0 = 0; b0 < n; b0 += chunk) {
-		const int m = (int)std::min<long long>(chunk, n - b0);
-		k_prepare<<<blocks(m, 256), 256, 0, st_>>>(m, feat + b0 * 8, 8, nullptr, 0, 0, 0, 0, norm_.p, (float)gamma_,
-		                                           x_.p, nullptr);
-		forward(m);
-		k_denormalise<<<blocks(m, 256), 256, 0, st_>>>(m, y_.p, feat + b0 * 8, 8, norm_.p, (float)gamma_,
-		                                               state + b0 * 8, 8);
+		MlpArgs p{};
+		p.n = (int)std::min<long long>(chunk, n - b0);
+		p.feat = feat + b0 * 8;
+		p.norm = norm_.p;
+		p.gamma = (float)gamma_;
+		p.master = master_.p;
+		p.wb = wb_.p;
+		p.out = state + b0 * 8;
+		k_mlp<false><<<std::min(sms_, blocks(p.n, TR)), MLP_TPB, sizeof(MlpShared), st_>>>(p);
 	}
 	ok(cudaGetLastError(), "predict");
 	ok(cudaStreamSynchronize(st_), "sync");

@@ -64,9 +64,13 @@ public:
 private:
 	void fit_normalisation();
 	void upload_params();
-	void forward(int n);                         // rows prepared in x_ (n <= work_n_)
-	void backward(int n, double* loss_out);      // against the targets in t_
+	struct AdamStep {
+		float lr, b1, b2, eps, c1, c2;
+	};
+	// loss and gradient of n rows (n <= work_n_), then an Adam step if given
+	void step_rows(int n, const float* feat, const float* state, long long n_store, const AdamStep* adam, double* loss);
 	void ensure_work(int n);
+	static constexpr int kSlices = 64;  // row slices of the weight gradients
 
 	int device_;
 	double gamma_;
@@ -82,9 +86,10 @@ private:
 	long long step_ = 0;
 	// per-minibatch work buffers
 	int work_n_ = 0;
-	DevBuf<uint16_t> x_, a1_, a2_, a3_, g1_, g2_, g3_;
-	DevBuf<float> z1_, z2_, z3_, y_, t_, part_, lossp_;
-	DevBuf<double> loss_d_;
+	int sms_ = 1;
+	DevBuf<uint16_t> x_, a1_, a2_, g1_, g2_, g3_;
+	DevBuf<float> part_, wpart_, lossp_;
+	DevBuf<double> loss_d_, hist_;  // loss of one call, of a run's steps
 };
 
 }  // namespace e3d
