@@ -24,7 +24,11 @@ void DevBuf<T>::alloc(size_t count) {
 template <class T>
 void DevBuf<T>::upload(const std::vector<T>& h) {
 	alloc(h.size());
-	if (!h.empty()) cuda_ok(cudaMemcpy(p, h.data(), h.size() * sizeof(T), cudaMemcpyHostToDevice), "upload");
+	if (h.empty()) return;
+	cuda_ok(cudaMemcpy(p, h.data(), h.size() * sizeof(T), cudaMemcpyHostToDevice), "upload");
+	// a copy from pageable memory may return with its last staged part still on the way, and the
+	// solver's streams do not wait for the default stream
+	cuda_ok(cudaStreamSynchronize(nullptr), "upload");
 }
 template <class T>
 void DevBuf<T>::free() {

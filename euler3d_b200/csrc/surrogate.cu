@@ -830,7 +830,7 @@ void Surrogate::get_params(float* out) const {
 	ok(cudaMemcpy(out, master_.p, S::N_PARAM * sizeof(float), cudaMemcpyDeviceToHost), "params");
 }
 void Surrogate::set_params(const float* in) {
-	ok(cudaMemcpy(master_.p, in, S::N_PARAM * sizeof(float), cudaMemcpyHostToDevice), "params");
+	ok(cudaMemcpyAsync(master_.p, in, S::N_PARAM * sizeof(float), cudaMemcpyHostToDevice, st_), "params");
 	upload_params();
 	ok(cudaStreamSynchronize(st_), "sync");
 }
