@@ -376,7 +376,7 @@ void Engine::build_blocks(const std::vector<const HostBlock*>& blocks, const std
 		block_case_d_.upload(block_case_);
 		std::vector<int> cwo(ncases_ + 1);
 		for (int c = 0; c <= ncases_; c++) cwo[c] = wall_off[case_boff_[c]];
-		case_wall_off_d_.upload(cwo);
+		case_wall_off_h_ = cwo;
 		case_ma_d_.upload(case_ma_h_);
 		fallback_d_.alloc(1);
 	}
@@ -1793,8 +1793,24 @@ double Engine::solve_batch(int max_iter, double criterion, int iters_per_launch,
 }
 
 // ---------------------------------------------------------------- warm start / precision
-void Engine::cell_features(float* dev_out) {
-	launch_cell_features(NR_, nb_, roff_d_.p, block_case_d_.p, cen_d_.p, case_wall_off_d_.p, wall_face_.p, fc_.p,
+void Engine::cell_features(float* dev_out, int c0, int n) {
+	if (n < 0) n = NR_ - c0;
+	if (!case_cluster_d_.n) {  // first use: the wall faces in clusters
+		std::vector<int> first, cc(1, 0);
+		for (int c = 0; c < ncases_; c++) {
+			for (int f = case_wall_off_h_[c]; f < case_wall_off_h_[c + 1]; f += WALL_CLUSTER) first.push_back(f);
+			cc.push_back((int)first.size());
+		}
+		first.push_back(case_wall_off_h_[ncases_]);
+		cluster_first_d_.upload(first);
+		wall_centre_.alloc(4 * std::max<size_t>(1, wall_face_.n));
+		wall_box_.alloc(8 * first.size());
+		launch_wall_clusters((int)first.size() - 1, cluster_first_d_.p, wall_face_.p, fc_.p,
+		                     reinterpret_cast<float4*>(wall_centre_.p), reinterpret_cast<float4*>(wall_box_.p), st_);
+		case_cluster_d_.upload(cc);
+	}
+	launch_cell_features(c0, n, nb_, roff_d_.p, block_case_d_.p, cen_d_.p, case_cluster_d_.p, cluster_first_d_.p,
+	                     reinterpret_cast<const float4*>(wall_centre_.p), reinterpret_cast<const float4*>(wall_box_.p),
 	                     case_ma_d_.p, dev_out, st_);
 	check("cell_features");
 }
@@ -1808,19 +1824,26 @@ void Engine::conservative_rows(float* dev_out) {
 	check("conservative_rows");
 }
 
-int Engine::apply_conservative(const float* dev_w, int ld) {
+void Engine::clear_fallbacks() {
+	require_not_delta("apply_conservative");  // before a caller queues work for it
+	cuda_ok(cudaMemsetAsync(fallback_d_.p, 0, sizeof(int), st_), "memset");
+}
+
+void Engine::apply_conservative(const float* dev_w, int ld, int c0, int n) {
 	require_not_delta("apply_conservative");
 	if (ld < 5) throw Error(E3D_ERR_ARG, "conservative rows need at least 5 columns");
-	cuda_ok(cudaMemsetAsync(fallback_d_.p, 0, sizeof(int), st_), "memset");
 	if (opt_.precision == PREC_FP32)
-		launch_apply_conservative<float>(NR_, NA_, nb_, roff_d_.p, block_case_d_.p, dev_w, ld, case_free_d_.p,
+		launch_apply_conservative<float>(c0, n, NR_, NA_, nb_, roff_d_.p, block_case_d_.p, dev_w, ld, case_free_d_.p,
 		                                 ph_.gamma, f32_.P0.p, f32_.P1.p, carry_ ? W0_.p : nullptr, fallback_d_.p,
 		                                 st_);
 	else
-		launch_apply_conservative<double>(NR_, NA_, nb_, roff_d_.p, block_case_d_.p, dev_w, ld, case_free_d_.p,
+		launch_apply_conservative<double>(c0, n, NR_, NA_, nb_, roff_d_.p, block_case_d_.p, dev_w, ld, case_free_d_.p,
 		                                  ph_.gamma, f64_.P0.p, f64_.P1.p, carry_ ? W0_.p : nullptr, fallback_d_.p,
 		                                  st_);
 	check("apply_conservative");
+}
+
+int Engine::fallbacks() {
 	int n = 0;
 	cuda_ok(cudaMemcpyAsync(&n, fallback_d_.p, sizeof(int), cudaMemcpyDeviceToHost, st_), "fallback count");
 	cuda_ok(cudaStreamSynchronize(st_), "sync");

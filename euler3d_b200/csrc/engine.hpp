@@ -153,14 +153,17 @@ public:
 	int n_cases() const { return ncases_; }
 
 	// --- warm start and precision switch (batched / learned forms)
-	// raw surrogate inputs of every real cell, [NR][8] floats on the device:
+	// raw surrogate inputs of real cells [c0, c0 + n) (n < 0: to the last), [n][8] floats on the device:
 	// centroid x y z, distance to the nearest wall-face centre of the cell's case, Mach, alpha (deg), 0, 0
-	void cell_features(float* dev_out);
+	void cell_features(float* dev_out, int c0 = 0, int n = -1);
 	// conservative state of every real cell, [NR][8] floats on the device (5 used)
 	void conservative_rows(float* dev_out);
-	// writes a conservative state ([NR][ld] floats on the device) into every real cell; cells whose
-	// prediction is not physical keep the freestream state of their case; returns how many did
-	int apply_conservative(const float* dev_w, int ld);
+	// writes a conservative state ([n][ld] floats on the device) into real cells [c0, c0 + n), queued on
+	// stream(); cells whose prediction is not physical keep the freestream state of their case and are
+	// counted: fallbacks() is their number since clear_fallbacks()
+	void clear_fallbacks();
+	void apply_conservative(const float* dev_w, int ld, int c0, int n);
+	int fallbacks();
 	// FP32 solver -> FP64 solver in place: FP64 geometry and state (real cells from the carried FP64
 	// conservative state), histories and reference norms kept, FP32 buffers released
 	void widen_to_fp64();
@@ -250,7 +253,10 @@ private:
 	DevBuf<double> case_free_d_, wall_denom_d_;
 	std::vector<float> case_ma_h_;        // Mach, alpha (deg) of each case
 	DevBuf<float> cen_d_, case_ma_d_;     // real-cell centroids [NR][3]; per-case Mach/alpha
-	DevBuf<int> block_case_d_, case_wall_off_d_, fallback_d_;
+	DevBuf<int> block_case_d_, fallback_d_;
+	std::vector<int> case_wall_off_h_;    // wall faces of each case
+	DevBuf<int> case_cluster_d_, cluster_first_d_;  // clusters of wall faces (cell_features), on first use
+	DevBuf<float> wall_centre_, wall_box_;
 	DevBuf<int> gcase_d_;
 	int carry_ = 0;
 	int grad_kind_ = GRAD_LEAST_SQUARES, lim_kind_ = LIM_VENKATAKRISHNAN, scheme_ = FLUX_ROE, order_ = 1;

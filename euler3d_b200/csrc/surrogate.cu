@@ -328,32 +328,33 @@ __global__ void __launch_bounds__(MLP_TPB, 1) k_mlp(MlpArgs p) {
 		copy_rows(s.a2, p.a2 + (size_t)i0 * H, rows);
 		b1sum += colsum16(s.a3, r16, col);
 	}
-	if (!TRAIN) return;
-	// the four row groups' sums in order, then the block's squared error
-	for (int grp = 0; grp < 4; grp++) {
-		__syncthreads();
-		if ((t >> 7) == grp) {
-			const bool z = grp == 0;
+	if constexpr (TRAIN) {
+		// the four row groups' sums in order, then the block's squared error
+		for (int grp = 0; grp < 4; grp++) {
+			__syncthreads();
+			if ((t >> 7) == grp) {
+				const bool z = grp == 0;
 #pragma unroll
-			for (int q = 0; q < S::OUT; q++) {
-				float& r = s.red[q * H + col];
-				const float v = q < S::N_OUT ? w4sum[q < S::N_OUT ? q : 0] : 0.f;
-				r = z ? v : r + v;
+				for (int q = 0; q < S::OUT; q++) {
+					float& r = s.red[q * H + col];
+					const float v = q < S::N_OUT ? w4sum[q < S::N_OUT ? q : 0] : 0.f;
+					r = z ? v : r + v;
+				}
+				if (col < S::OUT) s.red[PA_B4 + col] = z ? b4sum : s.red[PA_B4 + col] + b4sum;
+				s.red[PA_B3 + col] = z ? b3sum : s.red[PA_B3 + col] + b3sum;
+				s.red[PA_B2 + col] = z ? b2sum : s.red[PA_B2 + col] + b2sum;
+				s.red[PA_B1 + col] = z ? b1sum : s.red[PA_B1 + col] + b1sum;
 			}
-			if (col < S::OUT) s.red[PA_B4 + col] = z ? b4sum : s.red[PA_B4 + col] + b4sum;
-			s.red[PA_B3 + col] = z ? b3sum : s.red[PA_B3 + col] + b3sum;
-			s.red[PA_B2 + col] = z ? b2sum : s.red[PA_B2 + col] + b2sum;
-			s.red[PA_B1 + col] = z ? b1sum : s.red[PA_B1 + col] + b1sum;
 		}
-	}
-	for (int h = 16; h > 0; h >>= 1) se += __shfl_down_sync(0xffffffffu, se, h);
-	if (lane == 0) s.loss[warp] = se;
-	__syncthreads();
-	for (int i = t; i < PA_N; i += MLP_TPB) p.part[(size_t)blockIdx.x * PA_N + i] = s.red[i];
-	if (t == 0) {
-		float l = 0.f;
-		for (int w = 0; w < MLP_TPB / 32; w++) l += s.loss[w];
-		p.lossp[blockIdx.x] = l;
+		for (int h = 16; h > 0; h >>= 1) se += __shfl_down_sync(0xffffffffu, se, h);
+		if (lane == 0) s.loss[warp] = se;
+		__syncthreads();
+		for (int i = t; i < PA_N; i += MLP_TPB) p.part[(size_t)blockIdx.x * PA_N + i] = s.red[i];
+		if (t == 0) {
+			float l = 0.f;
+			for (int w = 0; w < MLP_TPB / 32; w++) l += s.loss[w];
+			p.lossp[blockIdx.x] = l;
+		}
 	}
 }
 
@@ -557,6 +558,7 @@ inline int blocks(long long n, int t) { return (int)((n + t - 1) / t); }
 Surrogate::Surrogate(int device, uint64_t seed, double gamma) : device_(device), gamma_(gamma), seed_(seed) {
 	if (device_ >= 0) ok(cudaSetDevice(device_), "cudaSetDevice");
 	ok(cudaStreamCreateWithFlags(&st_, cudaStreamNonBlocking), "cudaStreamCreate");
+	ok(cudaEventCreateWithFlags(&params_ready_, cudaEventDisableTiming), "event");
 	int dev = 0;
 	ok(cudaGetDevice(&dev), "cudaGetDevice");
 	ok(cudaDeviceGetAttribute(&sms_, cudaDevAttrMultiProcessorCount, dev), "SM count");
@@ -593,6 +595,7 @@ Surrogate::Surrogate(int device, uint64_t seed, double gamma) : device_(device),
 }
 
 Surrogate::~Surrogate() {
+	if (params_ready_) cudaEventDestroy(params_ready_);
 	if (st_) cudaStreamDestroy(st_);
 }
 
@@ -783,8 +786,12 @@ double Surrogate::gradient(const float* feat6, const float* state5, int n, std::
 	return loss;
 }
 
-void Surrogate::predict_device(const float* feat, long long n, float* state, cudaStream_t consumer) {
-	if (consumer) ok(cudaStreamSynchronize(consumer), "sync");
+// Rows queued on `st`, behind the parameters' last update.
+void Surrogate::predict_device(const float* feat, long long n, float* state, cudaStream_t st) {
+	if (st != st_) {
+		ok(cudaEventRecord(params_ready_, st_), "event");
+		ok(cudaStreamWaitEvent(st, params_ready_, 0), "event");
+	}
 	const long long chunk = 1 << 30;  // rows of a launch fit an int
 	for (long long b0 = 0; b0 < n; b0 += chunk) {
 		MlpArgs p{};
@@ -795,10 +802,9 @@ void Surrogate::predict_device(const float* feat, long long n, float* state, cud
 		p.master = master_.p;
 		p.wb = wb_.p;
 		p.out = state + b0 * 8;
-		k_mlp<false><<<std::min(sms_, blocks(p.n, TR)), MLP_TPB, sizeof(MlpShared), st_>>>(p);
+		k_mlp<false><<<std::min(sms_, blocks(p.n, TR)), MLP_TPB, sizeof(MlpShared), st>>>(p);
 	}
 	ok(cudaGetLastError(), "predict");
-	ok(cudaStreamSynchronize(st_), "sync");
 }
 
 void Surrogate::predict_host(const float* feat6, long long n, float* state5) {
@@ -809,21 +815,31 @@ void Surrogate::predict_host(const float* feat6, long long n, float* state5) {
 	DevBuf<float> fd, sd;
 	fd.upload(f);
 	sd.alloc((size_t)n * 8);
-	predict_device(fd.p, n, sd.p, nullptr);
+	predict_device(fd.p, n, sd.p, st_);
 	std::vector<float> s((size_t)n * 8);
-	ok(cudaMemcpy(s.data(), sd.p, s.size() * sizeof(float), cudaMemcpyDeviceToHost), "predict");
+	ok(cudaMemcpyAsync(s.data(), sd.p, s.size() * sizeof(float), cudaMemcpyDeviceToHost, st_), "predict");
+	ok(cudaStreamSynchronize(st_), "sync");
 	for (long long i = 0; i < n; i++)
 		for (int q = 0; q < 5; q++) state5[i * 5 + q] = s[i * 8 + q];
 }
 
+// Features, network and state write of kWarmRows cells at a time, on the engine's
+// stream: the two buffers stay (64 MB at most) instead of 64 bytes a cell
+// allocated and freed on every call.
 int Surrogate::warm_start(Engine& e) {
-	const int nr = e.n_real_total();
-	DevBuf<float> f, w;
-	f.alloc((size_t)nr * 8);
-	w.alloc((size_t)nr * 8);
-	e.cell_features(f.p);
-	predict_device(f.p, nr, w.p, e.stream());
-	return e.apply_conservative(w.p, 8);
+	const int nr = (int)e.n_real_total(), m = std::min(nr, kWarmRows);
+	if (warm_f_.n < (size_t)m * 8) {
+		warm_f_.alloc((size_t)m * 8);
+		warm_w_.alloc((size_t)m * 8);
+	}
+	e.clear_fallbacks();
+	for (int c0 = 0; c0 < nr; c0 += m) {
+		const int n = std::min(m, nr - c0);
+		e.cell_features(warm_f_.p, c0, n);
+		predict_device(warm_f_.p, n, warm_w_.p, e.stream());
+		e.apply_conservative(warm_w_.p, 8, c0, n);
+	}
+	return e.fallbacks();
 }
 
 void Surrogate::get_params(float* out) const {

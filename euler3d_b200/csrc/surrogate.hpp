@@ -50,8 +50,8 @@ public:
 	double train(int steps, int batch, double lr, std::vector<float>* loss_per_step);
 	// full-batch loss and gradient of the FP32 master parameters for the given host samples (no update)
 	double gradient(const float* feat6, const float* state5, int n, std::vector<float>& grad);
-	// inference: raw features [n][8] device -> conservative states [n][8] device
-	void predict_device(const float* feat, long long n, float* state, cudaStream_t consumer);
+	// inference: raw features [n][8] device -> conservative states [n][8] device, queued on st
+	void predict_device(const float* feat, long long n, float* state, cudaStream_t st);
 	void predict_host(const float* feat6, long long n, float* state5);
 	// predicted state into every real cell of every case of the solver; returns the fallback count
 	int warm_start(Engine& e);
@@ -89,6 +89,9 @@ private:
 	int sms_ = 1;
 	DevBuf<uint16_t> x_, a1_, a2_, g1_, g2_, g3_;
 	DevBuf<float> part_, wpart_, lossp_;
+	static constexpr int kWarmRows = 1 << 20;
+	DevBuf<float> warm_f_, warm_w_;  // features and predictions of a warm start's rows
+	cudaEvent_t params_ready_ = nullptr;
 	DevBuf<double> loss_d_, hist_;  // loss of one call, of a run's steps
 };
 

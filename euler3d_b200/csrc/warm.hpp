@@ -23,24 +23,30 @@ void launch_widen_state(int NA, int NR, const float* P32, const double* W, doubl
 // FP32 copy of an FP64 packed primitive state (all NA cells)
 void launch_narrow_state(int NA, const double* P64, float* P32, cudaStream_t st);
 
-// Raw surrogate inputs of every real cell, [NR][8] floats:
-// x, y, z (centroid), distance to the nearest wall-face centre of the cell's
-// case, Mach, alpha (degrees), 0, 0.  Cells of a case without wall faces get
-// distance 1.
-void launch_cell_features(int NR, int nb, const int* roff, const int* block_case, const float* centroid,
-                          const int* case_wall_off, const int* wall_face, const double* fc, const float* case_mach_aoa,
-                          float* out, cudaStream_t st);
+// Wall faces in clusters of at most WALL_CLUSTER consecutive ones of one case
+// (cluster k: wall faces [first[k], first[k+1])): their centres and boxes.
+constexpr int WALL_CLUSTER = 64;
+void launch_wall_clusters(int n, const int* first, const int* wall_face, const double* fc, float4* centre, float4* box,
+                          cudaStream_t st);
 
-// Writes a conservative state (rho, rho u, rho v, rho w, rho E), [NR][ld]
-// floats, into the real cells: primitives of both ping-pong buffers (T) and,
+// Raw surrogate inputs of real cells [c0, c0 + n), [n][8] floats:
+// x, y, z (centroid), distance to the nearest wall-face centre of the cell's
+// case (clusters [case_cluster[cs], case_cluster[cs+1])), Mach, alpha
+// (degrees), 0, 0.  Cells of a case without wall faces get distance 1.
+void launch_cell_features(int c0, int n, int nb, const int* roff, const int* block_case, const float* centroid,
+                          const int* case_cluster, const int* first, const float4* centre, const float4* box,
+                          const float* case_mach_aoa, float* out, cudaStream_t st);
+
+// Writes a conservative state (rho, rho u, rho v, rho w, rho E), [n][ld]
+// floats, into real cells [c0, c0 + n): primitives of both ping-pong buffers (T) and,
 // when W is non-null, the carried FP64 state.  A cell whose prediction is not
 // physical (non-finite, rho or p below 1e-3 of freestream) keeps the
 // freestream state of its case.  Returns nothing; the count of such cells is
 // added to *n_fallback (device int).
 template <class T>
-void launch_apply_conservative(int NR, int NA, int nb, const int* roff, const int* block_case, const float* Wpred,
-                               int ld, const double* case_free, double gamma, T* P0, T* P1, double* W,
-                               int* n_fallback, cudaStream_t st);
+void launch_apply_conservative(int c0, int n, int NR, int NA, int nb, const int* roff, const int* block_case,
+                               const float* Wpred, int ld, const double* case_free, double gamma, T* P0, T* P1,
+                               double* W, int* n_fallback, cudaStream_t st);
 
 // Conservative state of every real cell from the packed primitives, [NR][8]
 // floats (5 used).
