@@ -462,7 +462,7 @@ void Engine::init_state() {
 		f64_.dt.upload(std::vector<double>(NR_, 0.0));
 		f64_.FS.alloc(order_ == 2 ? 5 * (size_t)NS_ : 0);
 		srad_.upload(std::vector<double>(NR_, 0.0));
-		grad_.upload(std::vector<double>(15 * (size_t)NA_, 0.0));
+		grad_.upload(std::vector<double>(GRAD_LD * (size_t)NA_, 0.0));
 		lim_.upload(std::vector<double>(5 * (size_t)NA_, 0.0));
 	} else {
 		std::vector<float> Pf(P.begin(), P.end());
@@ -530,31 +530,6 @@ StateView Engine::state64() {
 	return s;
 }
 
-static GeoView make_geo(int NR, int NG, int NA, int NF, int NS, const int* sp, const int* sf, const int* sn,
-                        const int* flr, const double* S, const double* nh, const double* ar, const double* rl,
-                        const double* rr, const double* vol, const double* lsw, const signed char* gk,
-                        const signed char* gr) {
-	GeoView g{};
-	g.NR = NR;
-	g.NG = NG;
-	g.NA = NA;
-	g.NF = NF;
-	g.NS = NS;
-	g.slot_ptr = sp;
-	g.slot_face = sf;
-	g.slot_nbr = sn;
-	g.face_lr = flr;
-	g.S = S;
-	g.nhat = nh;
-	g.area = ar;
-	g.rl = rl;
-	g.rr = rr;
-	g.vol = vol;
-	g.lsw = lsw;
-	g.gkind = gk;
-	g.grefl = gr;
-	return g;
-}
 
 void Engine::block_range(int block, int& r0, int& r1, int& g0, int& g1) const {
 	if (block < -1 || block >= nb_) throw Error(E3D_ERR_ARG, "block index out of range");
@@ -571,36 +546,59 @@ void Engine::block_range(int block, int& r0, int& r1, int& g0, int& g1) const {
 	}
 }
 
-#define E3D_GEO                                                                                                     \
-	make_geo(NR_, NG_, NA_, NF_, NS_, slot_ptr_.p, slot_face_.p, slot_nbr_.p, face_lr_.p, S_.p, nhat_.p, area_.p, rl_.p, \
-	         rr_.p, vol64_.p, lsw64_.p, gkind_.p, grefl_.p)
+GeoView Engine::geo64() const {
+	GeoView g{};
+	g.NR = NR_;
+	g.NG = NG_;
+	g.NA = NA_;
+	g.NF = NF_;
+	g.NS = NS_;
+	g.tet4 = tet4_;
+	g.slot_ptr = slot_ptr_.p;
+	g.slot_face = slot_face_.p;
+	g.slot_nbr = slot_nbr_.p;
+	g.slot_mate = slot_mate_.p;
+	g.sgeo = f64_.sgeo.p;
+	g.srv = f64_.srv.p;
+	g.face_lr = face_lr_.p;
+	g.S = S_.p;
+	g.nhat = nhat_.p;
+	g.area = area_.p;
+	g.rl = rl_.p;
+	g.rr = rr_.p;
+	g.vol = vol64_.p;
+	g.lsw = lsw64_.p;
+	g.gkind = gkind_.p;
+	g.grefl = grefl_.p;
+	return g;
+}
 
 void Engine::save_w0(int block) {
 	require_fp64("save_w0");
 	int r0, r1, g0, g1;
 	block_range(block, r0, r1, g0, g1);
-	launch_save_w0(E3D_GEO, state64(), ph_, r0, r1, st_);
+	launch_save_w0(geo64(), state64(), ph_, r0, r1, st_);
 	check("save_w0");
 }
 void Engine::spectral_radius(int block) {
 	require_fp64("spectral_radius");
 	int r0, r1, g0, g1;
 	block_range(block, r0, r1, g0, g1);
-	launch_spectral_radius(E3D_GEO, state64(), ph_, r0, r1, st_);
+	launch_spectral_radius(geo64(), state64(), ph_, r0, r1, st_);
 	check("spectral_radius");
 }
 void Engine::timestep(int block) {
 	require_fp64("timestep");
 	int r0, r1, g0, g1;
 	block_range(block, r0, r1, g0, g1);
-	launch_timestep(E3D_GEO, state64(), ph_, r0, r1, st_);
+	launch_timestep(geo64(), state64(), ph_, r0, r1, st_);
 	check("timestep");
 }
 void Engine::gradients(int block, int kind) {
 	require_fp64("gradients");
 	int r0, r1, g0, g1;
 	block_range(block, r0, r1, g0, g1);
-	launch_gradients(E3D_GEO, state64(), kind, r0, r1, st_);
+	launch_gradients(geo64(), state64(), kind, r0, r1, st_);
 	check("gradients");
 }
 void Engine::limiters(int block, int kind, double omega, double k) {
@@ -610,28 +608,28 @@ void Engine::limiters(int block, int kind, double omega, double k) {
 	Physics ph = ph_;
 	ph.omega = omega;
 	ph.k3 = k * k * k;
-	launch_limiters(E3D_GEO, state64(), ph, kind, r0, r1, g0, g1, st_);
+	launch_limiters(geo64(), state64(), ph, kind, r0, r1, g0, g1, st_);
 	check("limiters");
 }
 void Engine::flux_conv(int block, int scheme) {
 	require_fp64("flux_conv");
 	int r0, r1, g0, g1;
 	block_range(block, r0, r1, g0, g1);
-	launch_flux_conv(E3D_GEO, state64(), ph_, scheme, r0, r1, st_);
+	launch_flux_conv(geo64(), state64(), ph_, scheme, r0, r1, st_);
 	check("flux_conv");
 }
 void Engine::flux_diss(int block, int scheme, double beta) {
 	require_fp64("flux_diss");
 	int r0, r1, g0, g1;
 	block_range(block, r0, r1, g0, g1);
-	launch_flux_diss(E3D_GEO, state64(), ph_, scheme, beta, r0, r1, st_);
+	launch_flux_diss(geo64(), state64(), ph_, scheme, beta, r0, r1, st_);
 	check("flux_diss");
 }
 void Engine::update_internal(int block, double alpha) {
 	require_fp64("update_internal");
 	int r0, r1, g0, g1;
 	block_range(block, r0, r1, g0, g1);
-	launch_update(E3D_GEO, state64(), ph_, alpha, r0, r1, st_);
+	launch_update(geo64(), state64(), ph_, alpha, r0, r1, st_);
 	check("update_internal");
 }
 void Engine::smooth_residual(int block) {
@@ -639,14 +637,14 @@ void Engine::smooth_residual(int block) {
 	int r0, r1, g0, g1;
 	block_range(block, r0, r1, g0, g1);
 	if (irs_.n < 10 * (size_t)NR_) irs_.alloc(10 * (size_t)NR_);
-	launch_smooth(E3D_GEO, state64(), irs_.p, r0, r1, st_);
+	launch_smooth(geo64(), state64(), irs_.p, r0, r1, st_);
 	check("smooth_residual");
 }
 void Engine::update_boundary(int block) {
 	require_fp64("update_boundary");
 	int r0, r1, g0, g1;
 	block_range(block, r0, r1, g0, g1);
-	launch_bc(E3D_GEO, state64(), ph_, g0, g1, st_);
+	launch_bc(geo64(), state64(), ph_, g0, g1, st_);
 	check("update_boundary");
 }
 void Engine::halo() {
@@ -1189,12 +1187,6 @@ void Engine::get(const std::string& name, int b, std::vector<double>& out) {
 	cuda_ok(cudaStreamSynchronize(st_), "sync");
 	const int nr = n_real_b_[b], na = n_all_b_[b], ng = na - nr, r0 = roff_[b], g0 = NR_ + goff_[b];
 	const bool f64 = opt_.precision == PREC_FP64;
-	auto rows_all = [&](int rows, auto* dev) {
-		out.assign((size_t)rows * na, 0.0);
-		d2h_rows(dev, NA_, rows, r0, nr, out, 0, na, st_);
-		d2h_rows(dev, NA_, rows, g0, ng, out, nr, na, st_);
-		to_local(b, out, rows, na);
-	};
 	auto rows_real = [&](int rows, auto* dev) {
 		out.assign((size_t)rows * nr, 0.0);
 		d2h_rows(dev, NR_, rows, r0, nr, out, 0, nr, st_);
@@ -1231,17 +1223,25 @@ void Engine::get(const std::string& name, int b, std::vector<double>& out) {
 		rows_real(1, srad_.p);
 	} else if (name == "limiter") {
 		require_fp64("limiter download");
-		rows_all(5, lim_.p);
+		packed_all(lim_.p);
 	} else if (name == "grad") {
 		require_fp64("grad download");
-		std::vector<double> t;
-		out.swap(t);
-		rows_all(15, grad_.p);  // [var*3+dim][cell]
-		std::vector<double> o((size_t)15 * na);
-		for (int q = 0; q < 5; q++)
-			for (int c = 0; c < na; c++)
-				for (int d = 0; d < 3; d++) o[((size_t)q * na + c) * 3 + d] = out[(size_t)(q * 3 + d) * na + c];
-		out.swap(o);
+		// device [cell][GRAD_LD] -> [var][cell][dim]
+		std::vector<double> t(GRAD_LD * (size_t)na);
+		for (int part = 0; part < 2; part++) {
+			const size_t n = part ? ng : nr, at = part ? nr : 0;
+			if (n)
+				cuda_ok(cudaMemcpyAsync(t.data() + GRAD_LD * at, grad_.p + GRAD_LD * (size_t)(part ? g0 : r0),
+				                        GRAD_LD * n * sizeof(double), cudaMemcpyDeviceToHost, st_),
+				        "d2h");
+		}
+		cuda_ok(cudaStreamSynchronize(st_), "sync");
+		out.resize((size_t)15 * na);
+		for (int c = 0; c < na; c++) {
+			const double* x = &t[GRAD_LD * (size_t)(c < nr ? pos_[b][c] : c)];
+			for (int q = 0; q < 5; q++)
+				for (int d = 0; d < 3; d++) out[((size_t)q * na + c) * 3 + d] = x[3 * q + d];
+		}
 	} else {
 		throw Error(E3D_ERR_ARG, "unknown state array '" + name + "'");
 	}
@@ -1254,13 +1254,6 @@ void Engine::set(const std::string& name, int b, const std::vector<double>& in_l
 	const int nr = n_real_b_[b], na = n_all_b_[b], ng = na - nr, r0 = roff_[b], g0 = NR_ + goff_[b];
 	const bool f64 = opt_.precision == PREC_FP64;
 	std::vector<double> in(in_local);  // real cells moved to device order below
-	auto put_all = [&](int rows, auto* dev) {
-		if (in.size() != (size_t)rows * na) throw Error(E3D_ERR_ARG, name + ": wrong length");
-		to_device(b, in, rows, na);
-		h2d_rows(dev, NA_, rows, r0, nr, in, 0, na, st_);
-		h2d_rows(dev, NA_, rows, g0, ng, in, nr, na, st_);
-		in = in_local;
-	};
 	auto put_real = [&](int rows, auto* dev) {
 		if (in.size() != (size_t)rows * nr) throw Error(E3D_ERR_ARG, name + ": wrong length");
 		to_device(b, in, rows, nr);
@@ -1296,17 +1289,24 @@ void Engine::set(const std::string& name, int b, const std::vector<double>& in_l
 		else put_real(1, f32_.dt.p);
 	} else if (name == "limiter") {
 		require_fp64("limiter upload");
-		put_all(5, lim_.p);
+		put_packed(lim_.p);
 	} else if (name == "grad") {
 		require_fp64("grad upload");
 		if (in.size() != (size_t)15 * na) throw Error(E3D_ERR_ARG, "grad: wrong length");
-		std::vector<double> t((size_t)15 * na);
-		for (int q = 0; q < 5; q++)
-			for (int c = 0; c < na; c++)
-				for (int d = 0; d < 3; d++) t[(size_t)(q * 3 + d) * na + c] = in[((size_t)q * na + c) * 3 + d];
-		to_device(b, t, 15, na);
-		h2d_rows(grad_.p, NA_, 15, r0, nr, t, 0, na, st_);
-		h2d_rows(grad_.p, NA_, 15, g0, ng, t, nr, na, st_);
+		std::vector<double> t(GRAD_LD * (size_t)na, 0.0);
+		for (int c = 0; c < na; c++) {
+			double* x = &t[GRAD_LD * (size_t)(c < nr ? pos_[b][c] : c)];
+			for (int q = 0; q < 5; q++)
+				for (int d = 0; d < 3; d++) x[3 * q + d] = in[((size_t)q * na + c) * 3 + d];
+		}
+		for (int part = 0; part < 2; part++) {
+			const size_t n = part ? ng : nr, at = part ? nr : 0;
+			if (n)
+				cuda_ok(cudaMemcpyAsync(grad_.p + GRAD_LD * (size_t)(part ? g0 : r0), t.data() + GRAD_LD * at,
+				                        GRAD_LD * n * sizeof(double), cudaMemcpyHostToDevice, st_),
+				        "h2d");
+		}
+		cuda_ok(cudaStreamSynchronize(st_), "sync");
 	} else {
 		throw Error(E3D_ERR_ARG, "unknown or read-only state array '" + name + "'");
 	}
@@ -1892,7 +1892,7 @@ void Engine::widen_to_fp64() {
 	cuda_ok(cudaMemsetAsync(f64_.dt.p, 0, f64_.dt.n * sizeof(double), st_), "memset");
 	f64_.FS.alloc(order_ == 2 ? 5 * (size_t)NS_ : 0);
 	srad_.alloc(NR_);
-	grad_.alloc(15 * (size_t)NA_);
+	grad_.alloc(GRAD_LD * (size_t)NA_);
 	lim_.alloc(5 * (size_t)NA_);
 	cuda_ok(cudaMemsetAsync(srad_.p, 0, srad_.n * sizeof(double), st_), "memset");
 	cuda_ok(cudaMemsetAsync(grad_.p, 0, grad_.n * sizeof(double), st_), "memset");

@@ -233,6 +233,7 @@ private:
 	void smoothed_iteration_body();
 	void block_range(int block, int& r0, int& r1, int& g0, int& g1) const;
 	void require_fp64(const char* what) const;
+	GeoView geo64() const;
 	StateView state64();
 	const double* cur_prim64() const;
 

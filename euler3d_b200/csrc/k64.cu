@@ -24,31 +24,41 @@ void launch_timestep(const GeoView& g, const StateView& s, const Physics& ph, in
 }
 void launch_gradients(const GeoView& g, const StateView& s, int kind, int r0, int r1, cudaStream_t st) {
 	if (r1 <= r0) return;
-	if (kind == GRAD_LEAST_SQUARES) k_grad_ls<<<blocks_for(r1 - r0, TPB), TPB, 0, st>>>(g, s, r0, r1);
-	else k_grad_gg<<<blocks_for(r1 - r0, TPB), TPB, 0, st>>>(g, s, r0, r1);
+	const int grid = blocks_for(5 * (r1 - r0), TPB);
+	if (kind == GRAD_LEAST_SQUARES) k_grad<GRAD_LEAST_SQUARES><<<grid, TPB, 0, st>>>(g, s, r0, r1);
+	else k_grad<GRAD_GREEN_GAUSS><<<grid, TPB, 0, st>>>(g, s, r0, r1);
 }
 void launch_limiters(const GeoView& g, const StateView& s, const Physics& ph, int kind, int r0, int r1, int g0, int g1,
                      cudaStream_t st) {
 	const int n = (r1 - r0) + (g1 - g0);
 	if (n <= 0) return;
-	if (kind == LIM_VENKATAKRISHNAN)
-		k_limiter<LIM_VENKATAKRISHNAN><<<blocks_for(n, TPB), TPB, 0, st>>>(g, s, ph, r0, r1, g0, g1);
-	else
-		k_limiter<LIM_BARTH_JESPERSEN><<<blocks_for(n, TPB), TPB, 0, st>>>(g, s, ph, r0, r1, g0, g1);
+	const int grid = blocks_for(5 * n, TPB);
+	if (kind == LIM_VENKATAKRISHNAN) k_limiter<LIM_VENKATAKRISHNAN><<<grid, TPB, 0, st>>>(g, s, ph, r0, r1, g0, g1);
+	else k_limiter<LIM_BARTH_JESPERSEN><<<grid, TPB, 0, st>>>(g, s, ph, r0, r1, g0, g1);
 }
+namespace {
+template <bool DISS>
+void launch_flux(const GeoView& g, const StateView& s, const Physics& ph, int scheme, double beta, int r0, int r1,
+                 cudaStream_t st) {
+	if (r1 <= r0) return;
+	const bool tet = g.tet4 != 0;
+	const int grid = blocks_for((tet ? 4 : 8) * (r1 - r0), TPB);
+	if (scheme == FLUX_AUSM) {
+		if (tet) k_flux<FLUX_AUSM, DISS, 4><<<grid, TPB, 0, st>>>(g, s, ph, beta, r0, r1);
+		else k_flux<FLUX_AUSM, DISS, 8><<<grid, TPB, 0, st>>>(g, s, ph, beta, r0, r1);
+	} else {
+		if (tet) k_flux<FLUX_ROE, DISS, 4><<<grid, TPB, 0, st>>>(g, s, ph, beta, r0, r1);
+		else k_flux<FLUX_ROE, DISS, 8><<<grid, TPB, 0, st>>>(g, s, ph, beta, r0, r1);
+	}
+}
+}  // namespace
 void launch_flux_conv(const GeoView& g, const StateView& s, const Physics& ph, int scheme, int r0, int r1,
                       cudaStream_t st) {
-	if (r1 <= r0) return;
-	if (scheme == FLUX_AUSM) k_flux_conv<FLUX_AUSM><<<blocks_for(r1 - r0, TPB), TPB, 0, st>>>(g, s, ph, r0, r1);
-	else k_flux_conv<FLUX_ROE><<<blocks_for(r1 - r0, TPB), TPB, 0, st>>>(g, s, ph, r0, r1);
+	launch_flux<false>(g, s, ph, scheme, 1.0, r0, r1, st);
 }
 void launch_flux_diss(const GeoView& g, const StateView& s, const Physics& ph, int scheme, double beta, int r0, int r1,
                       cudaStream_t st) {
-	if (r1 <= r0) return;
-	if (scheme == FLUX_AUSM)
-		k_flux_diss<FLUX_AUSM><<<blocks_for(r1 - r0, TPB), TPB, 0, st>>>(g, s, ph, beta, r0, r1);
-	else
-		k_flux_diss<FLUX_ROE><<<blocks_for(r1 - r0, TPB), TPB, 0, st>>>(g, s, ph, beta, r0, r1);
+	launch_flux<true>(g, s, ph, scheme, beta, r0, r1, st);
 }
 void launch_update(const GeoView& g, const StateView& s, const Physics& ph, double alpha, int r0, int r1,
                    cudaStream_t st) {
@@ -62,8 +72,9 @@ void launch_tail_sums(const ReduceArgs& a, int n, bool advance, cudaStream_t st)
 }
 void launch_smooth(const GeoView& g, const StateView& s, double* j1, int r0, int r1, cudaStream_t st) {
 	if (r1 <= r0) return;
-	k_irs_start<<<blocks_for(r1 - r0, TPB), TPB, 0, st>>>(g, s, j1, r0, r1);
-	k_irs_smooth<<<blocks_for(r1 - r0, TPB), TPB, 0, st>>>(g, s, j1, r0, r1);
+	const dim3 grid(blocks_for(r1 - r0, TPB), 10);
+	k_irs_start<<<grid, TPB, 0, st>>>(g, s, j1, r0, r1);
+	k_irs_smooth<<<grid, TPB, 0, st>>>(g, s, j1, r0, r1);
 }
 
 template void launch_halo<double>(int, const int*, const int*, int, double*, double*, cudaStream_t);

@@ -27,9 +27,13 @@ struct Physics {
 // Mesh topology and FP64 geometry (granular drop-in kernels).
 struct GeoView {
 	int NR, NG, NA, NF, NS;
+	int tet4;              // 1 when every real cell has exactly 4 slots
 	const int* slot_ptr;   // NA+1
 	const int* slot_face;  // NS
 	const int* slot_nbr;   // NS
+	const int* slot_mate;  // NS as in FusedView
+	const double* sgeo;    // 4*NS n, |S| of the slot's face (face orientation)
+	const double* srv;     // 3*NS r-vector of the slot's owner
 	const int* face_lr;    // 2*NF
 	const double* S;       // 3*NF area vector, left -> right
 	const double* nhat;    // 3*NF S/|S| as the reference normalises it
@@ -42,14 +46,16 @@ struct GeoView {
 	const signed char* grefl;  // NG 1: gradient reflected, 0: gradient zero
 };
 
+constexpr int GRAD_LD = 16;  // stored gradient values per cell: [var][dim], 15 used
+
 // FP64 state arrays in the reference's meaning (drop-in path).
 struct StateView {
-	double* prim;  // 5*NA  [var][cell]
+	double* prim;  // 5*NA packed: [cell] x (rho,u,v,w), then [cell] p
 	double* rc;    // 5*NR
 	double* rd;    // 5*NR
 	double* w0;    // 5*NR
-	double* grad;  // 15*NA [var][dim][cell]
-	double* lim;   // 5*NA
+	double* grad;  // 16*NA [cell][var][dim], padded
+	double* lim;   // 5*NA packed like prim
 	double* dt;    // NR
 	double* srad;  // NR
 };
