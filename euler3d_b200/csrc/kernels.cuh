@@ -32,9 +32,25 @@ struct Vec4<double> {
 	using type = double4;
 };
 
+// Four values as one memory instruction.  A double4 in C++ is two 16-byte
+// accesses; sm_100 has 32-byte ones, half the instructions and L1 tag look-ups
+// of every gathered FP64 state.  B200, 663k tets FP64: flux pass without
+// dissipation 88 -> 74 us, with 121 -> 117, first reconstruction 154 -> 145;
+// strategy-level central flux on 41k cells 14.4 -> 12.4.
+__device__ __forceinline__ float4 ldv4(const float* __restrict__ p) { return *reinterpret_cast<const float4*>(p); }
+__device__ __forceinline__ double4 ldv4(const double* __restrict__ p) {
+	double4 a;
+	asm volatile("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(a.x), "=d"(a.y), "=d"(a.z), "=d"(a.w) : "l"(p) : "memory");
+	return a;
+}
+__device__ __forceinline__ void stv4(float* p, const float4& a) { *reinterpret_cast<float4*>(p) = a; }
+__device__ __forceinline__ void stv4(double* p, const double4& a) {
+	asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(p), "d"(a.x), "d"(a.y), "d"(a.z), "d"(a.w) : "memory");
+}
+
 template <class T>
 __device__ __forceinline__ Q5<T> ld5(const T* __restrict__ P, int n, int c) {
-	const typename Vec4<T>::type a = reinterpret_cast<const typename Vec4<T>::type*>(P)[c];
+	const typename Vec4<T>::type a = ldv4(P + 4 * (size_t)c);
 	Q5<T> q;
 	q.r = a.x;
 	q.u = a.y;
@@ -50,7 +66,7 @@ __device__ __forceinline__ void st5(T* __restrict__ P, int n, int c, const Q5<T>
 	a.y = q.u;
 	a.z = q.v;
 	a.w = q.w;
-	reinterpret_cast<typename Vec4<T>::type*>(P)[c] = a;
+	stv4(P + 4 * (size_t)c, a);
 	P[4 * (size_t)n + c] = q.p;
 }
 template <class T>
@@ -111,8 +127,8 @@ __global__ void k_timestep(GeoView g, StateView s, Physics ph, int r0, int r1) {
 // a time and are bound by latency, so each takes several lanes per cell: one per
 // variable (gradients, limiters), one per slot (fluxes).  Every sum keeps the
 // reference's order.  B200, back to back on 41k cells, one thread per cell / this
-// form: Venkatakrishnan 14.4 / 10.3, central flux 14.4 / 14.4, Roe dissipation 18.5 /
-// 18.5 us; on 25k cells Barth-Jespersen 16.9 / 8.2, smoothing 21 / 9 us.
+// form: Venkatakrishnan 14.4 / 10.3, central flux 14.4 / 12.4, Roe dissipation 18.5 /
+// 16.5 us; on 25k cells Barth-Jespersen 16.9 / 8.2, smoothing 21 / 9 us.
 
 // Writes variable v's gradient of the ghosts owned by real cell c: reflected for ghosts of the
 // first n_real_boundaries markers, zero for the others (GreenGauss.cpp:68-81,
@@ -200,13 +216,14 @@ __global__ void k_limiter(GeoView g, StateView s, Physics ph, int r0, int r1, in
 __device__ __forceinline__ Q5<double> face_state(const GeoView& g, const StateView& s, int c, const double* __restrict__ r) {
 	Q5<double> q = ld5(s.prim, g.NA, c);
 	const Q5<double> phi = ld5(s.lim, g.NA, c);
-	const double2* g2 = reinterpret_cast<const double2*>(s.grad + GRAD_LD * (size_t)c);
 	double gr[GRAD_LD];
 #pragma unroll
-	for (int i = 0; i < GRAD_LD / 2; i++) {
-		const double2 x = g2[i];
-		gr[2 * i] = x.x;
-		gr[2 * i + 1] = x.y;
+	for (int i = 0; i < GRAD_LD / 4; i++) {
+		const double4 x = ldv4(s.grad + GRAD_LD * (size_t)c + 4 * i);
+		gr[4 * i] = x.x;
+		gr[4 * i + 1] = x.y;
+		gr[4 * i + 2] = x.z;
+		gr[4 * i + 3] = x.w;
 	}
 	const double rx = r[0], ry = r[1], rz = r[2];
 #pragma unroll
@@ -241,7 +258,7 @@ __global__ void __launch_bounds__(128, 6) k_flux(GeoView g, StateView s, Physics
 			qv(L, v) = left ? qv(qo, v) : qv(qn, v);
 			qv(R, v) = left ? qv(qn, v) : qv(qo, v);
 		}
-		const double4 geo = reinterpret_cast<const double4*>(g.sgeo)[sl];
+		const double4 geo = ldv4(g.sgeo + 4 * (size_t)sl);
 		const double nx = geo.x, ny = geo.y, nz = geo.z, nn = geo.w;
 		double fl[5];
 		if (DISS) {
@@ -469,11 +486,10 @@ __device__ __forceinline__ void load_int(const int* __restrict__ a, const SlotRa
 // face normal + area of each slot (face orientation)
 template <class T, int NSL>
 __device__ __forceinline__ void load_geo(const T* __restrict__ a, const SlotRange<T, NSL>& r, T o[MAXSL][4]) {
-	const typename Vec4<T>::type* p = reinterpret_cast<const typename Vec4<T>::type*>(a) + r.s0;
 #pragma unroll
 	for (int k = 0; k < (NSL == 4 ? 4 : MAXSL); k++) {
 		if (NSL != 4 && k >= r.n) break;
-		const typename Vec4<T>::type t = p[k];
+		const typename Vec4<T>::type t = ldv4(a + 4 * (size_t)(r.s0 + k));
 		o[k][0] = t.x;
 		o[k][1] = t.y;
 		o[k][2] = t.z;
@@ -919,7 +935,7 @@ __device__ __forceinline__ void flux_update_cell(const FusedView<T>& v, const Ph
 			qo = ld5(v.FS, v.NS, s);
 			qn = ld5(v.FS, v.NS, m);
 		}
-		const typename Vec4<T>::type geo = reinterpret_cast<const typename Vec4<T>::type*>(v.sgeo)[s];
+		const typename Vec4<T>::type geo = ldv4(v.sgeo + 4 * (size_t)s);
 		Q5<T> L, R;
 		for (int q = 0; q < 5; q++) {
 			qv(L, q) = left ? qv(qo, q) : qv(qn, q);
@@ -1016,7 +1032,7 @@ __device__ __forceinline__ void flux_update_slots(const FusedView<double>& v, co
 	const int nb = LPC == 4 ? (m < 4 * NR ? m >> 2 : m - 3 * NR) : v.slot_nbr[s];
 	const Q5<double> qo = ORDER1 ? ld5(v.Pin, v.NA, c) : ld5(v.FS, v.NS, s);
 	const Q5<double> qn = ORDER1 ? ld5(v.Pin, v.NA, nb) : ld5(v.FS, v.NS, m);
-	const typename Vec4<double>::type geo = reinterpret_cast<const typename Vec4<double>::type*>(v.sgeo)[s];
+	const double4 geo = ldv4(v.sgeo + 4 * (size_t)s);
 	// this lane's share of the cell: variable k, and variable 4 on lane 0
 	const int qk = k < 4 ? k : 0;
 	const double keep = 1.0 - beta;
