@@ -638,12 +638,8 @@ int e3d_history(const e3d_solver* s, int first, int count, e3d_iter_record* out)
 int e3d_state_get(e3d_solver* s, int block, const char* name, double* dst, int64_t count) {
 	if (!name || !dst) return fail(E3D_ERR_ARG, "null argument");
 	return guard([&] {
-		std::vector<double> v;
-		eng(s).get(name, block, v);
-		if (count != (int64_t)v.size())
-			throw e3d::Error(E3D_ERR_ARG, std::string(name) + ": count " + std::to_string(count) + " != " +
-			                                  std::to_string(v.size()));
-		std::memcpy(dst, v.data(), v.size() * sizeof(double));
+		if (count < 0) throw e3d::Error(E3D_ERR_ARG, "negative count");
+		eng(s).get(name, block, dst, (size_t)count);
 	});
 }
 

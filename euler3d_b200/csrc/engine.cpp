@@ -392,35 +392,8 @@ void Engine::build_blocks(const std::vector<const HostBlock*>& blocks, const std
 	lsw64_.upload(lsw);
 
 	// fused per-slot geometry, face orientation for fluxes, owner sign for GG
-	std::vector<double> sgeo(4 * (size_t)NS_), sS(3 * (size_t)NS_), srv(3 * (size_t)NS_);
-	for (int k = 0; k < NS_; k++) {
-		const int F = slot_face[k];
-		const bool left = face_slot_l[F] == k;
-		for (int d = 0; d < 3; d++) {
-			sgeo[4 * (size_t)k + d] = nhat[3 * (size_t)F + d];
-			double sv = S[3 * (size_t)F + d];
-			if (!left) sv *= -1.0;
-			sS[3 * (size_t)k + d] = sv;
-			srv[3 * (size_t)k + d] = left ? rl[3 * (size_t)F + d] : rr[3 * (size_t)F + d];
-		}
-		sgeo[4 * (size_t)k + 3] = area[F];
-	}
-	const bool need_gg = order_ == 2 && grad_kind_ == GRAD_GREEN_GAUSS;
-	const bool need_ls = order_ == 2 && grad_kind_ == GRAD_LEAST_SQUARES;
-	if (opt_.precision == PREC_FP64) {
-		f64_.sgeo.upload(sgeo);
-		if (need_gg) f64_.sS.upload(sS);
-		f64_.srv.upload(srv);
-		if (need_ls) f64_.lsw.upload(lsw);
-		f64_.vol.upload(vol);
-	} else {
-		auto tof = [](const std::vector<double>& a) { return std::vector<float>(a.begin(), a.end()); };
-		f32_.sgeo.upload(tof(sgeo));
-		if (need_gg) f32_.sS.upload(tof(sS));
-		f32_.srv.upload(tof(srv));
-		if (need_ls) f32_.lsw.upload(tof(lsw));
-		f32_.vol.upload(tof(vol));
-	}
+	if (opt_.precision == PREC_FP64) slot_geometry(f64_);
+	else slot_geometry(f32_);
 	// reductions: chunks of TAIL_CHUNK cells, never straddling a block
 	max_chunks_ = 1;
 	for (int b = 0; b < nb_; b++)
@@ -439,6 +412,26 @@ void Engine::build_blocks(const std::vector<const HostBlock*>& blocks, const std
 	cuda_ok(cudaMemset(zero_d_.p, 0, sizeof(int)), "memset");
 }
 
+// Per-slot and per-cell geometry of the fused path in its working precision,
+// from the FP64 arrays on the device.
+template <class T>
+void Engine::slot_geometry(Fused<T>& f) {
+	const bool need_gg = order_ == 2 && grad_kind_ == GRAD_GREEN_GAUSS;
+	const bool need_ls = order_ == 2 && grad_kind_ == GRAD_LEAST_SQUARES;
+	f.sgeo.alloc(4 * (size_t)NS_);
+	f.srv.alloc(3 * (size_t)NS_);
+	if (need_gg) f.sS.alloc(3 * (size_t)NS_);
+	launch_slot_geometry<T>(NS_, slot_face_.p, slot_mate_.p, S_.p, nhat_.p, area_.p, rl_.p, rr_.p, f.sgeo.p,
+	                        need_gg ? f.sS.p : nullptr, f.srv.p, st_);
+	if (need_ls) {
+		f.lsw.alloc(lsw64_.n);
+		launch_convert<T>(lsw64_.n, lsw64_.p, f.lsw.p, st_);
+	}
+	f.vol.alloc(vol64_.n);
+	launch_convert<T>(vol64_.n, vol64_.p, f.vol.p, st_);
+	check("slot geometry");
+}
+
 void Engine::init_state() {
 	// all cells, ghosts included, start at freestream
 	// (PrimitiveVariables::initializeFlowField, PrimitiveVariables.cpp:58-69);
@@ -453,27 +446,32 @@ void Engine::init_state() {
 		for (int c = roff_[b]; c < roff_[b + 1]; c++) fill_cell(c, f);
 		for (int g = NR_ + goff_[b]; g < NR_ + goff_[b + 1]; g++) fill_cell(g, f);
 	}
-	std::vector<double> zR(5 * (size_t)NR_, 0.0);
+	const auto zeros = [&](auto& buf, size_t n) {
+		buf.alloc(n);
+		if (n) cuda_ok(cudaMemsetAsync(buf.p, 0, n * sizeof(*buf.p), st_), "memset");
+	};
+	const auto same = [&](auto& buf, const auto& of) {
+		buf.alloc(of.n);
+		cuda_ok(cudaMemcpyAsync(buf.p, of.p, of.n * sizeof(*of.p), cudaMemcpyDeviceToDevice, st_), "d2d");
+	};
 	if (opt_.precision == PREC_FP64) {
 		f64_.P0.upload(P);
-		f64_.P1.upload(P);
-		f64_.Rc.upload(zR);
-		f64_.Rd.upload(zR);
-		f64_.dt.upload(std::vector<double>(NR_, 0.0));
+		same(f64_.P1, f64_.P0);
+		zeros(f64_.Rc, 5 * (size_t)NR_);
+		zeros(f64_.Rd, 5 * (size_t)NR_);
+		zeros(f64_.dt, NR_);
 		f64_.FS.alloc(order_ == 2 ? 5 * (size_t)NS_ : 0);
-		srad_.upload(std::vector<double>(NR_, 0.0));
-		grad_.upload(std::vector<double>(GRAD_LD * (size_t)NA_, 0.0));
-		lim_.upload(std::vector<double>(5 * (size_t)NA_, 0.0));
+		zeros(srad_, NR_);
+		zeros(grad_, GRAD_LD * (size_t)NA_);
+		zeros(lim_, 5 * (size_t)NA_);
 	} else {
-		std::vector<float> Pf(P.begin(), P.end());
-		f32_.P0.upload(Pf);
-		f32_.P1.upload(Pf);
-		f32_.Rc.upload(std::vector<float>(5 * (size_t)NR_, 0.f));
-		f32_.Rd.upload(std::vector<float>(5 * (size_t)NR_, 0.f));
-		f32_.dt.upload(std::vector<float>(NR_, 0.f));
+		f32_.P0.upload(std::vector<float>(P.begin(), P.end()));
+		same(f32_.P1, f32_.P0);
+		zeros(f32_.Rc, 5 * (size_t)NR_);
+		zeros(f32_.Rd, 5 * (size_t)NR_);
+		zeros(f32_.dt, NR_);
 		f32_.FS.alloc(order_ == 2 ? 5 * (size_t)NS_ : 0);
 	}
-	W0_.upload(zR);
 	if (deck_.smoothing) irs_.alloc(10 * (size_t)NR_);  // before any graph capture
 	if (carry_) {
 		// W carried in FP64 from the freestream conservative state
@@ -488,7 +486,10 @@ void Engine::init_state() {
 			W[4 * (size_t)NR_ + c] = 0.5 * f[0] * (f[1] * f[1] + f[2] * f[2] + f[3] * f[3]) + 1. / (ph_.gamma - 1.0) * f[4];
 		}
 		W0_.upload(W);
+	} else {
+		zeros(W0_, 5 * (size_t)NR_);
 	}
+	cuda_ok(cudaStreamSynchronize(st_), "sync");
 	cur_ = 0;
 	count_device_bytes();
 }
@@ -1101,34 +1102,6 @@ void Engine::sync() {
 // ---------------------------------------------------------------- state transfer
 namespace {
 template <class T>
-void d2h_rows(const T* dev, int ld, int rows, int begin, int count, std::vector<double>& out, size_t out_off,
-              int out_ld, cudaStream_t st) {
-	std::vector<T> tmp((size_t)count);
-	for (int q = 0; q < rows; q++) {
-		if (count == 0) continue;
-		cuda_ok(cudaMemcpyAsync(tmp.data(), dev + (size_t)q * ld + begin, count * sizeof(T), cudaMemcpyDeviceToHost, st),
-		        "d2h");
-		cuda_ok(cudaStreamSynchronize(st), "sync");
-		for (int i = 0; i < count; i++) out[out_off + (size_t)q * out_ld + i] = (double)tmp[i];
-	}
-}
-// Packed five-variable arrays (kernels.cuh ld5/st5): [n] x (rho,u,v,w) then [n] p.
-template <class T>
-void d2h_packed(const T* dev, int n, int begin, int count, std::vector<double>& out, size_t out_off, int out_ld,
-                cudaStream_t st) {
-	if (count == 0) return;
-	std::vector<T> v4(4 * (size_t)count), p((size_t)count);
-	cuda_ok(cudaMemcpyAsync(v4.data(), dev + 4 * (size_t)begin, 4 * (size_t)count * sizeof(T), cudaMemcpyDeviceToHost,
-	                        st),
-	        "d2h");
-	cuda_ok(cudaMemcpyAsync(p.data(), dev + 4 * (size_t)n + begin, count * sizeof(T), cudaMemcpyDeviceToHost, st), "d2h");
-	cuda_ok(cudaStreamSynchronize(st), "sync");
-	for (int i = 0; i < count; i++) {
-		for (int q = 0; q < 4; q++) out[out_off + (size_t)q * out_ld + i] = (double)v4[4 * (size_t)i + q];
-		out[out_off + 4 * (size_t)out_ld + i] = (double)p[i];
-	}
-}
-template <class T>
 void h2d_packed(T* dev, int n, int begin, int count, const std::vector<double>& in, size_t in_off, int in_ld,
                 cudaStream_t st) {
 	if (count == 0) return;
@@ -1160,18 +1133,9 @@ void h2d_rows(T* dev, int ld, int rows, int begin, int count, const std::vector<
 // Names and layouts match the reference's arrays for block `block`:
 //   prim [5][n_all], limiter [5][n_all], grad [5][n_all][3],
 //   conv_res/diss_res/w0 [5][n_real], dt/spectral_radius [n_real]
-// Real cells of block b sit on the device in the order pos_[b]; these move
-// the first nr entries of each of `rows` rows of length ld between device
-// order and the block's local (file) order.
-void Engine::to_local(int b, std::vector<double>& a, int rows, int ld) const {
-	const std::vector<int>& pos = pos_[b];
-	std::vector<double> t(pos.size());
-	for (int q = 0; q < rows; q++) {
-		double* r = a.data() + (size_t)q * ld;
-		for (size_t c = 0; c < pos.size(); c++) t[c] = r[pos[c]];
-		std::copy(t.begin(), t.end(), r);
-	}
-}
+// Real cells of block b sit on the device in the order pos_[b]; this moves
+// the first nr entries of each of `rows` rows of length ld from the block's
+// local (file) order to device order.
 void Engine::to_device(int b, std::vector<double>& a, int rows, int ld) const {
 	const std::vector<int>& pos = pos_[b];
 	std::vector<double> t(pos.size());
@@ -1182,22 +1146,39 @@ void Engine::to_device(int b, std::vector<double>& a, int rows, int ld) const {
 	}
 }
 
-void Engine::get(const std::string& name, int b, std::vector<double>& out) {
+// The device puts a block's values in file order and double precision, kStageValues
+// at a time, and one copy per piece brings them over: per-variable copies,
+// conversion and reordering on the host took 9 ms for 828k cells in six blocks,
+// twice the solver time of ten iterations.
+void Engine::get(const std::string& name, int b, double* dst, size_t count) {
 	if (b < 0 || b >= nb_) throw Error(E3D_ERR_ARG, "block index out of range");
 	cuda_ok(cudaStreamSynchronize(st_), "sync");
-	const int nr = n_real_b_[b], na = n_all_b_[b], ng = na - nr, r0 = roff_[b], g0 = NR_ + goff_[b];
+	const int nr = n_real_b_[b], na = n_all_b_[b], r0 = roff_[b], g0 = NR_ + goff_[b];
 	const bool f64 = opt_.precision == PREC_FP64;
-	auto rows_real = [&](int rows, auto* dev) {
-		out.assign((size_t)rows * nr, 0.0);
-		d2h_rows(dev, NR_, rows, r0, nr, out, 0, nr, st_);
-		to_local(b, out, rows, nr);
+	const auto bring = [&](StateLayout layout, int rows, auto* dev) {
+		const int n = layout == STATE_ROWS ? nr : na;
+		const size_t total = (size_t)rows * n;
+		if (count != total)
+			throw Error(E3D_ERR_ARG, name + ": count " + std::to_string(count) + " != " + std::to_string(total));
+		if (!pos_d_.n) {
+			std::vector<int> pos;
+			pos.reserve(NR_);
+			for (const auto& p : pos_) pos.insert(pos.end(), p.begin(), p.end());
+			pos_d_.upload(pos);
+		}
+		const size_t piece = std::min(total, kStageValues);
+		if (stage_.n < piece) stage_.alloc(piece);
+		for (size_t at = 0; at < total; at += piece) {
+			const size_t m = std::min(piece, total - at);
+			launch_state_out(layout, dev, layout == STATE_ROWS ? NR_ : NA_, n, r0, nr, g0, pos_d_.p + r0, at, m, stage_.p,
+			                 st_);
+			check("state out");
+			cuda_ok(cudaMemcpyAsync(dst + at, stage_.p, m * sizeof(double), cudaMemcpyDeviceToHost, st_), "d2h");
+		}
+		cuda_ok(cudaStreamSynchronize(st_), "sync");
 	};
-	auto packed_all = [&](auto* dev) {
-		out.assign((size_t)5 * na, 0.0);
-		d2h_packed(dev, NA_, r0, nr, out, 0, na, st_);
-		d2h_packed(dev, NA_, g0, ng, out, nr, na, st_);
-		to_local(b, out, 5, na);
-	};
+	const auto rows_real = [&](int rows, auto* dev) { bring(STATE_ROWS, rows, dev); };
+	const auto packed_all = [&](auto* dev) { bring(STATE_PACKED, 5, dev); };
 	if (delta_ && name != "prim" && name != "w0") throw Error(E3D_ERR_STATE, "only prim and w0 are readable in difference form");
 	if (delta_) {
 		rebase();  // differences folded into the base: base = full state
@@ -1226,22 +1207,7 @@ void Engine::get(const std::string& name, int b, std::vector<double>& out) {
 		packed_all(lim_.p);
 	} else if (name == "grad") {
 		require_fp64("grad download");
-		// device [cell][GRAD_LD] -> [var][cell][dim]
-		std::vector<double> t(GRAD_LD * (size_t)na);
-		for (int part = 0; part < 2; part++) {
-			const size_t n = part ? ng : nr, at = part ? nr : 0;
-			if (n)
-				cuda_ok(cudaMemcpyAsync(t.data() + GRAD_LD * at, grad_.p + GRAD_LD * (size_t)(part ? g0 : r0),
-				                        GRAD_LD * n * sizeof(double), cudaMemcpyDeviceToHost, st_),
-				        "d2h");
-		}
-		cuda_ok(cudaStreamSynchronize(st_), "sync");
-		out.resize((size_t)15 * na);
-		for (int c = 0; c < na; c++) {
-			const double* x = &t[GRAD_LD * (size_t)(c < nr ? pos_[b][c] : c)];
-			for (int q = 0; q < 5; q++)
-				for (int d = 0; d < 3; d++) out[((size_t)q * na + c) * 3 + d] = x[3 * q + d];
-		}
+		bring(STATE_GRAD, 15, grad_.p);
 	} else {
 		throw Error(E3D_ERR_ARG, "unknown state array '" + name + "'");
 	}
@@ -1866,19 +1832,7 @@ void Engine::widen_to_fp64() {
 	if (opt_.precision == PREC_FP64) return;
 	if (delta_) leave_delta();
 	cuda_ok(cudaStreamSynchronize(st_), "sync");
-	const bool need_gg = order_ == 2 && grad_kind_ == GRAD_GREEN_GAUSS;
-	const bool need_ls = order_ == 2 && grad_kind_ == GRAD_LEAST_SQUARES;
-	f64_.sgeo.alloc(4 * (size_t)NS_);
-	f64_.srv.alloc(3 * (size_t)NS_);
-	if (need_gg) f64_.sS.alloc(3 * (size_t)NS_);
-	launch_slot_geometry64(NS_, slot_face_.p, slot_mate_.p, S_.p, nhat_.p, area_.p, rl_.p, rr_.p, f64_.sgeo.p,
-	                       need_gg ? f64_.sS.p : nullptr, f64_.srv.p, st_);
-	if (need_ls) {
-		f64_.lsw.alloc(lsw64_.n);
-		cuda_ok(cudaMemcpyAsync(f64_.lsw.p, lsw64_.p, lsw64_.n * sizeof(double), cudaMemcpyDeviceToDevice, st_), "lsw");
-	}
-	f64_.vol.alloc(vol64_.n);
-	cuda_ok(cudaMemcpyAsync(f64_.vol.p, vol64_.p, vol64_.n * sizeof(double), cudaMemcpyDeviceToDevice, st_), "vol");
+	slot_geometry(f64_);
 	f64_.P0.alloc(5 * (size_t)NA_);
 	f64_.P1.alloc(5 * (size_t)NA_);
 	launch_widen_state(NA_, NR_, cur_ ? f32_.P1.p : f32_.P0.p, carry_ ? W0_.p : nullptr, ph_.gm1, f64_.P0.p,
@@ -1972,7 +1926,7 @@ void Engine::enter_delta() {
 	// every cell's base from the current state (real cells from the carried W,
 	// others from the FP32 primitives: ghosts that no condition or halo rewrites)
 	launch_widen_state(NA_, NR_, cur_ ? f32_.P1.p : f32_.P0.p, W0_.p, ph_.gm1, Pb64_.p, nullptr, st_);
-	launch_narrow_state(NA_, Pb64_.p, Pb32_.p, st_);
+	launch_convert<float>(Pb64_.n, Pb64_.p, Pb32_.p, st_);
 	cuda_ok(cudaMemsetAsync(dW_.p, 0, dW_.n * sizeof(float), st_), "memset");
 	cuda_ok(cudaMemsetAsync(f32_.P0.p, 0, f32_.P0.n * sizeof(float), st_), "memset");
 	cuda_ok(cudaMemsetAsync(f32_.P1.p, 0, f32_.P1.n * sizeof(float), st_), "memset");

@@ -182,7 +182,7 @@ public:
 	void sync();  // waits for queued work; throws on a CUDA error or a non-finite norm
 
 	// --- state transfer (block-local cell order, FP64 on the host side)
-	void get(const std::string& name, int block, std::vector<double>& out);
+	void get(const std::string& name, int block, double* dst, size_t count);
 	void set(const std::string& name, int block, const std::vector<double>& in);
 
 	int n_blocks() const { return nb_; }
@@ -220,9 +220,10 @@ private:
 	IterRecord make_record(int cs, const double* x, int nblocks, const int* n_real);
 	void require_exchanged(int n_iter) const;
 	void build_blocks(const std::vector<const HostBlock*>& blocks, const std::vector<Connexion>& conns);
-	void to_local(int b, std::vector<double>& a, int rows, int ld) const;
 	void to_device(int b, std::vector<double>& a, int rows, int ld) const;
 	void init_state();
+	template <class T>
+	void slot_geometry(Fused<T>& f);
 	void count_device_bytes();
 	void check(const char* what);
 	template <class T>
@@ -245,6 +246,9 @@ private:
 	std::vector<int> roff_, goff_, foff_, soff_;  // per block offsets (nb_+1)
 	std::vector<int> n_real_b_, n_all_b_;
 	std::vector<std::vector<int>> pos_;  // per block: device position (0..n_real-1) of each local real cell
+	DevBuf<int> pos_d_;                  // the same for all blocks, on first use
+	static constexpr size_t kStageValues = 1 << 22;
+	DevBuf<double> stage_;               // state on its way to the host
 	Physics ph_{};
 	double denom_ = 1.0, aoa_rad_ = 0.0;
 	int ncases_ = 1;

@@ -1,6 +1,7 @@
 // Surrogate inputs, warm-start state writes and FP32 -> FP64 widening.
 #include <cmath>
 
+#include "views.hpp"
 #include "warm.hpp"
 
 namespace e3d {
@@ -19,21 +20,22 @@ __device__ __forceinline__ int block_of(const int* __restrict__ roff, int nb, in
 	return lo;
 }
 
-__global__ void k_slot_geometry64(int NS, const int* __restrict__ slot_face, const int* __restrict__ slot_mate,
-                                  const double* __restrict__ S, const double* __restrict__ nhat,
-                                  const double* __restrict__ area, const double* __restrict__ rl,
-                                  const double* __restrict__ rr, double* __restrict__ sgeo, double* __restrict__ sS,
-                                  double* __restrict__ srv) {
+template <class T>
+__global__ void k_slot_geometry(int NS, const int* __restrict__ slot_face, const int* __restrict__ slot_mate,
+                                const double* __restrict__ S, const double* __restrict__ nhat,
+                                const double* __restrict__ area, const double* __restrict__ rl,
+                                const double* __restrict__ rr, T* __restrict__ sgeo, T* __restrict__ sS,
+                                T* __restrict__ srv) {
 	const int k = blockIdx.x * blockDim.x + threadIdx.x;
 	if (k >= NS) return;
 	const int F = slot_face[k];
 	const bool left = slot_mate[k] >= 0;
 	for (int d = 0; d < 3; d++) {
-		sgeo[4 * (size_t)k + d] = nhat[3 * (size_t)F + d];
-		if (sS) sS[3 * (size_t)k + d] = left ? S[3 * (size_t)F + d] : -S[3 * (size_t)F + d];
-		srv[3 * (size_t)k + d] = left ? rl[3 * (size_t)F + d] : rr[3 * (size_t)F + d];
+		sgeo[4 * (size_t)k + d] = (T)nhat[3 * (size_t)F + d];
+		if (sS) sS[3 * (size_t)k + d] = (T)(left ? S[3 * (size_t)F + d] : -S[3 * (size_t)F + d]);
+		srv[3 * (size_t)k + d] = (T)(left ? rl[3 * (size_t)F + d] : rr[3 * (size_t)F + d]);
 	}
-	sgeo[4 * (size_t)k + 3] = area[F];
+	sgeo[4 * (size_t)k + 3] = (T)area[F];
 }
 
 __global__ void k_widen_state(int NA, int NR, const float* __restrict__ P32, const double* __restrict__ W, double gm1,
@@ -60,9 +62,30 @@ __global__ void k_widen_state(int NA, int NR, const float* __restrict__ P32, con
 	}
 }
 
-__global__ void k_narrow_state(size_t n, const double* __restrict__ P64, float* __restrict__ P32) {
+template <class T>
+__global__ void k_convert(size_t n, const double* __restrict__ x, T* __restrict__ y) {
 	const size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
-	if (i < n) P32[i] = (float)P64[i];
+	if (i < n) y[i] = (T)x[i];
+}
+
+template <class T>
+__global__ void k_state_out(StateLayout layout, const T* __restrict__ dev, int ld, int n, int r0, int nr, int g0,
+                            const int* __restrict__ pos, size_t at, size_t m, double* __restrict__ out) {
+	const size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
+	if (t >= m) return;
+	size_t j = at + t;
+	int d = 0;
+	if (layout == STATE_GRAD) {  // [var][cell][dim]
+		d = (int)(j % 3);
+		j /= 3;
+	}
+	const int q = (int)(j / n), i = (int)(j % n);
+	const int c = i < nr ? r0 + pos[i] : g0 + (i - nr);
+	size_t src;
+	if (layout == STATE_GRAD) src = GRAD_LD * (size_t)c + 3 * q + d;
+	else if (layout == STATE_ROWS) src = q * (size_t)ld + c;
+	else src = q < 4 ? 4 * (size_t)c + q : 4 * (size_t)ld + c;
+	out[t] = (double)dev[src];
 }
 
 // Wall-face centres in FP32 and the box of each cluster of consecutive ones
@@ -248,21 +271,39 @@ void launch_prims_to_conservative(int NR, int NA, const T* P, double gamma, floa
 template void launch_prims_to_conservative<float>(int, int, const float*, double, float*, cudaStream_t);
 template void launch_prims_to_conservative<double>(int, int, const double*, double, float*, cudaStream_t);
 
-void launch_slot_geometry64(int NS, const int* slot_face, const int* slot_mate, const double* S, const double* nhat,
-                            const double* area, const double* rl, const double* rr, double* sgeo, double* sS,
-                            double* srv, cudaStream_t st) {
+template <class T>
+void launch_slot_geometry(int NS, const int* slot_face, const int* slot_mate, const double* S, const double* nhat,
+                          const double* area, const double* rl, const double* rr, T* sgeo, T* sS, T* srv,
+                          cudaStream_t st) {
 	if (NS > 0)
-		k_slot_geometry64<<<grid_for(NS), TPB, 0, st>>>(NS, slot_face, slot_mate, S, nhat, area, rl, rr, sgeo, sS, srv);
+		k_slot_geometry<T><<<grid_for(NS), TPB, 0, st>>>(NS, slot_face, slot_mate, S, nhat, area, rl, rr, sgeo, sS, srv);
 }
+template void launch_slot_geometry<float>(int, const int*, const int*, const double*, const double*, const double*,
+                                          const double*, const double*, float*, float*, float*, cudaStream_t);
+template void launch_slot_geometry<double>(int, const int*, const int*, const double*, const double*, const double*,
+                                           const double*, const double*, double*, double*, double*, cudaStream_t);
+
+template <class T>
+void launch_convert(size_t n, const double* x, T* y, cudaStream_t st) {
+	if (n > 0) k_convert<T><<<grid_for((long long)n), TPB, 0, st>>>(n, x, y);
+}
+template void launch_convert<float>(size_t, const double*, float*, cudaStream_t);
+template void launch_convert<double>(size_t, const double*, double*, cudaStream_t);
 
 void launch_widen_state(int NA, int NR, const float* P32, const double* W, double gm1, double* P0, double* P1,
                         cudaStream_t st) {
 	if (NA > 0) k_widen_state<<<grid_for(NA), TPB, 0, st>>>(NA, NR, P32, W, gm1, P0, P1);
 }
 
-void launch_narrow_state(int NA, const double* P64, float* P32, cudaStream_t st) {
-	if (NA > 0) k_narrow_state<<<grid_for(5LL * NA), TPB, 0, st>>>(5 * (size_t)NA, P64, P32);
+template <class T>
+void launch_state_out(StateLayout layout, const T* dev, int ld, int n, int r0, int nr, int g0, const int* pos, size_t at,
+                      size_t m, double* out, cudaStream_t st) {
+	if (m > 0) k_state_out<T><<<grid_for((long long)m), TPB, 0, st>>>(layout, dev, ld, n, r0, nr, g0, pos, at, m, out);
 }
+template void launch_state_out<float>(StateLayout, const float*, int, int, int, int, int, const int*, size_t, size_t,
+                                      double*, cudaStream_t);
+template void launch_state_out<double>(StateLayout, const double*, int, int, int, int, int, const int*, size_t, size_t,
+                                       double*, cudaStream_t);
 
 void launch_wall_clusters(int n, const int* first, const int* wall_face, const double* fc, float4* centre, float4* box,
                           cudaStream_t st) {

@@ -6,12 +6,16 @@
 
 namespace e3d {
 
-// Per-slot FP64 geometry of the fused path from the per-face arrays: unit
+// Per-slot geometry of the fused path from the FP64 per-face arrays: unit
 // normal and area (face orientation), area vector signed outward for the
 // slot's owner, and the owner's r-vector.  sS may be null.
-void launch_slot_geometry64(int NS, const int* slot_face, const int* slot_mate, const double* S, const double* nhat,
-                            const double* area, const double* rl, const double* rr, double* sgeo, double* sS,
-                            double* srv, cudaStream_t st);
+template <class T>
+void launch_slot_geometry(int NS, const int* slot_face, const int* slot_mate, const double* S, const double* nhat,
+                          const double* area, const double* rl, const double* rr, T* sgeo, T* sS, T* srv,
+                          cudaStream_t st);
+// n values in the working precision
+template <class T>
+void launch_convert(size_t n, const double* x, T* y, cudaStream_t st);
 
 // FP64 copy of an FP32 packed primitive state, into both ping-pong buffers
 // (only P0 when P1 is null).
@@ -19,9 +23,6 @@ void launch_slot_geometry64(int NS, const int* slot_face, const int* slot_mate, 
 // recomputed from it exactly; ghost cells are widened from P32.
 void launch_widen_state(int NA, int NR, const float* P32, const double* W, double gm1, double* P0, double* P1,
                         cudaStream_t st);
-
-// FP32 copy of an FP64 packed primitive state (all NA cells)
-void launch_narrow_state(int NA, const double* P64, float* P32, cudaStream_t st);
 
 // Wall faces in clusters of at most WALL_CLUSTER consecutive ones of one case
 // (cluster k: wall faces [first[k], first[k+1])): their centres and boxes.
@@ -52,5 +53,15 @@ void launch_apply_conservative(int c0, int n, int NR, int NA, int nb, const int*
 // floats (5 used).
 template <class T>
 void launch_prims_to_conservative(int NR, int NA, const T* P, double gamma, float* out, cudaStream_t st);
+
+// One block's state array in file order and double precision: values
+// [at, at + m) of [rows][n] into out.  Packed: five-variable arrays over all cells
+// (ld = NA); rows: [row][real cell] (ld = NR); grad: [cell][GRAD_LD] as
+// [var][cell][dim].  Real cell i of the block is device cell r0 + pos[i], ghost
+// nr + j is g0 + j.
+enum StateLayout : int { STATE_PACKED, STATE_ROWS, STATE_GRAD };
+template <class T>
+void launch_state_out(StateLayout layout, const T* dev, int ld, int n, int r0, int nr, int g0, const int* pos, size_t at,
+                      size_t m, double* out, cudaStream_t st);
 
 }  // namespace e3d
