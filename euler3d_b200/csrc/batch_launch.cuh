@@ -80,7 +80,8 @@ void flux_tiles(const FusedView<T>& v, const Physics& ph, bool order1, bool diss
 
 template <class T>
 cudaError_t launch_tiled_iterations(const FusedView<T>& v0, const FusedView<T>& v1, const Physics& ph,
-                                    const PersistArgs& a, int grad, int lim, int scheme, bool order2, cudaStream_t st) {
+                                    const PersistArgs& a, const ReduceArgs& r, int grad, int lim, int scheme, bool order2,
+                                    cudaStream_t st) {
 	if (a.n_work <= 0) return cudaSuccess;
 	int parity = a.start_parity;
 	for (int it = 0; it < a.iters; it++) {
@@ -109,11 +110,8 @@ cudaError_t launch_tiled_iterations(const FusedView<T>& v0, const FusedView<T>& 
 			else flux_tiles<T, FLUX_ROE>(v, ph, !order2, diss, al, be, last, a.carry, a.n_work, a.work, st);
 			parity ^= 1;
 		}
-		const FusedView<T>& vf = parity ? v1 : v0;
-		k_iter_tail<T><<<a.n_work, 128, 0, st>>>(vf, a);
-		k_iter_sums<<<a.nblocks, 128, 0, st>>>(a, it);
+		end_iteration<T>(parity ? v1 : v0, r, it, a.iters, st);
 	}
-	k_iter_add<<<1, 1, 0, st>>>(a.d_iter, a.iters);
 	return cudaGetLastError();
 }
 

@@ -412,7 +412,7 @@ inline int grid_of(long long n, int tpb) { return (int)((n + tpb - 1) / tpb); }
 namespace delta {
 
 cudaError_t launch_iterations(const FusedView<float>& v0, const FusedView<float>& v1, const Physics& ph,
-                              const PersistArgs& a, cudaStream_t st) {
+                              const PersistArgs& a, const ReduceArgs& r, cudaStream_t st) {
 	if (a.n_work <= 0) return cudaSuccess;
 	int parity = a.start_parity;
 	for (int it = 0; it < a.iters; it++) {
@@ -425,11 +425,8 @@ cudaError_t launch_iterations(const FusedView<float>& v0, const FusedView<float>
 			else k_delta_flux_tiles<false><<<a.n_work, 128, 0, st>>>(v, ph, al, be, last, a.work);
 			parity ^= 1;
 		}
-		const FusedView<float>& vf = parity ? v1 : v0;
-		k_iter_tail<float><<<a.n_work, 128, 0, st>>>(vf, a);
-		k_iter_sums<<<a.nblocks, 128, 0, st>>>(a, it);
+		end_iteration<float>(parity ? v1 : v0, r, it, a.iters, st);
 	}
-	k_iter_add<<<1, 1, 0, st>>>(a.d_iter, a.iters);
 	return cudaGetLastError();
 }
 

@@ -1422,6 +1422,7 @@ void Engine::build_work() {
 			}
 		bw[b + 1] = (int)work.size() / 4;
 	}
+	if (work == work_h_ && bw == block_work_h_) return;  // the list on the device, and a graph over it, stay
 	n_work_ = (int)work.size() / 4;
 	const size_t cap = 4 * ((size_t)NR_ / kPersistThreads + (size_t)nb_ + 1);
 	if (work_d_.n < cap) work_d_.alloc(cap);
@@ -1429,6 +1430,8 @@ void Engine::build_work() {
 	if (!work.empty())
 		cuda_ok(cudaMemcpyAsync(work_d_.p, work.data(), work.size() * sizeof(int), cudaMemcpyHostToDevice, st_), "work");
 	block_work_d_.upload(bw);
+	work_h_.swap(work);
+	block_work_h_.swap(bw);
 	if (pgraph_) {
 		cudaGraphExecDestroy(pgraph_);
 		pgraph_ = nullptr;
@@ -1505,18 +1508,20 @@ double Engine::run_persistent_t(int iters) {
 		}
 		return v;
 	};
-	a.Pb64 = delta_ ? Pb64_.p : nullptr;
+	ReduceArgs r = reduce_args(hist_d_.p, iter_d_.p, true);
+	r.block_work = block_work_d_.p;
+	r.Pb64 = delta_ ? Pb64_.p : nullptr;
 	const FusedView<T> v0 = view(false), v1 = view(true);
 	const int grid = tiled_ ? n_work_ : std::max(1, std::min(grid_, n_work_));
 	const bool fast = std::is_same<T, double>::value && fast64_;
 	auto launch = [&]() {
 		const bool o2 = order_ == 2;
 		if constexpr (std::is_same<T, float>::value)
-			if (delta_) return delta::launch_iterations(v0, v1, ph_, a, st_);
+			if (delta_) return delta::launch_iterations(v0, v1, ph_, a, r, st_);
 		if (fast)
-			return tiled_ ? batch_fast::launch_tiled_iterations<T>(v0, v1, ph_, a, grad_kind_, lim_kind_, scheme_, o2, st_)
+			return tiled_ ? batch_fast::launch_tiled_iterations<T>(v0, v1, ph_, a, r, grad_kind_, lim_kind_, scheme_, o2, st_)
 			              : batch_fast::launch_persistent<T>(v0, v1, ph_, a, grad_kind_, lim_kind_, scheme_, o2, grid, st_);
-		return tiled_ ? batch::launch_tiled_iterations<T>(v0, v1, ph_, a, grad_kind_, lim_kind_, scheme_, o2, st_)
+		return tiled_ ? batch::launch_tiled_iterations<T>(v0, v1, ph_, a, r, grad_kind_, lim_kind_, scheme_, o2, st_)
 		              : batch::launch_persistent<T>(v0, v1, ph_, a, grad_kind_, lim_kind_, scheme_, o2, grid, st_);
 	};
 	cudaEvent_t e0, e1;

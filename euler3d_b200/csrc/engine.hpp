@@ -304,6 +304,7 @@ private:
 	std::vector<char> case_active_, case_failed_;  // failed: residual turned non-finite in a batch solve
 	bool tolerate_nonfinite_ = false;
 	DevBuf<int> work_d_, block_work_d_;
+	std::vector<int> work_h_, block_work_h_;  // what they hold
 	DevBuf<double> wpart_d_;
 	int n_work_ = 0, tile_mult_ = 1, grid_ = 0;
 	Tuning tuning_;

@@ -12,7 +12,7 @@ template int batch::persistent_blocks_per_sm<float>(int, int, int, bool);
 template cudaError_t batch::launch_persistent<float>(const FusedView<float>&, const FusedView<float>&, const Physics&,
                                                      const PersistArgs&, int, int, int, bool, int, cudaStream_t);
 template cudaError_t batch::launch_tiled_iterations<float>(const FusedView<float>&, const FusedView<float>&,
-                                                           const Physics&, const PersistArgs&, int, int, int, bool,
+                                                           const Physics&, const PersistArgs&, const ReduceArgs&, int, int, int, bool,
                                                            cudaStream_t);
 
 }  // namespace e3d

@@ -90,6 +90,6 @@ template cudaError_t batch::launch_persistent<double>(const FusedView<double>&, 
                                                const PersistArgs&, int, int, int, bool, int, cudaStream_t);
 
 template cudaError_t batch::launch_tiled_iterations<double>(const FusedView<double>&, const FusedView<double>&, const Physics&,
-                                                    const PersistArgs&, int, int, int, bool, cudaStream_t);
+                                                    const PersistArgs&, const ReduceArgs&, int, int, int, bool, cudaStream_t);
 
 }  // namespace e3d

@@ -14,7 +14,7 @@ template cudaError_t batch_fast::launch_persistent<double>(const FusedView<doubl
                                                            const Physics&, const PersistArgs&, int, int, int, bool, int,
                                                            cudaStream_t);
 template cudaError_t batch_fast::launch_tiled_iterations<double>(const FusedView<double>&, const FusedView<double>&,
-                                                                 const Physics&, const PersistArgs&, int, int, int, bool,
+                                                                 const Physics&, const PersistArgs&, const ReduceArgs&, int, int, int, bool,
                                                                  cudaStream_t);
 
 }  // namespace e3d

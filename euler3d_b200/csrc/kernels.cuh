@@ -1201,7 +1201,8 @@ __global__ void __launch_bounds__(TAIL_TPB) k_tail(ReduceArgs a, const T* __rest
 	int w = blockIdx.x;
 	if (w < n_norm) {
 		const int b = w / a.max_chunks, ch = w - b * a.max_chunks;
-		const int beg = a.roff[b] + ch * TAIL_CHUNK, end = min(a.roff[b + 1], beg + TAIL_CHUNK);
+		const bool frozen = a.block_work && a.block_work[b] == a.block_work[b + 1];
+		const int beg = a.roff[b] + ch * TAIL_CHUNK, end = frozen ? beg : min(a.roff[b + 1], beg + TAIL_CHUNK);
 		double acc[5] = {0., 0., 0., 0., 0.};
 #pragma unroll
 		for (int j = 0; j < TAIL_CHUNK / TAIL_TPB; j++) {
@@ -1229,10 +1230,13 @@ __global__ void __launch_bounds__(TAIL_TPB) k_tail(ReduceArgs a, const T* __rest
 		const int i = w * TAIL_TPB + t;
 		if (i < a.n_wall) {
 			const int f = a.wall_face[i];
-			const T* p = P + 4 * (size_t)a.NA;
-			double o[5];
-			wall_face_terms((double)p[a.face_lr[2 * f]], (double)p[a.face_lr[2 * f + 1]],
-			                a.wall_denom ? a.wall_denom[i] : a.denom, a.S + 3 * (size_t)f, a.fc + 3 * (size_t)f, o);
+			const size_t i0 = 4 * (size_t)a.NA + a.face_lr[2 * f], i1 = 4 * (size_t)a.NA + a.face_lr[2 * f + 1];
+			double p0 = (double)P[i0], p1 = (double)P[i1], o[5];
+			if (a.Pb64) {
+				p0 += a.Pb64[i0];
+				p1 += a.Pb64[i1];
+			}
+			wall_face_terms(p0, p1, a.wall_denom ? a.wall_denom[i] : a.denom, a.S + 3 * (size_t)f, a.fc + 3 * (size_t)f, o);
 #pragma unroll
 			for (int q = 0; q < 5; q++) a.wall_terms[((size_t)slot * 5 + q) * a.n_wall + i] = o[q];
 		}
@@ -1288,8 +1292,6 @@ __global__ void __launch_bounds__(160) k_tail_sums(ReduceArgs a, int advance) {
 	}
 }
 
-constexpr int WALL_CHUNK = 1024;
-
 // ===================================================================== batches
 // Phases of one outer iteration over a work list (tiles of real cells of the
 // active cases), shared by the persistent kernel and the tiled per-pass
@@ -1321,20 +1323,11 @@ template <class T>
 __device__ __forceinline__ void wall_terms_range(const FusedView<T>& vf, const PersistArgs& a, int i0, int stride) {
 	for (int i = i0; i < a.n_wall; i += stride) {
 		const int f = a.wall_face[i];
-		const size_t i0 = 4 * (size_t)vf.NA + a.face_lr[2 * f], i1 = 4 * (size_t)vf.NA + a.face_lr[2 * f + 1];
-		double p0 = (double)vf.Pin[i0], p1 = (double)vf.Pin[i1];
-		if (a.Pb64) {  // difference form: base + difference
-			p0 += a.Pb64[i0];
-			p1 += a.Pb64[i1];
-		}
-		const double cp = (0.5 * (p0 + p1) - 1.) / (a.wall_denom ? a.wall_denom[i] : a.denom);
-		const double fx = cp * a.S[3 * f], fy = cp * a.S[3 * f + 1], fz = cp * a.S[3 * f + 2];
-		const double x = a.fc[3 * f], y = a.fc[3 * f + 1], z = a.fc[3 * f + 2];
-		a.wall_terms[i] = fy;
-		a.wall_terms[(size_t)a.n_wall + i] = fx;
-		a.wall_terms[2 * (size_t)a.n_wall + i] = y * fz - z * fy;
-		a.wall_terms[3 * (size_t)a.n_wall + i] = z * fx - x * fz;
-		a.wall_terms[4 * (size_t)a.n_wall + i] = x * fy - y * fx;
+		const T* p = vf.Pin + 4 * (size_t)vf.NA;
+		double o[5];
+		wall_face_terms((double)p[a.face_lr[2 * f]], (double)p[a.face_lr[2 * f + 1]],
+		                a.wall_denom ? a.wall_denom[i] : a.denom, a.S + 3 * (size_t)f, a.fc + 3 * (size_t)f, o);
+		for (int q = 0; q < 5; q++) a.wall_terms[q * (size_t)a.n_wall + i] = o[q];
 	}
 }
 
@@ -1351,9 +1344,8 @@ __device__ __forceinline__ void halo_range(const FusedView<T>& vf, const Persist
 // Per-block sums of block b into history slot `slot`: tiles in a fixed tree
 // order, wall faces sequentially in the reference's order.
 template <int TPB>
-__device__ __forceinline__ void block_sums(const PersistArgs& a, int b, int slot, double (*red)[TPB],
-                                           double (*wbuf)[WALL_CHUNK / 4]) {
-	const int w0 = a.block_work[b], w1 = a.block_work[b + 1];
+__device__ __forceinline__ void block_sums(const PersistArgs& a, int b, int slot, double (*red)[TPB], double (*wbuf)[128]) {
+	const int w0 = a.block_work[b], w1 = a.block_work[b + 1], warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 	double acc[5] = {0., 0., 0., 0., 0.};
 	for (int w = w0 + threadIdx.x; w < w1; w += TPB)
 		for (int q = 0; q < 5; q++) acc[q] += a.wpart[(size_t)w * 5 + q];
@@ -1370,20 +1362,10 @@ __device__ __forceinline__ void block_sums(const PersistArgs& a, int b, int slot
 		if (!isfinite(red[threadIdx.x][0]) && w1 > w0) *a.d_bad = 1;
 	}
 	const int beg = a.wall_off[b], end = a.wall_off[b + 1];
-	double fs = 0.;
-	constexpr int CH = WALL_CHUNK / 4;
-	for (int base_i = beg; base_i < end; base_i += CH) {
-		const int n = min(CH, end - base_i);
-		__syncthreads();
-		for (int j = threadIdx.x; j < 5 * n; j += TPB) {
-			const int q = j / n, i = j - q * n;
-			wbuf[q][i] = a.wall_terms[(size_t)q * a.n_wall + base_i + i];
-		}
-		__syncthreads();
-		if (threadIdx.x < 5)
-			for (int i = 0; i < n; i++) fs += wbuf[threadIdx.x][i];
+	for (int q = warp; q < 5; q += TPB / 32) {
+		const double f = warp_ordered_sum(a.wall_terms + q * (size_t)a.n_wall + beg, end - beg, wbuf[warp]);
+		if (lane == 0) out[5 + q] = f;
 	}
-	if (threadIdx.x < 5) out[5 + threadIdx.x] = fs;
 	__syncthreads();
 }
 
@@ -1396,7 +1378,7 @@ __global__ void __launch_bounds__(TPB, 512 / TPB) k_persistent(FusedView<T> v0, 
 	namespace cg = cooperative_groups;
 	cg::grid_group grid = cg::this_grid();
 	__shared__ double red[5][TPB];
-	__shared__ double wbuf[5][WALL_CHUNK / 4];
+	__shared__ __align__(16) double wbuf[TPB / 32][128];
 	const int base = *a.d_iter;
 	int parity = a.start_parity;  // which primitive buffer holds the current state
 	for (int it = 0; it < a.iters; it++) {
@@ -1468,25 +1450,6 @@ __global__ void __launch_bounds__(128, sizeof(T) == 4 ? 8 : 4) k_flux_update_til
 	const int c = t.x + threadIdx.x;
 	if (c < t.y) flux_update_cell<T, SCHEME, ORDER1, 4, DISS>(v, ph, alpha, beta, last, carry_w0, c);
 }
-
-// end of an iteration, part 1 (grid = n_work): tile norms, wall terms, halo
-template <class T>
-__global__ void __launch_bounds__(128) k_iter_tail(FusedView<T> vf, PersistArgs a) {
-	__shared__ double red[5][128];
-	tile_norms<T, 128>(vf, a, blockIdx.x, red);
-	wall_terms_range(vf, a, blockIdx.x * 128 + threadIdx.x, gridDim.x * 128);
-	halo_range(vf, a, blockIdx.x * 128 + threadIdx.x, gridDim.x * 128);
-}
-
-// end of an iteration, part 2 (grid = nblocks): per-block sums into history slot *d_iter + it
-__global__ void __launch_bounds__(128) k_iter_sums(PersistArgs a, int it) {
-	__shared__ double red[5][128];
-	__shared__ double wbuf[5][WALL_CHUNK / 4];
-	const int slot = min(*a.d_iter + it, a.hist_capacity - 1);
-	block_sums<128>(a, blockIdx.x, slot, red, wbuf);
-}
-
-__global__ void k_iter_add(int* d_iter, int n) { *d_iter += n; }
 
 }  // namespace
 }  // namespace e3d

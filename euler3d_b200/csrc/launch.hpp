@@ -40,6 +40,14 @@ void launch_tail(const ReduceArgs&, const T* Rc, const T* Rd, T* P, T* P2, cudaS
 // n: pending iterations; advance: move *d_iter on by n
 void launch_tail_sums(const ReduceArgs&, int n, bool advance, cudaStream_t);
 
+// tail of iteration `it` of `iters` of a batch launch (current state in v.Pin), with the sums once the ring is full
+template <class T>
+void end_iteration(const FusedView<T>& v, const ReduceArgs& r, int it, int iters, cudaStream_t st) {
+	launch_tail<T>(r, v.Rc, v.Rd, const_cast<T*>(v.Pin), v.Pout, st);
+	const int in_ring = it % TAIL_SLOTS + 1;
+	if (in_ring == TAIL_SLOTS || it == iters - 1) launch_tail_sums(r, in_ring, true, st);
+}
+
 // ---- fused stage kernels ----
 template <class T>
 void launch_recon(const FusedView<T>&, const Physics&, int grad, int lim, bool first, int carry, cudaStream_t);
@@ -61,7 +69,8 @@ cudaError_t launch_persistent(const FusedView<T>& v0, const FusedView<T>& v1, co
 // the same iterations as separate per-pass launches over the work list
 template <class T>
 cudaError_t launch_tiled_iterations(const FusedView<T>& v0, const FusedView<T>& v1, const Physics& ph,
-                                    const PersistArgs& a, int grad, int lim, int scheme, bool order2, cudaStream_t st);
+                                    const PersistArgs& a, const ReduceArgs& r, int grad, int lim, int scheme, bool order2,
+                                    cudaStream_t st);
 }  // namespace batch
 namespace batch_fast {
 template <class T>
@@ -72,14 +81,15 @@ cudaError_t launch_persistent(const FusedView<T>& v0, const FusedView<T>& v1, co
 // the same iterations as separate per-pass launches over the work list
 template <class T>
 cudaError_t launch_tiled_iterations(const FusedView<T>& v0, const FusedView<T>& v1, const Physics& ph,
-                                    const PersistArgs& a, int grad, int lim, int scheme, bool order2, cudaStream_t st);
+                                    const PersistArgs& a, const ReduceArgs& r, int grad, int lim, int scheme, bool order2,
+                                    cudaStream_t st);
 }  // namespace batch_fast
 
 // FP32 iterations in difference form (delta.cu): first-order AUSM, all-tetrahedron
 // meshes, tiled per-pass form.  v0/v1 carry the base and difference arrays.
 namespace delta {
 cudaError_t launch_iterations(const FusedView<float>& v0, const FusedView<float>& v1, const Physics& ph,
-                              const PersistArgs& a, cudaStream_t st);
+                              const PersistArgs& a, const ReduceArgs& r, cudaStream_t st);
 // new base state from W_b + dW (Wb: the FP64 base conserved state, updated in
 // place), base ghosts, base residual in FP64; differences d0, d1 cleared
 void launch_rebase(const FusedView<float>& v, const Physics& ph, double* Wb, const double* area64, int n_halo,

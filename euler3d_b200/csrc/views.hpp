@@ -124,6 +124,8 @@ struct ReduceArgs {
 	int* d_bad;
 	int* pend;             // iterations in the ring
 	unsigned* ticket;      // blocks of the running launch that are done
+	const int* block_work; // batches: nblocks+1 work-item offsets, a block without items is frozen; else null
+	const double* Pb64;    // difference form: FP64 base primitives (wall pressures are base + difference), else null
 };
 
 // One launch of the persistent batch kernel: several outer iterations over the
@@ -159,8 +161,6 @@ struct PersistArgs {
 	int n_halo;
 	const int* halo_dst;
 	const int* halo_src;
-	// difference form: FP64 base primitives (wall pressures are base + difference), else null
-	const double* Pb64;
 };
 
 }  // namespace e3d

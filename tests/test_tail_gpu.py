@@ -32,3 +32,21 @@ def test_ring_matches_single_iterations(n, blocks, iters, tmp_path):
     a.close()
     b.close()
     case.close()
+
+
+# the same ring inside one batch launch
+@pytest.mark.parametrize("iters", [31, 32, 33, 70])
+def test_batch_ring(iters, tmp_path, monkeypatch):
+    monkeypatch.setenv("E3D_BATCH_FORM", "per-pass")
+    cases = [api.Case(mg.write_case(str(tmp_path / str(n)), n, deck=mg.Deck(topology="", mach=0.5, flux="ausm")))
+             for n in (5, 8)]
+    a, b = (api.Batch(cases, precision="fp64") for _ in range(2))
+    a.solve_batch(iters, -1e300, iters_per_launch=iters)
+    b.solve_batch(iters, -1e300, iters_per_launch=1)
+    for c in range(2):
+        ha, hb = a.case_history(c), b.case_history(c)
+        assert len(ha["iter"]) == iters
+        for k in ha:
+            assert np.array_equal(ha[k], hb[k]), (c, k)
+    a.close()
+    b.close()
