@@ -506,7 +506,7 @@ void Engine::count_device_bytes() {
 	                &f64_.lsw, &f64_.vol})
 		bytes += b->n * sizeof(double);
 	for (auto* b : {&f32_.P0, &f32_.P1, &f32_.FS, &f32_.Rc, &f32_.Rd, &f32_.dt, &f32_.sgeo, &f32_.sS, &f32_.srv,
-	                &f32_.lsw, &f32_.vol, &Pb32_, &dW_, &Rb_})
+	                &f32_.lsw, &f32_.vol, &Pb32_, &dW_, &Rb_, &rec_})
 		bytes += b->n * sizeof(float);
 	bytes += Pb64_.n * sizeof(double);
 	dev_bytes_ = bytes;
@@ -1501,6 +1501,7 @@ double Engine::run_persistent_t(int iters) {
 		if (delta_) {
 			v.Pb = Pb32_.p;
 			v.Pb64 = Pb64_.p;
+			if constexpr (std::is_same<T, float>::value) delta_records(v, flip);
 			v.dW = dW_.p;
 			v.Rb = Rb_.p;
 			v.slot_face = slot_face_.p;
@@ -1900,11 +1901,19 @@ FusedView<float> Engine::delta_view(bool flip) const {
 	v.gcase = gcase_d_.p;
 	v.Pb = Pb32_.p;
 	v.Pb64 = Pb64_.p;
+	delta_records(v, flip);
 	v.dW = dW_.p;
 	v.Rb = Rb_.p;
 	v.slot_face = slot_face_.p;
 	v.nhat64 = nhat_.p;
 	return v;
+}
+
+void Engine::delta_records(FusedView<float>& v, bool flip) const {
+	const size_t n = 8 * (size_t)NA_;
+	v.rec_base = rec_.p;
+	v.rec_in = rec_.p + (flip ? 2 : 1) * n;
+	v.rec_out = rec_.p + (flip ? 1 : 2) * n;
 }
 
 // W_b <- W_b + dW, base primitives and ghosts from it, base residual in FP64,
@@ -1928,6 +1937,7 @@ void Engine::enter_delta() {
 	Pb64_.alloc(5 * (size_t)NA_);
 	dW_.alloc(5 * (size_t)NR_);
 	Rb_.alloc(5 * (size_t)NR_);
+	rec_.alloc(24 * (size_t)NA_);
 	// every cell's base from the current state (real cells from the carried W,
 	// others from the FP32 primitives: ghosts that no condition or halo rewrites)
 	launch_widen_state(NA_, NR_, cur_ ? f32_.P1.p : f32_.P0.p, W0_.p, ph_.gm1, Pb64_.p, nullptr, st_);
@@ -1966,7 +1976,7 @@ void Engine::leave_delta() {
 	cuda_ok(cudaMemcpyAsync(f32_.P0.p, Pb32_.p, Pb32_.n * sizeof(float), cudaMemcpyDeviceToDevice, st_), "d2d");
 	cuda_ok(cudaMemcpyAsync(f32_.P1.p, Pb32_.p, Pb32_.n * sizeof(float), cudaMemcpyDeviceToDevice, st_), "d2d");
 	cuda_ok(cudaStreamSynchronize(st_), "sync");
-	for (auto* b : {&Pb32_, &dW_, &Rb_}) b->free();
+	for (auto* b : {&Pb32_, &dW_, &Rb_, &rec_}) b->free();
 	Pb64_.free();
 	delta_ = false;
 	if (pgraph_) {

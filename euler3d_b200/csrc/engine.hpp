@@ -325,6 +325,8 @@ private:
 	// differences, base residual; W0_ holds the FP64 base conserved state
 	bool delta_ = false;
 	DevBuf<float> Pb32_, dW_, Rb_;
+	DevBuf<float> rec_;  // base records, then the difference records of either buffer, 8 NA each
+	void delta_records(FusedView<float>& v, bool flip) const;
 	DevBuf<double> Pb64_;
 	FusedView<float> delta_view(bool flip) const;
 	void rebase();

@@ -1247,6 +1247,14 @@ __global__ void __launch_bounds__(TAIL_TPB) k_tail(ReduceArgs a, const T* __rest
 			const Q5<T> q = ld5(P, a.NA, a.halo_src[i]);
 			st5(P, a.NA, d, q);
 			st5(P2, a.NA, d, q);
+			if (a.rec) {
+				const float4* r = reinterpret_cast<const float4*>(a.rec + 8 * (size_t)a.halo_src[i]);
+				const float4 x = r[0], y = r[1];
+				for (float* o : {a.rec, a.rec2}) {
+					reinterpret_cast<float4*>(o + 8 * (size_t)d)[0] = x;
+					reinterpret_cast<float4*>(o + 8 * (size_t)d)[1] = y;
+				}
+			}
 		}
 	}
 	__syncthreads();

@@ -43,7 +43,10 @@ void launch_tail_sums(const ReduceArgs&, int n, bool advance, cudaStream_t);
 // tail of iteration `it` of `iters` of a batch launch (current state in v.Pin), with the sums once the ring is full
 template <class T>
 void end_iteration(const FusedView<T>& v, const ReduceArgs& r, int it, int iters, cudaStream_t st) {
-	launch_tail<T>(r, v.Rc, v.Rd, const_cast<T*>(v.Pin), v.Pout, st);
+	ReduceArgs a = r;
+	a.rec = const_cast<float*>(v.rec_in);
+	a.rec2 = v.rec_out;
+	launch_tail<T>(a, v.Rc, v.Rd, const_cast<T*>(v.Pin), v.Pout, st);
 	const int in_ring = it % TAIL_SLOTS + 1;
 	if (in_ring == TAIL_SLOTS || it == iters - 1) launch_tail_sums(r, in_ring, true, st);
 }

@@ -89,6 +89,9 @@ struct FusedView {
 	// differences from the FP64 base W_b, Rb the FP64-evaluated base residual
 	const float* Pb;          // 5*NA
 	const double* Pb64;       // 5*NA
+	const float* rec_base;    // 8*NA per-cell flux quantities of the base state
+	const float* rec_in;      // 8*NA and their differences, of Pin
+	float* rec_out;           // 8*NA of Pout
 	float* dW;                // 5*NR
 	float* Rb;                // 5*NR
 	const int* slot_face;     // NS  (FP64 face normals of boundary slots)
@@ -126,6 +129,7 @@ struct ReduceArgs {
 	unsigned* ticket;      // blocks of the running launch that are done
 	const int* block_work; // batches: nblocks+1 work-item offsets, a block without items is frozen; else null
 	const double* Pb64;    // difference form: FP64 base primitives (wall pressures are base + difference), else null
+	float *rec, *rec2;     // difference form: 8 values a cell of either buffer, copied with the halo; else null
 };
 
 // One launch of the persistent batch kernel: several outer iterations over the
