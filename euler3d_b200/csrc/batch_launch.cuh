@@ -62,19 +62,19 @@ cudaError_t launch_persistent(const FusedView<T>& v0, const FusedView<T>& v1, co
 template <class T, int GRAD, int LIM>
 void recon_tiles(const FusedView<T>& v, const Physics& ph, int carry, bool first, int n_work, const int4* work,
                  cudaStream_t st) {
-	if (first) k_recon_tiles<T, GRAD, LIM, true><<<n_work, 128, 0, st>>>(v, ph, carry, work);
-	else k_recon_tiles<T, GRAD, LIM, false><<<n_work, 128, 0, st>>>(v, ph, carry, work);
+	if (first) launch_next(k_recon_tiles<T, GRAD, LIM, true>, n_work, 128, 0, st, v, ph, carry, work);
+	else launch_next(k_recon_tiles<T, GRAD, LIM, false>, n_work, 128, 0, st, v, ph, carry, work);
 }
 
 template <class T, int SCHEME>
 void flux_tiles(const FusedView<T>& v, const Physics& ph, bool order1, bool diss, T al, T be, int last, int carry,
                 int n_work, const int4* work, cudaStream_t st) {
 	if (order1) {
-		if (diss) k_flux_update_tiles<T, SCHEME, true, true><<<n_work, 128, 0, st>>>(v, ph, al, be, last, carry, work);
-		else k_flux_update_tiles<T, SCHEME, true, false><<<n_work, 128, 0, st>>>(v, ph, al, be, last, carry, work);
+		if (diss) launch_next(k_flux_update_tiles<T, SCHEME, true, true>, n_work, 128, 0, st, v, ph, al, be, last, carry, work);
+		else launch_next(k_flux_update_tiles<T, SCHEME, true, false>, n_work, 128, 0, st, v, ph, al, be, last, carry, work);
 	} else {
-		if (diss) k_flux_update_tiles<T, SCHEME, false, true><<<n_work, 128, 0, st>>>(v, ph, al, be, last, carry, work);
-		else k_flux_update_tiles<T, SCHEME, false, false><<<n_work, 128, 0, st>>>(v, ph, al, be, last, carry, work);
+		if (diss) launch_next(k_flux_update_tiles<T, SCHEME, false, true>, n_work, 128, 0, st, v, ph, al, be, last, carry, work);
+		else launch_next(k_flux_update_tiles<T, SCHEME, false, false>, n_work, 128, 0, st, v, ph, al, be, last, carry, work);
 	}
 }
 
@@ -101,7 +101,7 @@ cudaError_t launch_tiled_iterations(const FusedView<T>& v0, const FusedView<T>& 
 						recon_tiles<T, GRAD_GREEN_GAUSS, LIM_BARTH_JESPERSEN>(v, ph, a.carry, first, a.n_work, a.work, st);
 				}
 			} else if (s == 0) {
-				k_start_tiles<T><<<a.n_work, 128, 0, st>>>(v, ph, a.carry, a.work);
+				launch_next(k_start_tiles<T>, a.n_work, 128, 0, st, v, ph, a.carry, a.work);
 			}
 			const T al = T(a.alpha[s]), be = T(a.beta[s]);
 			const int last = s == a.stages - 1;

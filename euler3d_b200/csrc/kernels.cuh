@@ -74,6 +74,15 @@ __device__ __forceinline__ T& qv(Q5<T>& q, int v) { return (&q.r)[v]; }
 template <class T>
 __device__ __forceinline__ T qv(const Q5<T>& q, int v) { return (&q.r)[v]; }
 
+// Launched with programmatic serialization (launch_next): the next kernel's blocks
+// may take their places while this one's last blocks run, and every kernel waits
+// here for all memory of the one before it.  Only data that no kernel of an
+// iteration writes (topology, geometry) may be read before the wait.
+__device__ __forceinline__ void start_after_previous() {
+	cudaTriggerProgrammaticLaunchCompletion();
+	cudaGridDependencySynchronize();
+}
+
 // Thread index -> cell of a per-block range: real cells [r0, r1) then ghost
 // cells [NR+g0, NR+g1).
 __device__ __forceinline__ int range_cell(int t, int r0, int r1, int NR, int g0, int g1) {
@@ -87,6 +96,7 @@ __device__ __forceinline__ int range_cell(int t, int r0, int r1, int NR, int g0,
 // ===================================================================== granular
 // Solver::saveW0 (Solver/src/Solver.cpp:161-210).
 __global__ void k_save_w0(GeoView g, StateView s, Physics ph, int r0, int r1) {
+	start_after_previous();
 	const int c = r0 + blockIdx.x * blockDim.x + threadIdx.x;
 	if (c >= r1) return;
 	const Q5<double> q = ld5(s.prim, g.NA, c);
@@ -101,6 +111,7 @@ __global__ void k_save_w0(GeoView g, StateView s, Physics ph, int r0, int r1) {
 // Timestep::computeSpectralRadius (Solver/src/Timestep.cpp:26-121): the cell's
 // own state on every face.
 __global__ void k_spectral_radius(GeoView g, StateView s, Physics ph, int r0, int r1) {
+	start_after_previous();
 	const int c = r0 + blockIdx.x * blockDim.x + threadIdx.x;
 	if (c >= r1) return;
 	const Q5<double> q = ld5(s.prim, g.NA, c);
@@ -116,6 +127,7 @@ __global__ void k_spectral_radius(GeoView g, StateView s, Physics ph, int r0, in
 
 // Timestep::computeTimestep (Timestep.cpp:123-148).
 __global__ void k_timestep(GeoView g, StateView s, Physics ph, int r0, int r1) {
+	start_after_previous();
 	const int c = r0 + blockIdx.x * blockDim.x + threadIdx.x;
 	if (c >= r1) return;
 	s.dt[c] = ph.cfl * g.vol[c] / s.srad[c];
@@ -152,6 +164,7 @@ __device__ __forceinline__ double ld5q(const double* __restrict__ P, int n, int 
 // LeastSquares::computeGradients (Solver/src/LeastSquares.cpp:80-119), five lanes per cell.
 template <int GRAD>
 __global__ void k_grad(GeoView g, StateView s, int r0, int r1) {
+	start_after_previous();
 	const int t = blockIdx.x * blockDim.x + threadIdx.x, c = r0 + t / 5, v = t % 5;
 	if (c >= r1) return;
 	double gr[3] = {0.0, 0.0, 0.0};
@@ -185,6 +198,7 @@ __global__ void k_grad(GeoView g, StateView s, int r0, int r1) {
 // (Solver/src/BarthJespersen.cpp:88-331, Venkatakrishnan.cpp:87-324), all cells, five lanes per cell.
 template <int LIM>
 __global__ void k_limiter(GeoView g, StateView s, Physics ph, int r0, int r1, int g0, int g1) {
+	start_after_previous();
 	const int t = blockIdx.x * blockDim.x + threadIdx.x, v = t % 5;
 	const int c = range_cell(t / 5, r0, r1, g.NR, g0, g1);
 	if (c < 0) return;
@@ -239,6 +253,7 @@ __device__ __forceinline__ Q5<double> face_state(const GeoView& g, const StateVi
 // AusmScheme.cpp:84-243), Rd <- (1-beta) Rd + beta * D.
 template <int SCHEME, bool DISS, int LPC>
 __global__ void __launch_bounds__(128, 6) k_flux(GeoView g, StateView s, Physics ph, double beta, int r0, int r1) {
+	start_after_previous();
 	__shared__ double sm[4][5][33];
 	const int lane = threadIdx.x & 31, k = lane & (LPC - 1), first = lane - k;
 	const int c = r0 + (blockIdx.x * 128 + threadIdx.x) / LPC;
@@ -309,6 +324,7 @@ __device__ __forceinline__ Q5<T> conservative_update(const double w0[5], T coef,
 }
 
 __global__ void k_update(GeoView g, StateView s, Physics ph, double alpha, int r0, int r1) {
+	start_after_previous();
 	const int c = r0 + blockIdx.x * blockDim.x + threadIdx.x;
 	if (c >= r1) return;
 	const int n = g.NR;
@@ -332,6 +348,7 @@ __device__ __forceinline__ Q5<T> ghost_state(int kind, const Q5<T>& qi, const Q5
 }
 
 __global__ void k_bc(GeoView g, StateView s, Physics ph, int g0, int g1) {
+	start_after_previous();
 	const int t = blockIdx.x * blockDim.x + threadIdx.x;
 	if (t >= g1 - g0) return;
 	const int gi = g0 + t, c = g.NR + gi;
@@ -364,6 +381,7 @@ __global__ void k_bc(GeoView g, StateView s, Physics ph, int g0, int g1) {
 constexpr double IRS_EPS = 0.8;
 // One thread per (cell, array): blockIdx.y = 0..4 convective, 5..9 dissipative.
 __global__ void k_irs_start(GeoView g, StateView s, double* __restrict__ j1, int r0, int r1) {
+	start_after_previous();
 	const int c = r0 + blockIdx.x * blockDim.x + threadIdx.x, q = blockIdx.y;
 	if (c >= r1) return;
 	const int na = g.slot_ptr[c + 1] - g.slot_ptr[c];
@@ -374,6 +392,7 @@ __global__ void k_irs_start(GeoView g, StateView s, double* __restrict__ j1, int
 // Pass 2: R = (R + eps * sum of J1 over the real neighbours in slot order) / (1 + eps N),
 // in place (each thread reads only its own R and the neighbours' J1).
 __global__ void k_irs_smooth(GeoView g, StateView s, const double* __restrict__ j1, int r0, int r1) {
+	start_after_previous();
 	const int c = r0 + blockIdx.x * blockDim.x + threadIdx.x, q = blockIdx.y;
 	if (c >= r1) return;
 	const int k0 = g.slot_ptr[c], k1 = g.slot_ptr[c + 1];
@@ -389,6 +408,7 @@ __global__ void k_irs_smooth(GeoView g, StateView s, const double* __restrict__ 
 
 template <class T>
 __global__ void k_halo(int n, const int* __restrict__ dst, const int* __restrict__ src, int NA, T* b0, T* b1) {
+	start_after_previous();
 	const int t = blockIdx.x * blockDim.x + threadIdx.x;
 	if (t >= n) return;
 	const int d = dst[t], o = src[t];
@@ -735,6 +755,7 @@ __device__ __forceinline__ void recon_cell(const FusedView<T>& v, const Physics&
 #endif
 template <class T, int GRAD, int LIM, bool FIRST, int NSL>
 __global__ void __launch_bounds__(128, sizeof(T) == 4 ? E3D_RECON_MIN_BLOCKS : E3D_FP64_MIN_BLOCKS) k_recon(FusedView<T> v, Physics ph, int carry_w0) {
+	start_after_previous();
 	const int c = blockIdx.x * blockDim.x + threadIdx.x;
 	if (c < v.NR) recon_cell<T, GRAD, LIM, FIRST, NSL>(v, ph, carry_w0, c);
 }
@@ -772,18 +793,24 @@ __device__ __forceinline__ void stq(T* __restrict__ P, int n, int c, int q, T x)
 template <class T, int GRAD, int LIM, int NSL>
 __global__ void __launch_bounds__(5 * RV_CELLS, E3D_RV_MIN_BLOCKS) k_recon_var(FusedView<T> v, Physics ph) {
 	const int c = blockIdx.x * RV_CELLS + threadIdx.x / 5, q = threadIdx.x % 5;
-	if (c >= v.NR) return;
+	if (c >= v.NR) return start_after_previous();
 	const SlotRange<T, NSL> sr(v, c);
-	const T q0 = ldq(v.Pin, v.NA, c, q);
 	int nb[MAXSL];
-	if (NSL == 4) load_int<T, NSL>(v.slot_nbr, sr, nb);
+	if (NSL == 4) {
+		load_int<T, NSL>(v.slot_nbr, sr, nb);
+	} else {
+#pragma unroll
+		E3D_SLOTS(k, sr) nb[k] = __ldg(v.slot_nbr + sr.s0 + k);
+	}
+	const T V = v.vol[c];
+	start_after_previous();
+	const T q0 = ldq(v.Pin, v.NA, c, q);
 	T gr[3] = {T(0.0), T(0.0), T(0.0)};
 	T mx = q0, mn = q0;
 	{
 		const T* __restrict__ wa = (GRAD == GRAD_GREEN_GAUSS ? v.sS : v.lsw) + 3 * (size_t)sr.s0;
 #pragma unroll
 		E3D_SLOTS(k, sr) {
-			if (NSL != 4) nb[k] = __ldg(v.slot_nbr + sr.s0 + k);
 			const T w[3] = {__ldg(wa + 3 * k), __ldg(wa + 3 * k + 1), __ldg(wa + 3 * k + 2)};
 			const T qn = ldq(v.Pin, v.NA, nb[k], q);
 			if (GRAD == GRAD_GREEN_GAUSS) {
@@ -801,7 +828,6 @@ __global__ void __launch_bounds__(5 * RV_CELLS, E3D_RV_MIN_BLOCKS) k_recon_var(F
 			if (qn < mn) mn = qn;
 		}
 	}
-	const T V = v.vol[c];
 	if (GRAD == GRAD_GREEN_GAUSS)
 		for (int d = 0; d < 3; d++) gr[d] /= V;
 	const T* __restrict__ ra = v.srv + 3 * (size_t)sr.s0;
@@ -850,9 +876,14 @@ __global__ void __launch_bounds__(5 * RV_CELLS, E3D_RV_MIN_BLOCKS) k_recon_var(F
 }
 
 // W0 and the local time step without a reconstruction pass (first order).
-template <class T, int NSL>
+// WAIT: behind the previous kernel, with the geometry already on its way.
+template <class T, int NSL, bool WAIT = false>
 __device__ __forceinline__ void start_cell(const FusedView<T>& v, const Physics& ph, int carry_w0, int c) {
 	const SlotRange<T, NSL> sr(v, c);
+	T geo[MAXSL][4];
+	load_geo<T, NSL>(v.sgeo, sr, geo);
+	const T V = v.vol[c];
+	if (WAIT) start_after_previous();
 	const Q5<T> q0 = ld5(v.Pin, v.NA, c);
 	if (!carry_w0) {
 		const int n = v.NR;
@@ -863,19 +894,18 @@ __device__ __forceinline__ void start_cell(const FusedView<T>& v, const Physics&
 		v.W0[4 * n + c] = (double)(T(0.5) * q0.r * (q0.u * q0.u + q0.v * q0.v + q0.w * q0.w) +
 		                           T(1.) / (T(ph.gamma) - T(1.0)) * q0.p);
 	}
-	T geo[MAXSL][4];
-	load_geo<T, NSL>(v.sgeo, sr, geo);
 	const T cc = tsqrt(T(ph.gamma) * q0.p / q0.r);
 	T srad = T(0.0);
 #pragma unroll
 	E3D_SLOTS(k, sr) srad += (tabs((q0.u) * geo[k][0] + (q0.v) * geo[k][1] + (q0.w) * geo[k][2]) + (cc)) * geo[k][3];
-	v.dt[c] = T(ph.cfl) * v.vol[c] / srad;
+	v.dt[c] = T(ph.cfl) * V / srad;
 }
 
 template <class T, int NSL>
 __global__ void __launch_bounds__(128) k_start(FusedView<T> v, Physics ph, int carry_w0) {
 	const int c = blockIdx.x * blockDim.x + threadIdx.x;
-	if (c < v.NR) start_cell<T, NSL>(v, ph, carry_w0, c);
+	if (c < v.NR) start_cell<T, NSL, true>(v, ph, carry_w0, c);
+	else start_after_previous();
 }
 
 // Pass 2 of a stage, one thread per real cell: convective and dissipative
@@ -1000,6 +1030,7 @@ __device__ __forceinline__ void flux_update_cell(const FusedView<T>& v, const Ph
 #endif
 template <class T, int SCHEME, bool ORDER1, int NSL, bool DISS>
 __global__ void __launch_bounds__(128, sizeof(T) == 4 ? 8 : E3D_FLUX64_MIN_BLOCKS) k_flux_update(FusedView<T> v, Physics ph, T alpha, T beta, int last, int carry_w0) {
+	start_after_previous();
 	const int c = blockIdx.x * blockDim.x + threadIdx.x;
 	if (c < v.NR) flux_update_cell<T, SCHEME, ORDER1, NSL, DISS>(v, ph, alpha, beta, last, carry_w0, c);
 }
@@ -1030,9 +1061,11 @@ __device__ __forceinline__ void flux_update_slots(const FusedView<double>& v, co
 	const bool left = mt >= 0;
 	const int m = left ? mt : ~mt;
 	const int nb = LPC == 4 ? (m < 4 * NR ? m >> 2 : m - 3 * NR) : v.slot_nbr[s];
+	const double4 geo = ldv4(v.sgeo + 4 * (size_t)s);
+	const double vol = v.vol[c];
+	start_after_previous();
 	const Q5<double> qo = ORDER1 ? ld5(v.Pin, v.NA, c) : ld5(v.FS, v.NS, s);
 	const Q5<double> qn = ORDER1 ? ld5(v.Pin, v.NA, nb) : ld5(v.FS, v.NS, m);
-	const double4 geo = ldv4(v.sgeo + 4 * (size_t)s);
 	// this lane's share of the cell: variable k, and variable 4 on lane 0
 	const int qk = k < 4 ? k : 0;
 	const double keep = 1.0 - beta;
@@ -1043,7 +1076,7 @@ __device__ __forceinline__ void flux_update_slots(const FusedView<double>& v, co
 	}
 	const double w0 = v.W0[(size_t)qk * NR + c];
 	const double w04 = k == 0 ? v.W0[4 * (size_t)NR + c] : 0.0;
-	const double coef = alpha * v.dt[c] / v.vol[c];
+	const double coef = alpha * v.dt[c] / vol;
 	{
 		Q5<double> L, R;
 		for (int q = 0; q < 5; q++) {
@@ -1122,7 +1155,8 @@ __global__ void __launch_bounds__(128, 4)
 	__shared__ double sm[4][DISS ? 10 : 5][33];
 	const int c = (blockIdx.x * 128 + threadIdx.x) / LPC;
 	const bool in_range = c < v.NR;
-	if (__any_sync(0xffffffffu, in_range))
+	if (!__any_sync(0xffffffffu, in_range)) start_after_previous();
+	else
 		flux_update_slots<SCHEME, ORDER1, LPC, DISS>(v, ph, alpha, beta, last, carry_w0, in_range ? c : v.NR - 1,
 		                                                in_range, sm[threadIdx.x >> 5]);
 }
@@ -1195,6 +1229,7 @@ __device__ __forceinline__ void wall_face_terms(double p0, double p1, double den
 template <class T>
 __global__ void __launch_bounds__(TAIL_TPB) k_tail(ReduceArgs a, const T* __restrict__ Rc, const T* __restrict__ Rd,
                                                    T* __restrict__ P, T* __restrict__ P2) {
+	start_after_previous();
 	const int t = threadIdx.x;
 	const int slot = *a.pend;
 	const int n_norm = a.nblocks * a.max_chunks, n_wb = (a.n_wall + TAIL_TPB - 1) / TAIL_TPB;
@@ -1273,6 +1308,7 @@ __global__ void __launch_bounds__(TAIL_TPB) k_tail(ReduceArgs a, const T* __rest
 // silently in the reference).  The last block clears *pend and, with `advance`,
 // moves *d_iter on.
 __global__ void __launch_bounds__(160) k_tail_sums(ReduceArgs a, int advance) {
+	start_after_previous();
 	__shared__ __align__(16) double buf[5][128];
 	const int q = threadIdx.x >> 5, lane = threadIdx.x & 31, b = blockIdx.x, i = blockIdx.y;
 	const int base = *a.d_iter;
@@ -1437,6 +1473,7 @@ __global__ void __launch_bounds__(TPB, 512 / TPB) k_persistent(FusedView<T> v0, 
 template <class T, int GRAD, int LIM, bool FIRST>
 __global__ void __launch_bounds__(128, sizeof(T) == 4 ? 8 : 4) k_recon_tiles(FusedView<T> v, Physics ph, int carry_w0,
                                                                              const int4* __restrict__ work) {
+	start_after_previous();
 	const int4 t = work[blockIdx.x];
 	const int c = t.x + threadIdx.x;
 	if (c < t.y) recon_cell<T, GRAD, LIM, FIRST, 4>(v, ph, carry_w0, c);
@@ -1445,6 +1482,7 @@ __global__ void __launch_bounds__(128, sizeof(T) == 4 ? 8 : 4) k_recon_tiles(Fus
 template <class T>
 __global__ void __launch_bounds__(128) k_start_tiles(FusedView<T> v, Physics ph, int carry_w0,
                                                      const int4* __restrict__ work) {
+	start_after_previous();
 	const int4 t = work[blockIdx.x];
 	const int c = t.x + threadIdx.x;
 	if (c < t.y) start_cell<T, 4>(v, ph, carry_w0, c);
@@ -1454,6 +1492,7 @@ template <class T, int SCHEME, bool ORDER1, bool DISS>
 __global__ void __launch_bounds__(128, sizeof(T) == 4 ? 8 : 4) k_flux_update_tiles(FusedView<T> v, Physics ph, T alpha,
                                                                                    T beta, int last, int carry_w0,
                                                                                    const int4* __restrict__ work) {
+	start_after_previous();
 	const int4 t = work[blockIdx.x];
 	const int c = t.x + threadIdx.x;
 	if (c < t.y) flux_update_cell<T, SCHEME, ORDER1, 4, DISS>(v, ph, alpha, beta, last, carry_w0, c);

@@ -7,7 +7,7 @@ namespace e3d {
 
 template <class T>
 void launch_halo(int n, const int* dst, const int* src, int NA, T* b0, T* b1, cudaStream_t st) {
-	if (n > 0) k_halo<T><<<(n + 127) / 128, 128, 0, st>>>(n, dst, src, NA, b0, b1);
+	if (n > 0) launch_next(k_halo<T>, (n + 127) / 128, 128, 0, st, n, dst, src, NA, b0, b1);
 }
 
 template <class T>
@@ -24,14 +24,14 @@ template <class T>
 void launch_tail(const ReduceArgs& a, const T* Rc, const T* Rd, T* P, T* P2, cudaStream_t st) {
 	const auto blocks = [](int n) { return (n + TAIL_TPB - 1) / TAIL_TPB; };
 	const int grid = a.nblocks * a.max_chunks + blocks(a.n_wall) + blocks(a.n_halo);
-	k_tail<T><<<grid, TAIL_TPB, 0, st>>>(a, Rc, Rd, P, P2);
+	launch_next(k_tail<T>, grid, TAIL_TPB, 0, st, a, Rc, Rd, P, P2);
 }
 
 template <class T>
 void launch_start(const FusedView<T>& v, const Physics& ph, int carry, cudaStream_t st) {
 	if (v.NR <= 0) return;
-	if (v.tet4) k_start<T, 4><<<(v.NR + 127) / 128, 128, 0, st>>>(v, ph, carry);
-	else k_start<T, 0><<<(v.NR + 127) / 128, 128, 0, st>>>(v, ph, carry);
+	if (v.tet4) launch_next(k_start<T, 4>, (v.NR + 127) / 128, 128, 0, st, v, ph, carry);
+	else launch_next(k_start<T, 0>, (v.NR + 127) / 128, 128, 0, st, v, ph, carry);
 }
 
 // Which pass reconstructs: see k_recon_var.
@@ -40,12 +40,12 @@ void recon_dispatch_first(const FusedView<T>& v, const Physics& ph, bool first, 
 	const int grid = (v.NR + 127) / 128, gv = (v.NR + RV_CELLS - 1) / RV_CELLS;
 	if (!v.tet4) {
 		if (first) launch_start<T>(v, ph, carry, st);
-		k_recon_var<T, GRAD, LIM, 0><<<gv, 5 * RV_CELLS, 0, st>>>(v, ph);
+		launch_next(k_recon_var<T, GRAD, LIM, 0>, gv, 5 * RV_CELLS, 0, st, v, ph);
 		return;
 	}
-	if (first) k_recon<T, GRAD, LIM, true, 4><<<grid, 128, 0, st>>>(v, ph, carry);
-	else if constexpr (sizeof(T) == 8) k_recon_var<T, GRAD, LIM, 4><<<gv, 5 * RV_CELLS, 0, st>>>(v, ph);
-	else k_recon<T, GRAD, LIM, false, 4><<<grid, 128, 0, st>>>(v, ph, carry);
+	if (first) launch_next(k_recon<T, GRAD, LIM, true, 4>, grid, 128, 0, st, v, ph, carry);
+	else if constexpr (sizeof(T) == 8) launch_next(k_recon_var<T, GRAD, LIM, 4>, gv, 5 * RV_CELLS, 0, st, v, ph);
+	else launch_next(k_recon<T, GRAD, LIM, false, 4>, grid, 128, 0, st, v, ph, carry);
 }
 
 template <class T>
@@ -85,12 +85,12 @@ void launch_flux_update(const FusedView<T>& v, const Physics& ph, int scheme, bo
 	do {                                                                                                   \
 		if constexpr (sizeof(T) == 8)                                                                      \
 			if (slots) {                                                                                   \
-				if (v.tet4) k_flux_slots<S, O, 4, D><<<g4, 128, 0, st>>>(v, ph, a, b, last, carry);        \
-				else k_flux_slots<S, O, 8, D><<<g8, 128, 0, st>>>(v, ph, a, b, last, carry);               \
+				if (v.tet4) launch_next(k_flux_slots<S, O, 4, D>, g4, 128, 0, st, v, ph, a, b, last, carry);        \
+				else launch_next(k_flux_slots<S, O, 8, D>, g8, 128, 0, st, v, ph, a, b, last, carry);               \
 				break;                                                                                     \
 			}                                                                                              \
-		if (v.tet4) k_flux_update<T, S, O, 4, D><<<grid, 128, 0, st>>>(v, ph, a, b, last, carry);          \
-		else k_flux_update<T, S, O, 0, D><<<grid, 128, 0, st>>>(v, ph, a, b, last, carry);                 \
+		if (v.tet4) launch_next(k_flux_update<T, S, O, 4, D>, grid, 128, 0, st, v, ph, a, b, last, carry);          \
+		else launch_next(k_flux_update<T, S, O, 0, D>, grid, 128, 0, st, v, ph, a, b, last, carry);                 \
 	} while (0)
 #define E3D_FLUX(S, O)                                                                                     \
 	do {                                                                                                   \
