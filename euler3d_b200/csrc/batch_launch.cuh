@@ -60,22 +60,17 @@ cudaError_t launch_persistent(const FusedView<T>& v0, const FusedView<T>& v1, co
 
 // ---- tiled per-pass batch iterations (enqueued on `st`, captured by the caller)
 template <class T, int GRAD, int LIM>
-void recon_tiles(const FusedView<T>& v, const Physics& ph, int carry, bool first, int n_work, const int4* work,
-                 cudaStream_t st) {
-	if (first) launch_next(k_recon_tiles<T, GRAD, LIM, true>, n_work, 128, 0, st, v, ph, carry, work);
-	else launch_next(k_recon_tiles<T, GRAD, LIM, false>, n_work, 128, 0, st, v, ph, carry, work);
+void recon_tiles(const FusedView<T>& v, const Physics& ph, int n_work, const int4* work, cudaStream_t st) {
+	launch_next(k_recon_tiles<T, GRAD, LIM>, n_work, 128, 0, st, v, ph, work);
 }
 
-template <class T, int SCHEME>
-void flux_tiles(const FusedView<T>& v, const Physics& ph, bool order1, bool diss, T al, T be, int last, int carry,
+template <class T, int SCHEME, bool ORDER1>
+void flux_tiles(const FusedView<T>& v, const Physics& ph, bool first, bool diss, T al, T be, int last, int carry,
                 int n_work, const int4* work, cudaStream_t st) {
-	if (order1) {
-		if (diss) launch_next(k_flux_update_tiles<T, SCHEME, true, true>, n_work, 128, 0, st, v, ph, al, be, last, carry, work);
-		else launch_next(k_flux_update_tiles<T, SCHEME, true, false>, n_work, 128, 0, st, v, ph, al, be, last, carry, work);
-	} else {
-		if (diss) launch_next(k_flux_update_tiles<T, SCHEME, false, true>, n_work, 128, 0, st, v, ph, al, be, last, carry, work);
-		else launch_next(k_flux_update_tiles<T, SCHEME, false, false>, n_work, 128, 0, st, v, ph, al, be, last, carry, work);
-	}
+	const auto kernel = first  ? k_flux_update_tiles<T, SCHEME, ORDER1, STAGE_FIRST>
+	                    : diss ? k_flux_update_tiles<T, SCHEME, ORDER1, STAGE_DISS>
+	                           : k_flux_update_tiles<T, SCHEME, ORDER1, STAGE_NODISS>;
+	launch_next(kernel, n_work, 128, 0, st, v, ph, al, be, last, carry, work);
 }
 
 template <class T>
@@ -88,26 +83,24 @@ cudaError_t launch_tiled_iterations(const FusedView<T>& v0, const FusedView<T>& 
 		for (int s = 0; s < a.stages; s++) {
 			const FusedView<T>& v = parity ? v1 : v0;
 			if (order2) {
-				const bool first = s == 0;
 				if (grad == GRAD_LEAST_SQUARES) {
 					if (lim == LIM_VENKATAKRISHNAN)
-						recon_tiles<T, GRAD_LEAST_SQUARES, LIM_VENKATAKRISHNAN>(v, ph, a.carry, first, a.n_work, a.work, st);
+						recon_tiles<T, GRAD_LEAST_SQUARES, LIM_VENKATAKRISHNAN>(v, ph, a.n_work, a.work, st);
 					else
-						recon_tiles<T, GRAD_LEAST_SQUARES, LIM_BARTH_JESPERSEN>(v, ph, a.carry, first, a.n_work, a.work, st);
+						recon_tiles<T, GRAD_LEAST_SQUARES, LIM_BARTH_JESPERSEN>(v, ph, a.n_work, a.work, st);
 				} else {
 					if (lim == LIM_VENKATAKRISHNAN)
-						recon_tiles<T, GRAD_GREEN_GAUSS, LIM_VENKATAKRISHNAN>(v, ph, a.carry, first, a.n_work, a.work, st);
+						recon_tiles<T, GRAD_GREEN_GAUSS, LIM_VENKATAKRISHNAN>(v, ph, a.n_work, a.work, st);
 					else
-						recon_tiles<T, GRAD_GREEN_GAUSS, LIM_BARTH_JESPERSEN>(v, ph, a.carry, first, a.n_work, a.work, st);
+						recon_tiles<T, GRAD_GREEN_GAUSS, LIM_BARTH_JESPERSEN>(v, ph, a.n_work, a.work, st);
 				}
-			} else if (s == 0) {
-				launch_next(k_start_tiles<T>, a.n_work, 128, 0, st, v, ph, a.carry, a.work);
 			}
 			const T al = T(a.alpha[s]), be = T(a.beta[s]);
 			const int last = s == a.stages - 1;
 			const bool diss = a.beta[s] != 0.0;
-			if (scheme == FLUX_AUSM) flux_tiles<T, FLUX_AUSM>(v, ph, !order2, diss, al, be, last, a.carry, a.n_work, a.work, st);
-			else flux_tiles<T, FLUX_ROE>(v, ph, !order2, diss, al, be, last, a.carry, a.n_work, a.work, st);
+			const auto flux = scheme == FLUX_AUSM ? (order2 ? flux_tiles<T, FLUX_AUSM, false> : flux_tiles<T, FLUX_AUSM, true>)
+			                                      : (order2 ? flux_tiles<T, FLUX_ROE, false> : flux_tiles<T, FLUX_ROE, true>);
+			flux(v, ph, s == 0, diss, al, be, last, a.carry, a.n_work, a.work, st);
 			parity ^= 1;
 		}
 		end_iteration<T>(parity ? v1 : v0, r, it, a.iters, st);

@@ -255,36 +255,19 @@ __device__ __forceinline__ Q5<double> freestream64(const FusedView<float>& v, co
 
 // ------------------------------------------------------------ stage kernels (tiles of real cells)
 
-// stage 0: local time step from the full state (W is carried, no W0 pass)
-__global__ void __launch_bounds__(128) k_delta_start_tiles(FusedView<float> v, Physics ph,
-                                                           const int4* __restrict__ work) {
-	const int4 t = work[blockIdx.x];
-	const int c = t.x + threadIdx.x;
-	if (c >= t.y) return;
-	const Q5<float> b = ld5(v.Pb, v.NA, c), d = ld5(v.Pin, v.NA, c);
-	const Q5<float> q{b.r + d.r, b.u + d.u, b.v + d.v, b.w + d.w, b.p + d.p};
-	const float4* geo = reinterpret_cast<const float4*>(v.sgeo) + 4 * (size_t)c;
-	const float cc = sqrtf(float(ph.gamma) * q.p / q.r);
-	float srad = 0.f;
-#pragma unroll
-	for (int k = 0; k < 4; k++) {
-		const float4 n = geo[k];
-		srad += (fabsf(q.u * n.x + q.v * n.y + q.w * n.z) + cc) * n.w;
-	}
-	v.dt[c] = float(ph.cfl) * v.vol[c] / srad;
-}
-
 // one RK stage: flux differences, residual, conserved-difference update,
-// primitive differences and the boundary ghosts' differences
+// primitive differences and the boundary ghosts' differences; the first stage
+// forms the local time step from the full state as well
 #ifndef E3D_DELTA_MIN_BLOCKS
 #define E3D_DELTA_MIN_BLOCKS 6
 #endif
-template <bool DISS>
+template <int MODE>
 __global__ void __launch_bounds__(128, E3D_DELTA_MIN_BLOCKS) k_delta_flux_tiles(FusedView<float> v, Physics ph, float alpha, float beta,
                                                              int last, const int4* __restrict__ work) {
 	const int4 t = work[blockIdx.x];
 	const int c = t.x + threadIdx.x;
 	if (c >= t.y) return;
+	constexpr bool DISS = MODE != STAGE_NODISS, FIRST = MODE == STAGE_FIRST;
 	const float g = float(ph.gamma), gr = float(ph.gr), gm1 = float(ph.gm1);
 	const int NR = v.NR;
 	const float keep = 1.f - beta;
@@ -296,6 +279,12 @@ __global__ void __launch_bounds__(128, E3D_DELTA_MIN_BLOCKS) k_delta_flux_tiles(
 		if (DISS) ad[q] *= keep;
 	}
 	const DCell own = load_cell(v.rec_base, v.rec_in, c);
+	Q5<float> q{0.f, 0.f, 0.f, 0.f, 0.f};
+	float cc = 0.f, srad = 0.f;
+	if (FIRST) {
+		q = Q5<float>{own.b.r + v.dW[c], own.b.u + own.d.du, own.b.v + own.d.dv, own.b.w + own.d.dw, own.b.p + own.d.dp};
+		cc = sqrtf(g * q.p / q.r);
+	}
 	const float4* geo = reinterpret_cast<const float4*>(v.sgeo) + 4 * (size_t)c;
 	unsigned ghosts = 0;  // slots with a ghost neighbour
 #pragma unroll
@@ -306,6 +295,7 @@ __global__ void __launch_bounds__(128, E3D_DELTA_MIN_BLOCKS) k_delta_flux_tiles(
 		if (nb >= NR) ghosts |= 1u << k;
 		const DCell nbr = load_cell(v.rec_base, v.rec_in, nb);
 		const float4 n = geo[k];
+		if (FIRST) srad += (fabsf(q.u * n.x + q.v * n.y + q.w * n.z) + cc) * n.w;
 		float fc[5], fd[5];
 		// one call with the sides selected by value: a branch on the orientation
 		// would run the face arithmetic twice in warps whose cells differ
@@ -316,7 +306,15 @@ __global__ void __launch_bounds__(128, E3D_DELTA_MIN_BLOCKS) k_delta_flux_tiles(
 			if (DISS) ad[q] += (left ? fd[q] : -fd[q]) * beta;
 		}
 	}
-	const float coef = alpha * v.dt[c] / v.vol[c];
+	const float V = v.vol[c];
+	float dt;
+	if (FIRST) {
+		dt = float(ph.cfl) * V / srad;
+		v.dt[c] = dt;
+	} else {
+		dt = v.dt[c];
+	}
+	const float coef = alpha * dt / V;
 	float dw[5];
 #pragma unroll
 	for (int q = 0; q < 5; q++) {
@@ -328,7 +326,7 @@ __global__ void __launch_bounds__(128, E3D_DELTA_MIN_BLOCKS) k_delta_flux_tiles(
 	}
 	const Q5<float> dq = prim_delta(own.b, dw, gm1);
 	store_diff(v.rec_out, c, diff_record(own.b, dq, g, gr));
-	if (last) st5(v.Pout, v.NA, c, dq);  // the time step, wall pressures and norms read it once an iteration
+	if (last) st5(v.Pout, v.NA, c, dq);  // wall pressures read it once an iteration
 	// boundary ghosts in FP64: full state of the cell, FP64 face normal
 	while (ghosts) {
 		const int k = __ffs(ghosts) - 1;
@@ -471,11 +469,12 @@ cudaError_t launch_iterations(const FusedView<float>& v0, const FusedView<float>
 	for (int it = 0; it < a.iters; it++) {
 		for (int s = 0; s < a.stages; s++) {
 			const FusedView<float>& v = parity ? v1 : v0;
-			if (s == 0) k_delta_start_tiles<<<a.n_work, 128, 0, st>>>(v, ph, a.work);
 			const float al = float(a.alpha[s]), be = float(a.beta[s]);
 			const int last = s == a.stages - 1;
-			if (a.beta[s] != 0.0) k_delta_flux_tiles<true><<<a.n_work, 128, 0, st>>>(v, ph, al, be, last, a.work);
-			else k_delta_flux_tiles<false><<<a.n_work, 128, 0, st>>>(v, ph, al, be, last, a.work);
+			const auto kernel = s == 0               ? k_delta_flux_tiles<STAGE_FIRST>
+			                    : a.beta[s] != 0.0 ? k_delta_flux_tiles<STAGE_DISS>
+			                                       : k_delta_flux_tiles<STAGE_NODISS>;
+			kernel<<<a.n_work, 128, 0, st>>>(v, ph, al, be, last, a.work);
 			parity ^= 1;
 		}
 		end_iteration<float>(parity ? v1 : v0, r, it, a.iters, st);

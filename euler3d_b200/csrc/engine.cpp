@@ -767,16 +767,13 @@ void Engine::iteration_body(Fused<T>& f, int parity, std::vector<cudaEvent_t>* m
 		v.case_free = ncases_ > 1 ? case_free_d_.p : nullptr;  // single case: Physics::free
 		v.gcase = gcase_d_.p;
 		if (order_ == 2) {
-			launch_recon<T>(v, ph_, grad_kind_, lim_kind_, s == 0, carry_, st_);
-			mark();
-		} else if (s == 0) {
-			launch_start<T>(v, ph_, carry_, st_);
+			launch_recon<T>(v, ph_, grad_kind_, lim_kind_, st_);
 			mark();
 		}
 		// the reference always evaluates the dissipative flux: its guard
 		// `beta > (10^-16)` is an XOR (== -6) and is always true
 		// (ResidualCalculator.cpp:33)
-		launch_flux_update<T>(v, ph_, scheme_, order_ == 1, alpha_[s], beta_[s], s == stages - 1, carry_, st_);
+		launch_flux_update<T>(v, ph_, scheme_, order_ == 1, s == 0, alpha_[s], beta_[s], s == stages - 1, carry_, st_);
 		mark();
 		p ^= 1;
 	}
@@ -793,7 +790,7 @@ int Engine::launches_per_iteration() const {
 	const int stages = (int)alpha_.size();
 	if (deck_.smoothing)  // W0, spectral radius, time step; per stage (grad, lim,) conv, diss, 2 smoothing, update, BC; tail
 		return 3 + stages * ((order_ == 2 ? 2 : 0) + 6) + 1;
-	return (order_ == 2 ? 2 * stages + (tet4_ ? 0 : 1) : stages + 1) + 1 /*tail; its sums once per TAIL_SLOTS iterations*/;
+	return (order_ == 2 ? 2 * stages : stages) + 1 /*tail; its sums once per TAIL_SLOTS iterations*/;
 }
 
 // Launches one outer iteration (its captured graph, or eagerly); the tail's
@@ -1279,37 +1276,30 @@ void Engine::set(const std::string& name, int b, const std::vector<double>& in_l
 }
 
 // ---------------------------------------------------------------- measurement
-double Engine::bytes_recon(bool first) const {
+double Engine::bytes_recon() const {
 	const double b = opt_.precision == PREC_FP64 ? 8.0 : 4.0;
 	const double NSR = tet4_ ? 4.0 * NR_ : (double)NS_ - NG_;
-	double x = 5 * b * NA_                                  // cell states, every cell read once
-	           + 4.0 * NSR + 4.0 * NG_                      // neighbour ids (+ ghost mates)
-	           + 3 * b * NSR                                // LS weights or signed area vectors
-	           + 3 * b * NS_                                // r-vectors, ghost slots included
-	           + b * NA_                                    // volumes
-	           + 4 * b * NG_ + 2.0 * NG_                    // ghost face normals, ghost flags
-	           + 5 * b * NS_;                               // face states written
-	if (first) x += 5 * 8.0 * (carry_ ? 0 : NR_) + b * NR_ + 4 * b * NSR;  // W0, dt written; face normals
-	return x;
+	return 5 * b * NA_              // cell states, every cell read once
+	       + 4.0 * NSR + 4.0 * NG_  // neighbour ids (+ ghost mates)
+	       + 3 * b * NSR            // LS weights or signed area vectors
+	       + 3 * b * NS_            // r-vectors, ghost slots included
+	       + b * NA_                // volumes
+	       + 4 * b * NG_ + 2.0 * NG_  // ghost face normals, ghost flags
+	       + 5 * b * NS_;           // face states written
 }
-double Engine::bytes_start() const {
+double Engine::bytes_flux(bool order1, bool first, bool diss, bool last) const {
 	const double b = opt_.precision == PREC_FP64 ? 8.0 : 4.0;
 	const double NSR = tet4_ ? 4.0 * NR_ : (double)NS_ - NG_;
-	return 5 * b * NR_ + 4 * b * NSR + b * NR_ + 5 * 8.0 * (carry_ ? 0 : NR_) + b * NR_;
-}
-double Engine::bytes_flux(bool order1, bool diss, bool last) const {
-	const double b = opt_.precision == PREC_FP64 ? 8.0 : 4.0;
-	const double NSR = tet4_ ? 4.0 * NR_ : (double)NS_ - NG_;
-	double x = 4.0 * NSR + 4.0 * NSR       // mate and neighbour ids
-	           + 4 * b * NSR               // face normal and area
-	           + 5 * b * NR_               // Rd read
-	           + 5 * 8.0 * NR_             // W0 read
-	           + 2 * b * NR_               // dt, volume
-	           + 5 * b * NA_               // new cell and ghost states written
-	           + 1.0 * NG_;                // ghost kinds
-	x += order1 ? 5 * b * NA_ : 5 * b * NS_;  // cell states or face states read
-	if (diss) x += 5 * b * NR_;               // Rd written
-	if (last) x += 5 * b * NR_ + (carry_ ? 5 * 8.0 * NR_ : 0.0);  // Rc (and carried W) written
+	double x = 4.0 * NSR + (tet4_ ? 0.0 : 4.0 * NSR)  // mate ids (and neighbour ids: on tetrahedra they follow)
+	           + 4 * b * NSR                          // face normal and area
+	           + (first ? 0.0 : 5 * b * NR_)          // Rd read
+	           + 5 * 8.0 * NR_                        // W0 read (first: written, or read when carried)
+	           + 2 * b * NR_                          // dt (first: written), volume
+	           + 5 * b * NA_                          // new cell and ghost states written
+	           + 1.0 * NG_;                           // ghost kinds
+	x += order1 ? 5 * b * NA_ : 5 * b * NS_ + (first ? 5 * b * NR_ : 0.0);  // cell states or face states read
+	if (diss) x += 5 * b * NR_;                                             // Rd written
+	if (last) x += 5 * b * NR_ + (carry_ ? 5 * 8.0 * NR_ : 0.0);            // Rc (and carried W) written
 	return x;
 }
 
@@ -1323,15 +1313,12 @@ std::vector<Engine::KernelTime> Engine::time_kernels(int n) {
 	std::vector<double> bytes;
 	for (int s = 0; s < stages; s++) {
 		if (order_ == 2) {
-			names.push_back(s == 0 ? "recon_first" : "recon");
-			bytes.push_back(bytes_recon(s == 0));
-		} else if (s == 0) {
-			names.push_back("start");
-			bytes.push_back(bytes_start());
+			names.push_back("recon");
+			bytes.push_back(bytes_recon());
 		}
-		const bool diss = beta_[s] != 0.0, last = s == stages - 1;
-		names.push_back(last ? "flux_update_last" : diss ? "flux_update" : "flux_update_nodiss");
-		bytes.push_back(bytes_flux(order_ == 1, diss, last));
+		const bool first = s == 0, diss = beta_[s] != 0.0, last = s == stages - 1;
+		names.push_back(last ? "flux_update_last" : first ? "flux_update_first" : diss ? "flux_update" : "flux_update_nodiss");
+		bytes.push_back(bytes_flux(order_ == 1, first, diss, last));
 	}
 	names.push_back("reduce_halo");
 	bytes.push_back(0.0);

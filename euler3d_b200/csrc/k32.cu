@@ -8,9 +8,8 @@ template void launch_halo<float>(int, const int*, const int*, int, float*, float
 template void launch_halo_pack<float>(int, const int*, int, const float*, float*, cudaStream_t);
 template void launch_halo_unpack<float>(int, const int*, int, const float*, float*, float*, cudaStream_t);
 template void launch_tail<float>(const ReduceArgs&, const float*, const float*, float*, float*, cudaStream_t);
-template void launch_recon<float>(const FusedView<float>&, const Physics&, int, int, bool, int, cudaStream_t);
-template void launch_start<float>(const FusedView<float>&, const Physics&, int, cudaStream_t);
-template void launch_flux_update<float>(const FusedView<float>&, const Physics&, int, bool, double, double, int, int,
+template void launch_recon<float>(const FusedView<float>&, const Physics&, int, int, cudaStream_t);
+template void launch_flux_update<float>(const FusedView<float>&, const Physics&, int, bool, bool, double, double, int, int,
                                         cudaStream_t);
 
 

@@ -81,10 +81,9 @@ template void launch_halo<double>(int, const int*, const int*, int, double*, dou
 template void launch_halo_pack<double>(int, const int*, int, const double*, double*, cudaStream_t);
 template void launch_halo_unpack<double>(int, const int*, int, const double*, double*, double*, cudaStream_t);
 template void launch_tail<double>(const ReduceArgs&, const double*, const double*, double*, double*, cudaStream_t);
-template void launch_recon<double>(const FusedView<double>&, const Physics&, int, int, bool, int, cudaStream_t);
-template void launch_start<double>(const FusedView<double>&, const Physics&, int, cudaStream_t);
-template void launch_flux_update<double>(const FusedView<double>&, const Physics&, int, bool, double, double, int, int,
-                                         cudaStream_t);
+template void launch_recon<double>(const FusedView<double>&, const Physics&, int, int, cudaStream_t);
+template void launch_flux_update<double>(const FusedView<double>&, const Physics&, int, bool, bool, double, double, int, int,
+                                        cudaStream_t);
 template int batch::persistent_blocks_per_sm<double>(int, int, int, bool);
 template cudaError_t batch::launch_persistent<double>(const FusedView<double>&, const FusedView<double>&, const Physics&,
                                                const PersistArgs&, int, int, int, bool, int, cudaStream_t);

@@ -594,34 +594,9 @@ __device__ __forceinline__ void ausm_face_sides(const AusmSide<T>& L, const Ausm
 }
 
 // Pass 1 of a stage, one thread per real cell: gradient, limiter and MUSCL
-// face states of the cell and of its ghost cells.  FIRST additionally computes
-// W0 (unless carried) and the local time step from the stage-0 state.
-// first stage only: W0 (unless carried) and the local time step (Timestep.cpp:26-148)
-template <class T, int NSL>
-__device__ __forceinline__ void first_stage_extras(const FusedView<T>& v, const Physics& ph, int carry_w0, int c) {
-	const SlotRange<T, NSL> sr(v, c);
-	const Q5<T> q0 = ld5(v.Pin, v.NA, c);
-	const T V = v.vol[c];
-	if (!carry_w0) {
-		const int n = v.NR;
-		v.W0[c] = (double)q0.r;
-		v.W0[n + c] = (double)(q0.r * q0.u);
-		v.W0[2 * n + c] = (double)(q0.r * q0.v);
-		v.W0[3 * n + c] = (double)(q0.r * q0.w);
-		v.W0[4 * n + c] = (double)(T(0.5) * q0.r * (q0.u * q0.u + q0.v * q0.v + q0.w * q0.w) +
-		                           T(1.) / (T(ph.gamma) - T(1.0)) * q0.p);
-	}
-	T geo[MAXSL][4];
-	load_geo<T, NSL>(v.sgeo, sr, geo);
-	const T cc = tsqrt(T(ph.gamma) * q0.p / q0.r);
-	T srad = T(0.0);
-#pragma unroll
-	E3D_SLOTS(k, sr) srad += (tabs((q0.u) * geo[k][0] + (q0.v) * geo[k][1] + (q0.w) * geo[k][2]) + (cc)) * geo[k][3];
-	v.dt[c] = T(ph.cfl) * V / srad;
-}
-
-template <class T, int GRAD, int LIM, bool FIRST, int NSL>
-__device__ __forceinline__ void recon_cell(const FusedView<T>& v, const Physics& ph, int carry_w0, int c) {
+// face states of the cell and of its ghost cells.
+template <class T, int GRAD, int LIM, int NSL>
+__device__ __forceinline__ void recon_cell(const FusedView<T>& v, const Physics& ph, int c) {
 	const SlotRange<T, NSL> sr(v, c);
 	const Q5<T> q0 = ld5(v.Pin, v.NA, c);
 	int nb[MAXSL];
@@ -704,11 +679,10 @@ __device__ __forceinline__ void recon_cell(const FusedView<T>& v, const Physics&
 		}
 	}
 	// ghost cells of this cell's boundary faces: gradient (reflected or zero),
-	// limiter (the ghost's only neighbour is c) and face state.  Later stages read
-	// the slot neighbours again (a cache hit) rather than hold them through the
-	// pass, which takes the FP32 pass from 32-68 bytes of spills to none; the
-	// first stage spills less keeping them.
-	if (!FIRST) load_int<T, NSL>(v.slot_nbr, sr, nb);
+	// limiter (the ghost's only neighbour is c) and face state.  The slot neighbours
+	// are read again (a cache hit) rather than held through the pass, which takes
+	// the FP32 pass from 32-68 bytes of spills to none.
+	load_int<T, NSL>(v.slot_nbr, sr, nb);
 #pragma unroll
 	E3D_SLOTS(k, sr) {
 		if (nb[k] >= v.NR) {
@@ -742,7 +716,6 @@ __device__ __forceinline__ void recon_cell(const FusedView<T>& v, const Physics&
 			st5(v.FS, v.NS, ms, fs);
 		}
 	}
-	if (FIRST) first_stage_extras<T, NSL>(v, ph, carry_w0, c);
 }
 
 // resident blocks per SM the FP32 reconstruction pass is compiled for (8: 64
@@ -753,28 +726,25 @@ __device__ __forceinline__ void recon_cell(const FusedView<T>& v, const Physics&
 #ifndef E3D_FP64_MIN_BLOCKS
 #define E3D_FP64_MIN_BLOCKS 4
 #endif
-template <class T, int GRAD, int LIM, bool FIRST, int NSL>
-__global__ void __launch_bounds__(128, sizeof(T) == 4 ? E3D_RECON_MIN_BLOCKS : E3D_FP64_MIN_BLOCKS) k_recon(FusedView<T> v, Physics ph, int carry_w0) {
+template <class T, int GRAD, int LIM, int NSL>
+__global__ void __launch_bounds__(128, sizeof(T) == 4 ? E3D_RECON_MIN_BLOCKS : E3D_FP64_MIN_BLOCKS) k_recon(FusedView<T> v, Physics ph) {
 	start_after_previous();
 	const int c = blockIdx.x * blockDim.x + threadIdx.x;
-	if (c < v.NR) recon_cell<T, GRAD, LIM, FIRST, NSL>(v, ph, carry_w0, c);
+	if (c < v.NR) recon_cell<T, GRAD, LIM, NSL>(v, ph, c);
 }
 
-// Reconstruction with one lane per (cell, variable): FP64 later stages on
-// tetrahedra, every stage and both precisions on other cells.  Gradient, limiter
-// and face states of one variable depend on that variable alone, so five lanes
-// per cell run the same per-variable arithmetic as recon_cell, in the same order
-// (FP64: bit for bit), with a fifth of its gradient/limiter state and the slot
-// weights read per slot: 48 registers instead of 128, 40 resident warps per SM
-// instead of 16 (663k tets FP64: 118 us at 6 blocks of 64 registers, 115 at 8).  A block covers RV_CELLS cells (5 * RV_CELLS threads,
-// cell-major: the four lanes of a cell's (rho, u, v, w) read and write one
-// 32-byte vector together).  Measured on B200 (3.07M tets, FP64 second order):
-// 2.61 TB/s against 2.44 for the one-thread-per-cell pass.  On tetrahedra the
-// first stage keeps recon_cell: its time step and W0 need the whole cell, and
-// one lane of five doing them made that pass slower (2.82 against 2.89 TB/s).
-// With slot counts known only at run time, one thread per cell kept its slot
-// arrays in local memory: 65k hexahedra FP64 40 us a launch, 25 here (the
-// first stage with W0 and the time step in k_start).
+// Reconstruction with one lane per (cell, variable): FP64, and both precisions on
+// cells other than tetrahedra.  Gradient, limiter and face states of one variable
+// depend on that variable alone, so five lanes per cell run the same per-variable
+// arithmetic as recon_cell, in the same order (FP64: bit for bit), with a fifth of
+// its gradient/limiter state and the slot weights read per slot: 48 registers
+// instead of 128, 40 resident warps per SM instead of 16 (663k tets FP64: 118 us
+// at 6 blocks of 64 registers, 115 at 8).  A block covers RV_CELLS cells (5 *
+// RV_CELLS threads, cell-major: the four lanes of a cell's (rho, u, v, w) read and
+// write one 32-byte vector together).  Measured on B200 (3.07M tets, FP64 second
+// order): 2.61 TB/s against 2.44 for the one-thread-per-cell pass.  With slot
+// counts known only at run time, one thread per cell kept its slot arrays in local
+// memory: 65k hexahedra FP64 40 us a launch, 25 here.
 constexpr int RV_CELLS = 32;
 #ifndef E3D_RV_MIN_BLOCKS
 #define E3D_RV_MIN_BLOCKS 8
@@ -875,39 +845,6 @@ __global__ void __launch_bounds__(5 * RV_CELLS, E3D_RV_MIN_BLOCKS) k_recon_var(F
 	}
 }
 
-// W0 and the local time step without a reconstruction pass (first order).
-// WAIT: behind the previous kernel, with the geometry already on its way.
-template <class T, int NSL, bool WAIT = false>
-__device__ __forceinline__ void start_cell(const FusedView<T>& v, const Physics& ph, int carry_w0, int c) {
-	const SlotRange<T, NSL> sr(v, c);
-	T geo[MAXSL][4];
-	load_geo<T, NSL>(v.sgeo, sr, geo);
-	const T V = v.vol[c];
-	if (WAIT) start_after_previous();
-	const Q5<T> q0 = ld5(v.Pin, v.NA, c);
-	if (!carry_w0) {
-		const int n = v.NR;
-		v.W0[c] = (double)q0.r;
-		v.W0[n + c] = (double)(q0.r * q0.u);
-		v.W0[2 * n + c] = (double)(q0.r * q0.v);
-		v.W0[3 * n + c] = (double)(q0.r * q0.w);
-		v.W0[4 * n + c] = (double)(T(0.5) * q0.r * (q0.u * q0.u + q0.v * q0.v + q0.w * q0.w) +
-		                           T(1.) / (T(ph.gamma) - T(1.0)) * q0.p);
-	}
-	const T cc = tsqrt(T(ph.gamma) * q0.p / q0.r);
-	T srad = T(0.0);
-#pragma unroll
-	E3D_SLOTS(k, sr) srad += (tabs((q0.u) * geo[k][0] + (q0.v) * geo[k][1] + (q0.w) * geo[k][2]) + (cc)) * geo[k][3];
-	v.dt[c] = T(ph.cfl) * V / srad;
-}
-
-template <class T, int NSL>
-__global__ void __launch_bounds__(128) k_start(FusedView<T> v, Physics ph, int carry_w0) {
-	const int c = blockIdx.x * blockDim.x + threadIdx.x;
-	if (c < v.NR) start_cell<T, NSL, true>(v, ph, carry_w0, c);
-	else start_after_previous();
-}
-
 // Pass 2 of a stage, one thread per real cell: convective and dissipative
 // fluxes of each face (computed identically from both sides), residual gather,
 // conservative update into Pout and the ghost states of the cell's boundary
@@ -927,10 +864,23 @@ __global__ void __launch_bounds__(128) k_start(FusedView<T> v, Physics ph, int c
 // slot_nbr is not read, and beta = 1 drops Rd unread.  B200, us a launch with /
 // without dissipation: 663k tets FP64 Roe 136 / 100 -> 121 / 88; 3.07M FP32
 // Roe 184 / 147 -> 175 / 144 (FP32 keeps the loop unrolled: 178 / 156 rolled).
-template <class T, int SCHEME, bool ORDER1, int NSL, bool DISS>
+// FIRST (the first stage): W0 (unless carried) and the local time step
+// (Timestep.cpp:26-148) are formed here from the state the stage starts from,
+// with the normals the fluxes read anyway, instead of in a pass of their own or
+// in the first reconstruction (663k tets FP64 second order, us an iteration:
+// first reconstruction 145 -> 115, this pass 117 -> 129; 3.07M FP32 185 -> 160 and
+// 180 -> 192).
+enum StageMode : int { STAGE_NODISS, STAGE_DISS, STAGE_FIRST };
+template <class T>
+__device__ __forceinline__ T conserved(const Q5<T>& q, int k, double gamma) {
+	if (k == 4) return T(0.5) * q.r * (q.u * q.u + q.v * q.v + q.w * q.w) + T(1.) / (T(gamma) - T(1.0)) * q.p;
+	return k == 0 ? q.r : k == 1 ? q.r * q.u : k == 2 ? q.r * q.v : q.r * q.w;
+}
+template <class T, int SCHEME, bool ORDER1, int NSL, int MODE>
 __device__ __forceinline__ void flux_update_cell(const FusedView<T>& v, const Physics& ph, T alpha, T beta, int last,
                                                  int carry_w0, int c) {
 	constexpr int UNROLL = NSL == 4 && sizeof(T) == 4 ? 4 : 1;
+	constexpr bool DISS = MODE != STAGE_NODISS, FIRST = MODE == STAGE_FIRST;
 	const int NR = v.NR;
 	const SlotRange<T, NSL> sr(v, c);
 	const T g = T(ph.gamma), gr = T(ph.gr), gm1 = T(ph.gm1);
@@ -942,7 +892,9 @@ __device__ __forceinline__ void flux_update_cell(const FusedView<T>& v, const Ph
 		if (DISS) ad[q] *= keep;
 	}
 	Q5<T> qc;
-	if (ORDER1) qc = ld5(v.Pin, v.NA, c);
+	if (ORDER1 || FIRST) qc = ld5(v.Pin, v.NA, c);
+	const T cc = FIRST ? tsqrt(g * qc.p / qc.r) : T(0.0);
+	T srad = T(0.0);
 #ifdef E3D_SHARED_SIDES
 	constexpr bool shared_sides = ORDER1 && SCHEME == FLUX_AUSM;
 	AusmSide<T> own;
@@ -966,6 +918,7 @@ __device__ __forceinline__ void flux_update_cell(const FusedView<T>& v, const Ph
 			qn = ld5(v.FS, v.NS, m);
 		}
 		const typename Vec4<T>::type geo = ldv4(v.sgeo + 4 * (size_t)s);
+		if (FIRST) srad += (tabs((qc.u) * geo.x + (qc.v) * geo.y + (qc.w) * geo.z) + (cc)) * geo.w;
 		Q5<T> L, R;
 		for (int q = 0; q < 5; q++) {
 			qv(L, q) = left ? qv(qo, q) : qv(qn, q);
@@ -996,9 +949,22 @@ __device__ __forceinline__ void flux_update_cell(const FusedView<T>& v, const Ph
 	for (int q = 0; q < 5; q++) {
 		if (last) v.Rc[q * (size_t)NR + c] = ac[q];
 		if (DISS) v.Rd[q * (size_t)NR + c] = ad[q];
-		w0[q] = v.W0[q * (size_t)NR + c];
+		if (FIRST && !carry_w0) {
+			w0[q] = (double)conserved(qc, q, ph.gamma);
+			v.W0[q * (size_t)NR + c] = w0[q];
+		} else {
+			w0[q] = v.W0[q * (size_t)NR + c];
+		}
 	}
-	const T coef = alpha * v.dt[c] / v.vol[c];
+	const T V = v.vol[c];
+	T dt;
+	if (FIRST) {
+		dt = T(ph.cfl) * V / srad;
+		v.dt[c] = dt;
+	} else {
+		dt = v.dt[c];
+	}
+	const T coef = alpha * dt / V;
 	const Q5<T> qnew = conservative_update<T>(w0, coef, ac, ad, gm1, wn);
 	st5(v.Pout, v.NA, c, qnew);
 	if (last && carry_w0)
@@ -1028,11 +994,11 @@ __device__ __forceinline__ void flux_update_cell(const FusedView<T>& v, const Ph
 #ifndef E3D_FLUX64_MIN_BLOCKS
 #define E3D_FLUX64_MIN_BLOCKS 5
 #endif
-template <class T, int SCHEME, bool ORDER1, int NSL, bool DISS>
+template <class T, int SCHEME, bool ORDER1, int NSL, int MODE>
 __global__ void __launch_bounds__(128, sizeof(T) == 4 ? 8 : E3D_FLUX64_MIN_BLOCKS) k_flux_update(FusedView<T> v, Physics ph, T alpha, T beta, int last, int carry_w0) {
 	start_after_previous();
 	const int c = blockIdx.x * blockDim.x + threadIdx.x;
-	if (c < v.NR) flux_update_cell<T, SCHEME, ORDER1, NSL, DISS>(v, ph, alpha, beta, last, carry_w0, c);
+	if (c < v.NR) flux_update_cell<T, SCHEME, ORDER1, NSL, MODE>(v, ph, alpha, beta, last, carry_w0, c);
 }
 
 // FP64 pass 2 with one lane per slot, LPC lanes per cell (4: tetrahedra; 8: up to
@@ -1043,10 +1009,11 @@ __global__ void __launch_bounds__(128, sizeof(T) == 4 ? 8 : E3D_FLUX64_MIN_BLOCK
 // memory and lane k adds up variable k over the slots in ascending face id
 // (the reference's order, so FP64 results are the same bits) and updates it;
 // lane 0 has the energy too.
-template <int SCHEME, bool ORDER1, int LPC, bool DISS>
+template <int SCHEME, bool ORDER1, int LPC, int MODE>
 __device__ __forceinline__ void flux_update_slots(const FusedView<double>& v, const Physics& ph, double alpha, double beta, int last,
                                                   int carry_w0, int c, bool in_range, double (*sm)[33]) {
 	constexpr unsigned FULL = 0xffffffffu;
+	constexpr bool DISS = MODE != STAGE_NODISS, FIRST = MODE == STAGE_FIRST;
 	const int lane = threadIdx.x & 31, k = lane & (LPC - 1), first = lane - k;
 	const int NR = v.NR;
 	const double g = ph.gamma, gr = ph.gr, gm1 = ph.gm1;
@@ -1074,9 +1041,34 @@ __device__ __forceinline__ void flux_update_slots(const FusedView<double>& v, co
 		rd = v.Rd[(size_t)qk * NR + c];
 		if (k == 0) rd4 = v.Rd[4 * (size_t)NR + c];
 	}
-	const double w0 = v.W0[(size_t)qk * NR + c];
-	const double w04 = k == 0 ? v.W0[4 * (size_t)NR + c] : 0.0;
-	const double coef = alpha * v.dt[c] / vol;
+	Q5<double> qc;
+	if (FIRST) qc = ORDER1 ? qo : ld5(v.Pin, v.NA, c);
+	double w0, w04 = 0.0;
+	if (FIRST && !carry_w0) {
+		w0 = conserved(qc, qk, ph.gamma);
+		w04 = conserved(qc, 4, ph.gamma);
+		if (in_range && k < 4) v.W0[(size_t)k * NR + c] = w0;
+		if (in_range && k == 0) v.W0[4 * (size_t)NR + c] = w04;
+	} else {
+		w0 = v.W0[(size_t)qk * NR + c];
+		if (k == 0) w04 = v.W0[4 * (size_t)NR + c];
+	}
+	double dt;
+	if (FIRST) {  // ahead of the fluxes, whose arithmetic covers its divisions
+		sm[10][lane] = (fabs((qc.u) * geo.x + (qc.v) * geo.y + (qc.w) * geo.z) + (sqrt(g * qc.p / qc.r))) * geo.w;
+		__syncwarp();
+		double srad = 0.0;
+#pragma unroll
+		for (int i = 0; i < (LPC == 4 ? 4 : MAXSL); i++) {
+			if (LPC != 4 && i >= n) break;
+			srad += sm[10][first + i];
+		}
+		dt = ph.cfl * vol / srad;
+		if (in_range && k == 0) v.dt[c] = dt;
+	} else {
+		dt = v.dt[c];
+	}
+	const double coef = alpha * dt / vol;
 	{
 		Q5<double> L, R;
 		for (int q = 0; q < 5; q++) {
@@ -1149,15 +1141,15 @@ __device__ __forceinline__ void flux_update_slots(const FusedView<double>& v, co
 	}
 }
 
-template <int SCHEME, bool ORDER1, int LPC, bool DISS>
+template <int SCHEME, bool ORDER1, int LPC, int MODE>
 __global__ void __launch_bounds__(128, 4)
     k_flux_slots(FusedView<double> v, Physics ph, double alpha, double beta, int last, int carry_w0) {
-	__shared__ double sm[4][DISS ? 10 : 5][33];
+	__shared__ double sm[4][MODE == STAGE_FIRST ? 11 : MODE == STAGE_DISS ? 10 : 5][33];
 	const int c = (blockIdx.x * 128 + threadIdx.x) / LPC;
 	const bool in_range = c < v.NR;
 	if (!__any_sync(0xffffffffu, in_range)) start_after_previous();
 	else
-		flux_update_slots<SCHEME, ORDER1, LPC, DISS>(v, ph, alpha, beta, last, carry_w0, in_range ? c : v.NR - 1,
+		flux_update_slots<SCHEME, ORDER1, LPC, MODE>(v, ph, alpha, beta, last, carry_w0, in_range ? c : v.NR - 1,
 		                                                in_range, sm[threadIdx.x >> 5]);
 }
 
@@ -1428,17 +1420,10 @@ __global__ void __launch_bounds__(TPB, 512 / TPB) k_persistent(FusedView<T> v0, 
 	for (int it = 0; it < a.iters; it++) {
 		for (int s = 0; s < a.stages; s++) {
 			const FusedView<T>& v = parity ? v1 : v0;
-			if (ORDER2 || s == 0) {
+			if (ORDER2) {
 				for (int w = blockIdx.x; w < a.n_work; w += gridDim.x) {
 					const int4 t = a.work[w];
-					for (int c = t.x + threadIdx.x; c < t.y; c += TPB) {
-						if (ORDER2) {
-							if (s == 0) recon_cell<T, GRAD, LIM, true, 4>(v, ph, a.carry, c);
-							else recon_cell<T, GRAD, LIM, false, 4>(v, ph, a.carry, c);
-						} else {
-							start_cell<T, 4>(v, ph, a.carry, c);
-						}
-					}
+					for (int c = t.x + threadIdx.x; c < t.y; c += TPB) recon_cell<T, GRAD, LIM, 4>(v, ph, c);
 				}
 				grid.sync();
 			}
@@ -1447,8 +1432,9 @@ __global__ void __launch_bounds__(TPB, 512 / TPB) k_persistent(FusedView<T> v0, 
 			for (int w = blockIdx.x; w < a.n_work; w += gridDim.x) {
 				const int4 t = a.work[w];
 				for (int c = t.x + threadIdx.x; c < t.y; c += TPB) {
-					if (a.beta[s] != 0.0) flux_update_cell<T, SCHEME, !ORDER2, 4, true>(v, ph, al, be, last, a.carry, c);
-					else flux_update_cell<T, SCHEME, !ORDER2, 4, false>(v, ph, al, be, last, a.carry, c);
+					if (s == 0) flux_update_cell<T, SCHEME, !ORDER2, 4, STAGE_FIRST>(v, ph, al, be, last, a.carry, c);
+					else if (a.beta[s] != 0.0) flux_update_cell<T, SCHEME, !ORDER2, 4, STAGE_DISS>(v, ph, al, be, last, a.carry, c);
+					else flux_update_cell<T, SCHEME, !ORDER2, 4, STAGE_NODISS>(v, ph, al, be, last, a.carry, c);
 				}
 			}
 			grid.sync();
@@ -1470,32 +1456,23 @@ __global__ void __launch_bounds__(TPB, 512 / TPB) k_persistent(FusedView<T> v0, 
 // list (one block of 128 threads per tile of at most 128 cells), captured in a
 // CUDA graph by the host.  Each pass keeps only its own registers and shared
 // memory, so more warps stay resident than in the persistent kernel.
-template <class T, int GRAD, int LIM, bool FIRST>
-__global__ void __launch_bounds__(128, sizeof(T) == 4 ? 8 : 4) k_recon_tiles(FusedView<T> v, Physics ph, int carry_w0,
+template <class T, int GRAD, int LIM>
+__global__ void __launch_bounds__(128, sizeof(T) == 4 ? 8 : 4) k_recon_tiles(FusedView<T> v, Physics ph,
                                                                              const int4* __restrict__ work) {
 	start_after_previous();
 	const int4 t = work[blockIdx.x];
 	const int c = t.x + threadIdx.x;
-	if (c < t.y) recon_cell<T, GRAD, LIM, FIRST, 4>(v, ph, carry_w0, c);
+	if (c < t.y) recon_cell<T, GRAD, LIM, 4>(v, ph, c);
 }
 
-template <class T>
-__global__ void __launch_bounds__(128) k_start_tiles(FusedView<T> v, Physics ph, int carry_w0,
-                                                     const int4* __restrict__ work) {
-	start_after_previous();
-	const int4 t = work[blockIdx.x];
-	const int c = t.x + threadIdx.x;
-	if (c < t.y) start_cell<T, 4>(v, ph, carry_w0, c);
-}
-
-template <class T, int SCHEME, bool ORDER1, bool DISS>
+template <class T, int SCHEME, bool ORDER1, int MODE>
 __global__ void __launch_bounds__(128, sizeof(T) == 4 ? 8 : 4) k_flux_update_tiles(FusedView<T> v, Physics ph, T alpha,
                                                                                    T beta, int last, int carry_w0,
                                                                                    const int4* __restrict__ work) {
 	start_after_previous();
 	const int4 t = work[blockIdx.x];
 	const int c = t.x + threadIdx.x;
-	if (c < t.y) flux_update_cell<T, SCHEME, ORDER1, 4, DISS>(v, ph, alpha, beta, last, carry_w0, c);
+	if (c < t.y) flux_update_cell<T, SCHEME, ORDER1, 4, MODE>(v, ph, alpha, beta, last, carry_w0, c);
 }
 
 }  // namespace

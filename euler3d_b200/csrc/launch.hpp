@@ -75,9 +75,7 @@ void end_iteration(const FusedView<T>& v, const ReduceArgs& r, int it, int iters
 
 // ---- fused stage kernels ----
 template <class T>
-void launch_recon(const FusedView<T>&, const Physics&, int grad, int lim, bool first, int carry, cudaStream_t);
-template <class T>
-void launch_start(const FusedView<T>&, const Physics&, int carry, cudaStream_t);
+void launch_recon(const FusedView<T>&, const Physics&, int grad, int lim, cudaStream_t);
 
 // batch launchers: threads per block; per namespace: resident blocks per SM of
 // the persistent kernel, its cooperative launch, and the tiled per-pass form.
@@ -122,7 +120,7 @@ void launch_rebase(const FusedView<float>& v, const Physics& ph, double* Wb, con
 }  // namespace delta
 
 template <class T>
-void launch_flux_update(const FusedView<T>&, const Physics&, int scheme, bool order1, double alpha, double beta,
-                        int last, int carry, cudaStream_t);
+void launch_flux_update(const FusedView<T>&, const Physics&, int scheme, bool order1, bool first, double alpha,
+                        double beta, int last, int carry, cudaStream_t);
 
 }  // namespace e3d

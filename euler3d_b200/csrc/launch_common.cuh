@@ -27,40 +27,24 @@ void launch_tail(const ReduceArgs& a, const T* Rc, const T* Rd, T* P, T* P2, cud
 	launch_next(k_tail<T>, grid, TAIL_TPB, 0, st, a, Rc, Rd, P, P2);
 }
 
-template <class T>
-void launch_start(const FusedView<T>& v, const Physics& ph, int carry, cudaStream_t st) {
-	if (v.NR <= 0) return;
-	if (v.tet4) launch_next(k_start<T, 4>, (v.NR + 127) / 128, 128, 0, st, v, ph, carry);
-	else launch_next(k_start<T, 0>, (v.NR + 127) / 128, 128, 0, st, v, ph, carry);
-}
-
 // Which pass reconstructs: see k_recon_var.
 template <class T, int GRAD, int LIM>
-void recon_dispatch_first(const FusedView<T>& v, const Physics& ph, bool first, int carry, cudaStream_t st) {
+void recon_pass(const FusedView<T>& v, const Physics& ph, cudaStream_t st) {
 	const int grid = (v.NR + 127) / 128, gv = (v.NR + RV_CELLS - 1) / RV_CELLS;
-	if (!v.tet4) {
-		if (first) launch_start<T>(v, ph, carry, st);
-		launch_next(k_recon_var<T, GRAD, LIM, 0>, gv, 5 * RV_CELLS, 0, st, v, ph);
-		return;
-	}
-	if (first) launch_next(k_recon<T, GRAD, LIM, true, 4>, grid, 128, 0, st, v, ph, carry);
+	if (!v.tet4) launch_next(k_recon_var<T, GRAD, LIM, 0>, gv, 5 * RV_CELLS, 0, st, v, ph);
 	else if constexpr (sizeof(T) == 8) launch_next(k_recon_var<T, GRAD, LIM, 4>, gv, 5 * RV_CELLS, 0, st, v, ph);
-	else launch_next(k_recon<T, GRAD, LIM, false, 4>, grid, 128, 0, st, v, ph, carry);
+	else launch_next(k_recon<T, GRAD, LIM, 4>, grid, 128, 0, st, v, ph);
 }
 
 template <class T>
-void launch_recon(const FusedView<T>& v, const Physics& ph, int grad, int lim, bool first, int carry, cudaStream_t st) {
+void launch_recon(const FusedView<T>& v, const Physics& ph, int grad, int lim, cudaStream_t st) {
 	if (v.NR <= 0) return;
 	if (grad == GRAD_LEAST_SQUARES) {
-		if (lim == LIM_VENKATAKRISHNAN)
-			recon_dispatch_first<T, GRAD_LEAST_SQUARES, LIM_VENKATAKRISHNAN>(v, ph, first, carry, st);
-		else
-			recon_dispatch_first<T, GRAD_LEAST_SQUARES, LIM_BARTH_JESPERSEN>(v, ph, first, carry, st);
+		if (lim == LIM_VENKATAKRISHNAN) recon_pass<T, GRAD_LEAST_SQUARES, LIM_VENKATAKRISHNAN>(v, ph, st);
+		else recon_pass<T, GRAD_LEAST_SQUARES, LIM_BARTH_JESPERSEN>(v, ph, st);
 	} else {
-		if (lim == LIM_VENKATAKRISHNAN)
-			recon_dispatch_first<T, GRAD_GREEN_GAUSS, LIM_VENKATAKRISHNAN>(v, ph, first, carry, st);
-		else
-			recon_dispatch_first<T, GRAD_GREEN_GAUSS, LIM_BARTH_JESPERSEN>(v, ph, first, carry, st);
+		if (lim == LIM_VENKATAKRISHNAN) recon_pass<T, GRAD_GREEN_GAUSS, LIM_VENKATAKRISHNAN>(v, ph, st);
+		else recon_pass<T, GRAD_GREEN_GAUSS, LIM_BARTH_JESPERSEN>(v, ph, st);
 	}
 }
 
@@ -75,8 +59,8 @@ void launch_recon(const FusedView<T>& v, const Physics& ph, int grad, int lim, b
 constexpr int slot_pass_cells(int scheme) { return scheme == FLUX_ROE ? 220000 : 80000; }
 
 template <class T>
-void launch_flux_update(const FusedView<T>& v, const Physics& ph, int scheme, bool order1, double alpha, double beta,
-                        int last, int carry, cudaStream_t st) {
+void launch_flux_update(const FusedView<T>& v, const Physics& ph, int scheme, bool order1, bool first, double alpha,
+                        double beta, int last, int carry, cudaStream_t st) {
 	if (v.NR <= 0) return;
 	const int grid = (v.NR + 127) / 128, g4 = (v.NR + 31) / 32, g8 = (v.NR + 15) / 16;
 	const bool slots = sizeof(T) == 8 && v.NR <= slot_pass_cells(scheme) / (v.tet4 ? 1 : 2);
@@ -94,8 +78,9 @@ void launch_flux_update(const FusedView<T>& v, const Physics& ph, int scheme, bo
 	} while (0)
 #define E3D_FLUX(S, O)                                                                                     \
 	do {                                                                                                   \
-		if (beta != 0.0) E3D_FLUX_D(S, O, true);                                                           \
-		else E3D_FLUX_D(S, O, false);                                                                      \
+		if (first) E3D_FLUX_D(S, O, STAGE_FIRST);                                                          \
+		else if (beta != 0.0) E3D_FLUX_D(S, O, STAGE_DISS);                                                \
+		else E3D_FLUX_D(S, O, STAGE_NODISS);                                                               \
 	} while (0)
 	if (scheme == FLUX_AUSM) {
 		if (order1) E3D_FLUX(FLUX_AUSM, true);
