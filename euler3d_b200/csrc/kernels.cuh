@@ -744,11 +744,8 @@ __global__ void __launch_bounds__(128, sizeof(T) == 4 ? E3D_RECON_MIN_BLOCKS : E
 // write one 32-byte vector together).  Measured on B200 (3.07M tets, FP64 second
 // order): 2.61 TB/s against 2.44 for the one-thread-per-cell pass.  With slot
 // counts known only at run time, one thread per cell kept its slot arrays in local
-// memory: 65k hexahedra FP64 40 us a launch, 25 here.
+// memory: 65k hexahedra FP64 40 us a launch, 23 here (7 resident blocks; 25 at 8).
 constexpr int RV_CELLS = 32;
-#ifndef E3D_RV_MIN_BLOCKS
-#define E3D_RV_MIN_BLOCKS 8
-#endif
 
 template <class T>
 __device__ __forceinline__ T ldq(const T* __restrict__ P, int n, int c, int q) {
@@ -761,7 +758,7 @@ __device__ __forceinline__ void stq(T* __restrict__ P, int n, int c, int q, T x)
 }
 
 template <class T, int GRAD, int LIM, int NSL>
-__global__ void __launch_bounds__(5 * RV_CELLS, E3D_RV_MIN_BLOCKS) k_recon_var(FusedView<T> v, Physics ph) {
+__global__ void __launch_bounds__(5 * RV_CELLS, NSL == 4 ? 8 : 7) k_recon_var(FusedView<T> v, Physics ph) {
 	const int c = blockIdx.x * RV_CELLS + threadIdx.x / 5, q = threadIdx.x % 5;
 	if (c >= v.NR) return start_after_previous();
 	const SlotRange<T, NSL> sr(v, c);
