@@ -252,15 +252,15 @@ __device__ __forceinline__ float limiter_venkat_face<float>(float d2, float dmax
 	const float A = fmaf(D, D, eps2);
 	return fmaf(2.0f * d2, D, A) / fmaf(d2, fmaf(2.0f, d2, D), A);
 }
+// The two signs of d2 share one copy of the expression: as branches, a warp with
+// both ran four divisions a face.
 template <>
 __device__ __forceinline__ double limiter_venkat_face<double>(double d2, double dmax, double dmin, double eps2) {
-	if (d2 > double(0.0))
-		return (double(1.0) / d2) * ((dmax * dmax + eps2) * d2 + double(2.0) * d2 * d2 * dmax) /
-		       (dmax * dmax + double(2.0) * d2 * d2 + dmax * d2 + eps2);
-	if (d2 < double(0.0))
-		return (double(1.0) / d2) * ((dmin * dmin + eps2) * d2 + double(2.0) * d2 * d2 * dmin) /
-		       (dmin * dmin + double(2.0) * d2 * d2 + dmin * d2 + eps2);
-	return double(1.0);
+	const bool pos = d2 > double(0.0), some = pos || d2 < double(0.0);
+	const double D = pos ? dmax : dmin, x = some ? d2 : double(1.0);
+	const double lf = (double(1.0) / x) * ((D * D + eps2) * x + double(2.0) * x * x * D) /
+	                  (D * D + double(2.0) * x * x + D * x + eps2);
+	return some ? lf : double(1.0);
 }
 
 // Slip wall / symmetry ghost state (WallCellIds.cpp:40-62, SymmetryCellIds.cpp:41-63).
