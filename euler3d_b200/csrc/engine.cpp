@@ -561,12 +561,9 @@ GeoView Engine::geo64() const {
 	g.slot_mate = slot_mate_.p;
 	g.sgeo = f64_.sgeo.p;
 	g.srv = f64_.srv.p;
-	g.face_lr = face_lr_.p;
 	g.S = S_.p;
 	g.nhat = nhat_.p;
 	g.area = area_.p;
-	g.rl = rl_.p;
-	g.rr = rr_.p;
 	g.vol = vol64_.p;
 	g.lsw = lsw64_.p;
 	g.gkind = gkind_.p;

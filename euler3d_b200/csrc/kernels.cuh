@@ -718,16 +718,12 @@ __device__ __forceinline__ void recon_cell(const FusedView<T>& v, const Physics&
 	}
 }
 
-// resident blocks per SM the FP32 reconstruction pass is compiled for (8: 64
-// registers) and the FP64 stage passes (4: 128 registers)
+// resident blocks per SM the FP32 reconstruction pass is compiled for (64 registers)
 #ifndef E3D_RECON_MIN_BLOCKS
 #define E3D_RECON_MIN_BLOCKS 8
 #endif
-#ifndef E3D_FP64_MIN_BLOCKS
-#define E3D_FP64_MIN_BLOCKS 4
-#endif
 template <class T, int GRAD, int LIM, int NSL>
-__global__ void __launch_bounds__(128, sizeof(T) == 4 ? E3D_RECON_MIN_BLOCKS : E3D_FP64_MIN_BLOCKS) k_recon(FusedView<T> v, Physics ph) {
+__global__ void __launch_bounds__(128, E3D_RECON_MIN_BLOCKS) k_recon(FusedView<T> v, Physics ph) {
 	start_after_previous();
 	const int c = blockIdx.x * blockDim.x + threadIdx.x;
 	if (c < v.NR) recon_cell<T, GRAD, LIM, NSL>(v, ph, c);

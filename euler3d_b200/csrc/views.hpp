@@ -34,12 +34,9 @@ struct GeoView {
 	const int* slot_mate;  // NS as in FusedView
 	const double* sgeo;    // 4*NS n, |S| of the slot's face (face orientation)
 	const double* srv;     // 3*NS r-vector of the slot's owner
-	const int* face_lr;    // 2*NF
 	const double* S;       // 3*NF area vector, left -> right
 	const double* nhat;    // 3*NF S/|S| as the reference normalises it
 	const double* area;    // NF
-	const double* rl;      // 3*NF
-	const double* rr;      // 3*NF
 	const double* vol;     // NA
 	const double* lsw;     // 3*NS (real-cell slots)
 	const signed char* gkind;  // NG boundary-condition kind of each ghost
