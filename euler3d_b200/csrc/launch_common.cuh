@@ -48,22 +48,25 @@ void launch_recon(const FusedView<T>& v, const Physics& ph, int grad, int lim, c
 	}
 }
 
-// Largest mesh (tetrahedra; half of it for 8 lanes per cell) whose FP64 flux
-// pass runs one lane per slot.  Below it a launch is latency: four times the
-// threads, each with a quarter of the chain.  Above it the exchange through shared
-// memory costs more than it hides.  B200, us a launch with dissipation, per cell /
-// per slot: Roe 3k 19 / 11, 48k 25 / 20, 132k 40 / 34, 216k 53 / 50 (second order
-// 57 / 55), 384k 80 / 88; AUSM 3k 16 / 10, 48k 18 / 16, 83k 20 / 21, 216k 33 / 39.
+// Largest mesh whose FP64 flux pass runs one lane per slot.  Below it a launch is
+// latency: four times the threads, each with a quarter of the chain.  Above it the
+// exchange through shared memory (and, on hexahedra, two idle lanes of eight) costs
+// more than it hides.  B200, us a launch with dissipation, per cell / per slot.
+// Tetrahedra: Roe 25k 22 / 15, 132k 40 / 34, 216k 54 / 52 (second order 57 / 58; without
+// dissipation 25 / 30), 384k 81 / 92; AUSM 25k 16.5 / 12.7, 83k 19.9 / 20.5, 132k 25 / 27.
+// Hexahedra: Roe 20k 26 / 19, 64k 32 / 36; AUSM 20k 20.5 / 16.2, 64k 23 / 29.
 // FP32 gains little (3k 10 / 8, 48k 10.5 / 10.6) and keeps one form, so that the
 // batch kernels and this path round alike.
-constexpr int slot_pass_cells(int scheme) { return scheme == FLUX_ROE ? 220000 : 80000; }
+constexpr int slot_pass_cells(int scheme, bool tet) {
+	return scheme == FLUX_ROE ? (tet ? 180000 : 40000) : (tet ? 60000 : 30000);
+}
 
 template <class T>
 void launch_flux_update(const FusedView<T>& v, const Physics& ph, int scheme, bool order1, bool first, double alpha,
                         double beta, int last, int carry, cudaStream_t st) {
 	if (v.NR <= 0) return;
 	const int grid = (v.NR + 127) / 128, g4 = (v.NR + 31) / 32, g8 = (v.NR + 15) / 16;
-	const bool slots = sizeof(T) == 8 && v.NR <= slot_pass_cells(scheme) / (v.tet4 ? 1 : 2);
+	const bool slots = sizeof(T) == 8 && v.NR <= slot_pass_cells(scheme, v.tet4);
 	const T a = T(alpha), b = T(beta);
 #define E3D_FLUX_D(S, O, D)                                                                                \
 	do {                                                                                                   \

@@ -11,10 +11,11 @@ from euler3d_b200 import meshgen as mg
 pytestmark = pytest.mark.gpu
 
 
-# tetrahedra: 80,000 cells (AUSM) and 220,000 (Roe); hexahedra: half of these; last blocks partly filled
+# one lane per slot up to 60,000 (AUSM) and 180,000 (Roe) tetrahedra, 30,000 and 40,000 hexahedra; last blocks partly filled
 @pytest.mark.parametrize("mesh,n,nz,flux,order", [
-    ("bump", 23, 1, "ausm", 2), ("bump", 24, 1, "ausm", 1), ("bump", 33, 1, "roe", 2), ("bump", 34, 1, "roe", 1),
-    ("hex", 20, 100, "ausm", 2), ("hex", 20, 101, "ausm", 2), ("hex", 3, 1, "roe", 2),
+    ("bump", 21, 1, "ausm", 2), ("bump", 22, 1, "ausm", 1), ("bump", 31, 1, "roe", 2), ("bump", 32, 1, "roe", 1),
+    ("hex", 20, 75, "ausm", 2), ("hex", 20, 76, "ausm", 2), ("hex", 20, 100, "roe", 1), ("hex", 20, 101, "roe", 2),
+    ("hex", 3, 1, "roe", 2),
 ])
 def test_matches_oracle(mesh, n, nz, flux, order, tmp_path):
     deck = mg.Deck(topology="", mach=0.7, aoa_deg=2.0, flux=flux, order=order)
