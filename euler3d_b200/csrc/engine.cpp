@@ -16,34 +16,6 @@
 namespace e3d {
 
 template <class T>
-void DevBuf<T>::alloc(size_t count) {
-	free();
-	n = count;
-	if (count) cuda_ok(cudaMalloc(&p, count * sizeof(T)), "cudaMalloc");
-}
-template <class T>
-void DevBuf<T>::upload(const std::vector<T>& h) {
-	alloc(h.size());
-	if (h.empty()) return;
-	cuda_ok(cudaMemcpy(p, h.data(), h.size() * sizeof(T), cudaMemcpyHostToDevice), "upload");
-	// a copy from pageable memory may return with its last staged part still on the way, and the
-	// solver's streams do not wait for the default stream
-	cuda_ok(cudaStreamSynchronize(nullptr), "upload");
-}
-template <class T>
-void DevBuf<T>::free() {
-	if (p) cudaFree(p);
-	p = nullptr;
-	n = 0;
-}
-template struct DevBuf<int>;
-template struct DevBuf<signed char>;
-template struct DevBuf<double>;
-template struct DevBuf<float>;
-template struct DevBuf<unsigned char>;
-template struct DevBuf<unsigned short>;
-
-template <class T>
 FusedView<T> Engine::Fused<T>::view(bool flip) const {
 	FusedView<T> v{};
 	v.Pin = flip ? P1.p : P0.p;
@@ -634,7 +606,7 @@ void Engine::smooth_residual(int block) {
 	require_fp64("smooth_residual");
 	int r0, r1, g0, g1;
 	block_range(block, r0, r1, g0, g1);
-	if (irs_.n < 10 * (size_t)NR_) irs_.alloc(10 * (size_t)NR_);
+	irs_.reserve(10 * (size_t)NR_);
 	launch_smooth(geo64(), state64(), irs_.p, r0, r1, st_);
 	check("smooth_residual");
 }
@@ -1161,7 +1133,7 @@ void Engine::get(const std::string& name, int b, double* dst, size_t count) {
 			pos_d_.upload(pos);
 		}
 		const size_t piece = std::min(total, kStageValues);
-		if (stage_.n < piece) stage_.alloc(piece);
+		stage_.reserve(piece);
 		for (size_t at = 0; at < total; at += piece) {
 			const size_t m = std::min(piece, total - at);
 			launch_state_out(layout, dev, layout == STATE_ROWS ? NR_ : NA_, n, r0, nr, g0, pos_d_.p + r0, at, m, stage_.p,
@@ -1407,10 +1379,12 @@ void Engine::build_work() {
 		bw[b + 1] = (int)work.size() / 4;
 	}
 	if (work == work_h_ && bw == block_work_h_) return;  // the list on the device, and a graph over it, stay
+	work_h_.clear();  // nothing is kept if the rest throws
+	block_work_h_.clear();
 	n_work_ = (int)work.size() / 4;
 	const size_t cap = 4 * ((size_t)NR_ / kPersistThreads + (size_t)nb_ + 1);
-	if (work_d_.n < cap) work_d_.alloc(cap);
-	if (wpart_d_.n < cap / 4 * 5) wpart_d_.alloc(cap / 4 * 5);
+	work_d_.reserve(cap);
+	wpart_d_.reserve(cap / 4 * 5);
 	if (!work.empty())
 		cuda_ok(cudaMemcpyAsync(work_d_.p, work.data(), work.size() * sizeof(int), cudaMemcpyHostToDevice, st_), "work");
 	block_work_d_.upload(bw);
@@ -1566,7 +1540,7 @@ void Engine::snapshot(bool save) {
 	const size_t ep = opt_.precision == PREC_FP32 ? sizeof(float) : sizeof(double);
 	const size_t np = (opt_.precision == PREC_FP32 ? f32_.P0.n : f64_.P0.n) * ep;
 	const size_t nw = W0_.n * sizeof(double);
-	if (snap_.n < 2 * np + nw + 16) snap_.alloc(2 * np + nw + 16);
+	snap_.reserve(2 * np + nw + 16);
 	void* p0 = opt_.precision == PREC_FP32 ? (void*)f32_.P0.p : (void*)f64_.P0.p;
 	void* p1 = opt_.precision == PREC_FP32 ? (void*)f32_.P1.p : (void*)f64_.P1.p;
 	unsigned char* b = snap_.p;

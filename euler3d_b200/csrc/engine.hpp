@@ -7,6 +7,7 @@
 #include <string>
 #include <vector>
 
+#include "devbuf.hpp"
 #include "launch.hpp"
 #include "mesh.hpp"
 
@@ -59,20 +60,6 @@ struct IterRecord {
 	double rms[5];          // mesh residual norms (sum of per-block norms)
 	double conv[5];         // log10(rms) - log10(rms at iteration 0)
 	double cl, cd, cmx, cmy, cmz;
-};
-
-inline void cuda_ok(cudaError_t e, const char* what) {
-	if (e != cudaSuccess) throw Error(E3D_ERR_CUDA, std::string(what) + ": " + cudaGetErrorString(e));
-}
-
-template <class T>
-struct DevBuf {
-	T* p = nullptr;
-	size_t n = 0;
-	void alloc(size_t count);
-	void upload(const std::vector<T>& h);
-	void free();
-	~DevBuf() { free(); }
 };
 
 class Engine {

@@ -692,13 +692,11 @@ void Surrogate::fit_normalisation() {
 }
 
 void Surrogate::ensure_work(int n) {
-	if (n <= work_n_) return;
-	work_n_ = n;
-	x_.alloc((size_t)n * S::IN);
-	for (auto* b : {&a1_, &a2_, &g1_, &g2_, &g3_}) b->alloc((size_t)n * H);
-	lossp_.alloc((size_t)sms_);
-	part_.alloc((size_t)sms_ * PA_N);
-	wpart_.alloc((size_t)kSlices * WG_N);
+	x_.reserve((size_t)n * S::IN);
+	for (auto* b : {&a1_, &a2_, &g1_, &g2_, &g3_}) b->reserve((size_t)n * H);
+	lossp_.reserve((size_t)sms_);
+	part_.reserve((size_t)sms_ * PA_N);
+	wpart_.reserve((size_t)kSlices * WG_N);
 }
 
 // Loss and gradient partials of n rows (part_, wpart_, lossp_); `grad`: gradient
@@ -744,7 +742,7 @@ double Surrogate::train(int steps, int batch, double lr, std::vector<float>* los
 	if (n_samples_ < 2) throw Error(E3D_ERR_STATE, "surrogate: no training samples");
 	if (!normalised_) fit_normalisation();
 	ensure_work(batch);
-	if (hist_.n < (size_t)steps) hist_.alloc((size_t)steps);
+	hist_.reserve((size_t)steps);
 	AdamStep ad{0.f, 0.9f, 0.999f, 1e-8f, 1.f, 1.f};
 	for (int s = 0; s < steps; s++) {
 		// cosine decay to 5% of lr over this call
@@ -828,10 +826,8 @@ void Surrogate::predict_host(const float* feat6, long long n, float* state5) {
 // allocated and freed on every call.
 int Surrogate::warm_start(Engine& e) {
 	const int nr = (int)e.n_real_total(), m = std::min(nr, kWarmRows);
-	if (warm_f_.n < (size_t)m * 8) {
-		warm_f_.alloc((size_t)m * 8);
-		warm_w_.alloc((size_t)m * 8);
-	}
+	warm_f_.reserve((size_t)m * 8);
+	warm_w_.reserve((size_t)m * 8);
 	e.clear_fallbacks();
 	for (int c0 = 0; c0 < nr; c0 += m) {
 		const int n = std::min(m, nr - c0);

@@ -67,7 +67,7 @@ private:
 	struct AdamStep {
 		float lr, b1, b2, eps, c1, c2;
 	};
-	// loss and gradient of n rows (n <= work_n_), then an Adam step if given
+	// loss and gradient of n rows (after ensure_work(n)), then an Adam step if given
 	void step_rows(int n, const float* feat, const float* state, long long n_store, const AdamStep* adam, double* loss);
 	void ensure_work(int n);
 	static constexpr int kSlices = 64;  // row slices of the weight gradients
@@ -85,7 +85,6 @@ private:
 	bool normalised_ = false;
 	long long step_ = 0;
 	// per-minibatch work buffers
-	int work_n_ = 0;
 	int sms_ = 1;
 	DevBuf<uint16_t> x_, a1_, a2_, g1_, g2_, g3_;
 	DevBuf<float> part_, wpart_, lossp_;
