@@ -77,7 +77,10 @@ __device__ __forceinline__ T qv(const Q5<T>& q, int v) { return (&q.r)[v]; }
 // Launched with programmatic serialization (launch_next): the next kernel's blocks
 // may take their places while this one's last blocks run, and every kernel waits
 // here for all memory of the one before it.  Only data that no kernel of an
-// iteration writes (topology, geometry) may be read before the wait.
+// iteration writes (topology, geometry) may be read before the wait, and only
+// pointers to such data may be `const __restrict__` parameters of the kernel: the
+// qualifiers promise constant data from the kernel's first instruction on, and allow
+// loads past the coherent path, while here the kernel before may still be writing.
 __device__ __forceinline__ void start_after_previous() {
 	cudaTriggerProgrammaticLaunchCompletion();
 	cudaGridDependencySynchronize();
@@ -391,7 +394,7 @@ __global__ void k_irs_start(GeoView g, StateView s, double* __restrict__ j1, int
 
 // Pass 2: R = (R + eps * sum of J1 over the real neighbours in slot order) / (1 + eps N),
 // in place (each thread reads only its own R and the neighbours' J1).
-__global__ void k_irs_smooth(GeoView g, StateView s, const double* __restrict__ j1, int r0, int r1) {
+__global__ void k_irs_smooth(GeoView g, StateView s, const double* j1, int r0, int r1) {
 	start_after_previous();
 	const int c = r0 + blockIdx.x * blockDim.x + threadIdx.x, q = blockIdx.y;
 	if (c >= r1) return;
@@ -1212,8 +1215,7 @@ __device__ __forceinline__ void wall_face_terms(double p0, double p1, double den
 // blocks), then wall faces, then halo entries, TAIL_TPB of each per block.  The
 // last block to finish moves *pend on, after every block has read it.
 template <class T>
-__global__ void __launch_bounds__(TAIL_TPB) k_tail(ReduceArgs a, const T* __restrict__ Rc, const T* __restrict__ Rd,
-                                                   T* __restrict__ P, T* __restrict__ P2) {
+__global__ void __launch_bounds__(TAIL_TPB) k_tail(ReduceArgs a, const T* Rc, const T* Rd, T* P, T* P2) {
 	start_after_previous();
 	const int t = threadIdx.x;
 	const int slot = *a.pend;
