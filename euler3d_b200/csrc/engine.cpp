@@ -367,10 +367,16 @@ void Engine::build_blocks(const std::vector<const HostBlock*>& blocks, const std
 	if (opt_.precision == PREC_FP64) slot_geometry(f64_);
 	else slot_geometry(f32_);
 	// reductions: chunks of TAIL_CHUNK cells, never straddling a block
-	max_chunks_ = 1;
-	for (int b = 0; b < nb_; b++)
-		max_chunks_ = std::max(max_chunks_, (roff_[b + 1] - roff_[b] + TAIL_CHUNK - 1) / TAIL_CHUNK);
-	partial_.alloc((size_t)TAIL_SLOTS * nb_ * max_chunks_ * 5);
+	std::vector<int> chunk, chunk_off(1, 0);
+	for (int b = 0; b < nb_; b++) {
+		for (int c = roff_[b]; c < roff_[b + 1]; c += TAIL_CHUNK)
+			chunk.insert(chunk.end(), {c, std::min(c + TAIL_CHUNK, roff_[b + 1]), b, 0});
+		chunk_off.push_back((int)chunk.size() / 4);
+	}
+	n_chunks_ = chunk_off[nb_];
+	chunk_d_.upload(chunk);
+	chunk_off_d_.upload(chunk_off);
+	partial_.alloc((size_t)TAIL_SLOTS * 5 * n_chunks_);
 	hist_d_.alloc(opt_.hist_capacity * (size_t)nb_ * 10);
 	fd_hist_.alloc((size_t)nb_ * 10);
 	wall_terms_.alloc(TAIL_SLOTS * 5 * std::max<size_t>(1, wall_face_.n));
@@ -469,7 +475,7 @@ void Engine::init_state() {
 void Engine::count_device_bytes() {
 	size_t bytes = 0;
 	for (auto* b : {&slot_ptr_, &slot_face_, &slot_nbr_, &slot_mate_, &face_lr_, &halo_dst_, &halo_src_, &wall_off_,
-	                &wall_face_, &roff_d_, &xsend_, &xrecv_})
+	                &wall_face_, &roff_d_, &chunk_d_, &chunk_off_d_, &xsend_, &xrecv_})
 		bytes += b->n * sizeof(int);
 	for (auto* b : {&S_, &nhat_, &area_, &rl_, &rr_, &fc_, &vol64_, &lsw64_, &W0_, &srad_, &grad_, &lim_, &partial_,
 	                &hist_d_, &wall_terms_})
@@ -633,8 +639,9 @@ ReduceArgs Engine::reduce_args(double* hist, int* d_iter, bool with_halo) const 
 	a.NR = NR_;
 	a.NA = NA_;
 	a.nblocks = nb_;
-	a.roff = roff_d_.p;
-	a.max_chunks = max_chunks_;
+	a.n_chunks = n_chunks_;
+	a.chunk = reinterpret_cast<const int4*>(chunk_d_.p);
+	a.chunk_off = chunk_off_d_.p;
 	a.partial = partial_.p;
 	a.wall_off = wall_off_.p;
 	a.wall_face = wall_face_.p;

@@ -266,7 +266,8 @@ private:
 	DevBuf<double> partial_, hist_d_, fd_hist_, wall_terms_;
 	DevBuf<int> iter_d_, bad_d_, zero_d_;
 	bool started_ = false;
-	int max_chunks_ = 0;
+	int n_chunks_ = 0;                  // norm chunks, TAIL_CHUNK cells of one block at most
+	DevBuf<int> chunk_d_, chunk_off_d_;  // (first cell, end, block, 0) of each; offsets per block
 	DevBuf<int> pend_d_;  // iterations in the tail ring, block counter of the running tail launch
 	int pend_ = 0;        // the same count on the host
 	ReduceArgs reduce_args(double* hist, int* d_iter, bool with_halo) const;

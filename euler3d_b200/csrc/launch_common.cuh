@@ -23,7 +23,7 @@ void launch_halo_unpack(int n, const int* dst, int NA, const T* buf, T* b0, T* b
 template <class T>
 void launch_tail(const ReduceArgs& a, const T* Rc, const T* Rd, T* P, T* P2, cudaStream_t st) {
 	const auto blocks = [](int n) { return (n + TAIL_TPB - 1) / TAIL_TPB; };
-	const int grid = a.nblocks * a.max_chunks + blocks(a.n_wall) + blocks(a.n_halo);
+	const int grid = a.n_chunks + blocks(a.n_wall) + blocks(a.n_halo);
 	launch_next(k_tail<T>, grid, TAIL_TPB, 0, st, a, Rc, Rd, P, P2);
 }
 

@@ -103,9 +103,10 @@ constexpr int TAIL_CHUNK = 1024;  // cells per norm chunk: 48 blocks at 48k cell
 constexpr int TAIL_SLOTS = 32;    // iterations the ring holds
 struct ReduceArgs {
 	int NR, NA, nblocks;
-	const int* roff;       // nblocks+1 real-cell offsets
-	int max_chunks;        // TAIL_CHUNK-cell chunks of the largest block
-	double* partial;       // TAIL_SLOTS*nblocks*5*max_chunks
+	int n_chunks;          // norm chunks of all blocks, one block after the other
+	const int4* chunk;     // first cell, end, block
+	const int* chunk_off;  // nblocks+1 chunk offsets
+	double* partial;       // TAIL_SLOTS*5*n_chunks
 	const int* wall_off;   // nblocks+1
 	const int* wall_face;
 	int n_wall;
