@@ -376,10 +376,11 @@ void Engine::build_blocks(const std::vector<const HostBlock*>& blocks, const std
 	n_chunks_ = chunk_off[nb_];
 	chunk_d_.upload(chunk);
 	chunk_off_d_.upload(chunk_off);
-	partial_.alloc((size_t)TAIL_SLOTS * 5 * n_chunks_);
+	tail_slots_ = tail_slots(n_chunks_, wall_face_.n, NR_, opt_.hist_capacity);
+	partial_.alloc((size_t)tail_slots_ * 5 * n_chunks_);
 	hist_d_.alloc(opt_.hist_capacity * (size_t)nb_ * 10);
 	fd_hist_.alloc((size_t)nb_ * 10);
-	wall_terms_.alloc(TAIL_SLOTS * 5 * std::max<size_t>(1, wall_face_.n));
+	wall_terms_.alloc((size_t)tail_slots_ * 5 * std::max<size_t>(1, wall_face_.n));
 	pend_d_.alloc(2);
 	cuda_ok(cudaMemset(pend_d_.p, 0, 2 * sizeof(int)), "memset");
 	iter_d_.alloc(1);
@@ -642,6 +643,7 @@ ReduceArgs Engine::reduce_args(double* hist, int* d_iter, bool with_halo) const 
 	a.n_chunks = n_chunks_;
 	a.chunk = reinterpret_cast<const int4*>(chunk_d_.p);
 	a.chunk_off = chunk_off_d_.p;
+	a.slots = tail_slots_;
 	a.partial = partial_.p;
 	a.wall_off = wall_off_.p;
 	a.wall_face = wall_face_.p;
@@ -766,11 +768,11 @@ int Engine::launches_per_iteration() const {
 	const int stages = (int)alpha_.size();
 	if (deck_.smoothing)  // W0, spectral radius, time step; per stage (grad, lim,) conv, diss, 2 smoothing, update, BC; tail
 		return 3 + stages * ((order_ == 2 ? 2 : 0) + 6) + 1;
-	return (order_ == 2 ? 2 * stages : stages) + 1 /*tail; its sums once per TAIL_SLOTS iterations*/;
+	return (order_ == 2 ? 2 * stages : stages) + 1 /*tail; its sums once per tail_slots_ iterations*/;
 }
 
 // Launches one outer iteration (its captured graph, or eagerly); the tail's
-// sums follow once per TAIL_SLOTS iterations and before the caller reads them.
+// sums follow once per tail_slots_ iterations and before the caller reads them.
 template <class T>
 void Engine::step(Fused<T>& f) {
 	if (opt_.use_graph) {
@@ -788,7 +790,7 @@ void Engine::step(Fused<T>& f) {
 		check("iteration");
 	}
 	cur_ ^= deck_.smoothing ? 0 : ((int)alpha_.size() & 1);
-	if (++pend_ == TAIL_SLOTS) flush_tail();
+	if (++pend_ == tail_slots_) flush_tail();
 }
 
 template <class T>

@@ -268,6 +268,7 @@ private:
 	bool started_ = false;
 	int n_chunks_ = 0;                  // norm chunks, TAIL_CHUNK cells of one block at most
 	DevBuf<int> chunk_d_, chunk_off_d_;  // (first cell, end, block, 0) of each; offsets per block
+	int tail_slots_ = TAIL_SLOTS;  // iterations the tail ring holds
 	DevBuf<int> pend_d_;  // iterations in the tail ring, block counter of the running tail launch
 	int pend_ = 0;        // the same count on the host
 	ReduceArgs reduce_args(double* hist, int* d_iter, bool with_halo) const;

@@ -1159,7 +1159,7 @@ __global__ void __launch_bounds__(128, 4)
 // pending iterations at once, one thread block per (iteration, mesh block).
 // The force sums keep the reference's wall-face order, a serial chain of FP64
 // adds (2.7k faces: 71 us per iteration as a kernel of its own); with up to
-// TAIL_SLOTS iterations pending the chains run side by side, and their time is
+// 32 iterations pending (tail_slots) the chains run side by side, and their time is
 // paid once per call instead of once per iteration.  Measured on B200 per
 // iteration, norms + forces + counter: 107 us before (304k cells, 2,738 wall
 // faces), 39 us at 1k cells.

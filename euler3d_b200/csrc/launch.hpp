@@ -69,8 +69,8 @@ void end_iteration(const FusedView<T>& v, const ReduceArgs& r, int it, int iters
 	a.rec = const_cast<float*>(v.rec_in);
 	a.rec2 = v.rec_out;
 	launch_tail<T>(a, v.Rc, v.Rd, const_cast<T*>(v.Pin), v.Pout, st);
-	const int in_ring = it % TAIL_SLOTS + 1;
-	if (in_ring == TAIL_SLOTS || it == iters - 1) launch_tail_sums(r, in_ring, true, st);
+	const int in_ring = it % r.slots + 1;
+	if (in_ring == r.slots || it == iters - 1) launch_tail_sums(r, in_ring, true, st);
 }
 
 // ---- fused stage kernels ----

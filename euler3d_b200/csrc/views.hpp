@@ -100,17 +100,30 @@ struct FusedView {
 // iterations into hist[(*d_iter + i)*stride + b*10 + (0..4 norms, 5..9 forces)].
 constexpr int TAIL_TPB = 256;     // threads per block of k_tail
 constexpr int TAIL_CHUNK = 1024;  // cells per norm chunk: 48 blocks at 48k cells, 3,000 at 3.07M
-constexpr int TAIL_SLOTS = 32;    // iterations the ring holds
+constexpr int TAIL_SLOTS = 32;    // iterations the ring holds at most
+// Iterations the ring of a solver holds.  One iteration's slot is 40 bytes a norm chunk
+// and wall face; 64 meshes with 230k wall faces would keep 0.3 GB in 32 of them.  The
+// ring stays within 8 bytes a cell or 16 MB, whichever is more: fewer iterations'
+// chains then run side by side, but so many faces come in many blocks, whose chains do
+// too (B200, 100 iterations of 64 meshes with 578 wall faces each, 10 slots / 32: FP32
+// 45.8 / 45.8 ms, FP64 120.2 / 119.8; 1,339 / 1,373 MB).
+inline int tail_slots(size_t n_chunks, size_t n_wall, size_t n_cells, size_t hist_capacity) {
+	const size_t slot = 5 * sizeof(double) * (n_chunks + n_wall), room = n_cells > (2u << 20) ? 8 * n_cells : 16u << 20;
+	size_t n = slot ? room / slot : TAIL_SLOTS;
+	n = n < hist_capacity ? n : hist_capacity;
+	return n < 1 ? 1 : n < TAIL_SLOTS ? (int)n : TAIL_SLOTS;
+}
 struct ReduceArgs {
 	int NR, NA, nblocks;
 	int n_chunks;          // norm chunks of all blocks, one block after the other
 	const int4* chunk;     // first cell, end, block
 	const int* chunk_off;  // nblocks+1 chunk offsets
-	double* partial;       // TAIL_SLOTS*5*n_chunks
+	int slots;             // iterations the ring holds
+	double* partial;       // slots*5*n_chunks
 	const int* wall_off;   // nblocks+1
 	const int* wall_face;
 	int n_wall;
-	double* wall_terms;    // TAIL_SLOTS*5*n_wall
+	double* wall_terms;    // slots*5*n_wall
 	const int* face_lr;
 	const double* S;
 	const double* fc;
