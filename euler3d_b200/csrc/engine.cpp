@@ -470,25 +470,20 @@ void Engine::init_state() {
 	}
 	cuda_ok(cudaStreamSynchronize(st_), "sync");
 	cur_ = 0;
-	count_device_bytes();
 }
 
-void Engine::count_device_bytes() {
-	size_t bytes = 0;
-	for (auto* b : {&slot_ptr_, &slot_face_, &slot_nbr_, &slot_mate_, &face_lr_, &halo_dst_, &halo_src_, &wall_off_,
-	                &wall_face_, &roff_d_, &chunk_d_, &chunk_off_d_, &xsend_, &xrecv_})
-		bytes += b->n * sizeof(int);
-	for (auto* b : {&S_, &nhat_, &area_, &rl_, &rr_, &fc_, &vol64_, &lsw64_, &W0_, &srad_, &grad_, &lim_, &partial_,
-	                &hist_d_, &wall_terms_})
-		bytes += b->n * sizeof(double);
-	for (auto* b : {&f64_.P0, &f64_.P1, &f64_.FS, &f64_.Rc, &f64_.Rd, &f64_.dt, &f64_.sgeo, &f64_.sS, &f64_.srv,
-	                &f64_.lsw, &f64_.vol})
-		bytes += b->n * sizeof(double);
-	for (auto* b : {&f32_.P0, &f32_.P1, &f32_.FS, &f32_.Rc, &f32_.Rd, &f32_.dt, &f32_.sgeo, &f32_.sS, &f32_.srv,
-	                &f32_.lsw, &f32_.vol, &Pb32_, &dW_, &Rb_, &rec_})
-		bytes += b->n * sizeof(float);
-	bytes += Pb64_.n * sizeof(double);
-	dev_bytes_ = bytes;
+size_t Engine::device_bytes() const {
+	const auto sum = [](auto... b) { return (0 + ... + (b->n * sizeof(*b->p))); };
+	const auto fused = [&](const auto& f) {
+		return sum(&f.P0, &f.P1, &f.FS, &f.Rc, &f.Rd, &f.dt, &f.sgeo, &f.sS, &f.srv, &f.lsw, &f.vol);
+	};
+	return fused(f64_) + fused(f32_) +
+	       sum(&slot_ptr_, &slot_face_, &slot_nbr_, &slot_mate_, &face_lr_, &halo_dst_, &halo_src_, &wall_off_, &wall_face_,
+	           &roff_d_, &gkind_, &grefl_, &S_, &nhat_, &area_, &rl_, &rr_, &fc_, &vol64_, &lsw64_, &xsend_, &xrecv_) +
+	       sum(&W0_, &srad_, &grad_, &lim_, &irs_, &Pb32_, &dW_, &Rb_, &rec_, &Pb64_, &snap_) +
+	       sum(&partial_, &hist_d_, &fd_hist_, &wall_terms_, &chunk_d_, &chunk_off_d_, &pend_d_, &iter_d_, &bad_d_, &zero_d_) +
+	       sum(&work_d_, &block_work_d_, &wpart_d_, &case_free_d_, &wall_denom_d_, &gcase_d_, &block_case_d_, &fallback_d_) +
+	       sum(&pos_d_, &stage_, &cen_d_, &case_ma_d_, &case_cluster_d_, &cluster_first_d_, &wall_centre_, &wall_box_);
 }
 
 void Engine::require_fp64(const char* what) const {
@@ -1842,7 +1837,6 @@ void Engine::widen_to_fp64() {
 	grid_ = 0;
 	tuning_ = Tuning{};
 	snap_.free();
-	count_device_bytes();
 }
 
 // ---------------------------------------------------------------- difference form
@@ -1933,7 +1927,6 @@ void Engine::enter_delta() {
 	tuning_.tile_cells = kPersistThreads;
 	tuning_.tiled = true;
 	snap_.free();
-	count_device_bytes();
 }
 
 // back to the plain FP32 form: fold the differences into the base and write the
@@ -1952,7 +1945,6 @@ void Engine::leave_delta() {
 	}
 	grid_ = 0;
 	tuning_ = Tuning{};
-	count_device_bytes();
 }
 
 }  // namespace e3d

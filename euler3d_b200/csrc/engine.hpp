@@ -177,7 +177,7 @@ public:
 	long long n_real_total() const { return NR_; }
 	int precision() const { return opt_.precision; }
 	cudaStream_t stream() const { return st_; }
-	size_t device_bytes() const { return dev_bytes_; }
+	size_t device_bytes() const;  // of all buffers held now, those made on first use included
 	// number of kernel launches one outer iteration issues
 	int launches_per_iteration() const;
 	const Deck& deck() const { return deck_; }
@@ -210,7 +210,6 @@ private:
 	void init_state();
 	template <class T>
 	void slot_geometry(Fused<T>& f);
-	void count_device_bytes();
 	void check(const char* what);
 	template <class T>
 	void iteration_body(Fused<T>& f, int parity, std::vector<cudaEvent_t>* marks);
@@ -320,7 +319,6 @@ private:
 	void rebase();
 	void leave_delta();
 	void require_not_delta(const char* what) const;
-	size_t dev_bytes_ = 0;
 };
 
 template <>

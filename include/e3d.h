@@ -133,6 +133,9 @@ int e3d_case_cell_order(const e3d_case* c, int block, int mode, int32_t* order, 
 int e3d_solver_create(const e3d_case* c, const e3d_options* opt, e3d_solver** out);
 int e3d_solver_free(e3d_solver* s);
 int e3d_solver_sync(e3d_solver* s);
+/* Device memory the solver holds now.  It grows when a call first needs a buffer
+ * that is then kept: reading state back (8 bytes a value of the largest array, 32 MB
+ * at most, and 4 a cell), cell features, batch solves. */
 int e3d_solver_device_bytes(const e3d_solver* s, int64_t* bytes);
 
 /* Strategy-level calls (FP64 solver only), one per reference method. */
