@@ -1425,7 +1425,6 @@ double Engine::run_persistent_t(int iters) {
 	a.carry = carry_;
 	a.iters = iters;
 	a.start_parity = cur_;
-	a.tile_mult = tile_mult_;
 	a.wpart = wpart_d_.p;
 	a.wall_off = wall_off_.p;
 	a.wall_face = wall_face_.p;

@@ -467,57 +467,36 @@ struct SlotRange {
 };
 constexpr int MAXSL = 6;  // hexahedra
 
-// 3 consecutive values per slot (r-vectors, LS weights, signed area vectors)
-template <class T, int NSL>
-__device__ __forceinline__ void load3(const T* __restrict__ a, const SlotRange<T, NSL>& r, T o[MAXSL][3]) {
-	if (NSL == 4 && sizeof(T) == 4) {
-		const float4* p = reinterpret_cast<const float4*>(a + 3 * (size_t)r.s0);
+// A tetrahedron's four slots from s0 on: 3 consecutive values each (r-vectors, LS
+// weights, signed area vectors), and one integer each
+template <class T>
+__device__ __forceinline__ void load3(const T* __restrict__ a, int s0, T o[4][3]) {
+	T f[12];
+	if constexpr (sizeof(T) == 4) {
+		const float4* p = reinterpret_cast<const float4*>(a + 3 * (size_t)s0);
 		const float4 x = __ldg(p), y = __ldg(p + 1), z = __ldg(p + 2);
-		const float f[12] = {x.x, x.y, x.z, x.w, y.x, y.y, y.z, y.w, z.x, z.y, z.z, z.w};
+		const float g[12] = {x.x, x.y, x.z, x.w, y.x, y.y, y.z, y.w, z.x, z.y, z.z, z.w};
 #pragma unroll
-		for (int k = 0; k < 4; k++)
-			for (int d = 0; d < 3; d++) o[k][d] = (T)f[3 * k + d];
-	} else if (NSL == 4) {
-		const double2* p = reinterpret_cast<const double2*>(a + 3 * (size_t)r.s0);
-		double f[12];
+		for (int i = 0; i < 12; i++) f[i] = g[i];
+	} else {
+		const double2* p = reinterpret_cast<const double2*>(a + 3 * (size_t)s0);
 #pragma unroll
 		for (int i = 0; i < 6; i++) {
 			const double2 t = __ldg(p + i);
 			f[2 * i] = t.x;
 			f[2 * i + 1] = t.y;
 		}
+	}
 #pragma unroll
-		for (int k = 0; k < 4; k++)
-			for (int d = 0; d < 3; d++) o[k][d] = (T)f[3 * k + d];
-	} else {
-		for (int k = 0; k < r.n; k++)
-			for (int d = 0; d < 3; d++) o[k][d] = a[3 * (size_t)(r.s0 + k) + d];
-	}
+	for (int k = 0; k < 4; k++)
+		for (int d = 0; d < 3; d++) o[k][d] = f[3 * k + d];
 }
-template <class T, int NSL>
-__device__ __forceinline__ void load_int(const int* __restrict__ a, const SlotRange<T, NSL>& r, int o[MAXSL]) {
-	if (NSL == 4) {
-		const int4 x = __ldg(reinterpret_cast<const int4*>(a + r.s0));
-		o[0] = x.x;
-		o[1] = x.y;
-		o[2] = x.z;
-		o[3] = x.w;
-	} else {
-		for (int k = 0; k < r.n; k++) o[k] = a[r.s0 + k];
-	}
-}
-// face normal + area of each slot (face orientation)
-template <class T, int NSL>
-__device__ __forceinline__ void load_geo(const T* __restrict__ a, const SlotRange<T, NSL>& r, T o[MAXSL][4]) {
-#pragma unroll
-	for (int k = 0; k < (NSL == 4 ? 4 : MAXSL); k++) {
-		if (NSL != 4 && k >= r.n) break;
-		const typename Vec4<T>::type t = ldv4(a + 4 * (size_t)(r.s0 + k));
-		o[k][0] = t.x;
-		o[k][1] = t.y;
-		o[k][2] = t.z;
-		o[k][3] = t.w;
-	}
+__device__ __forceinline__ void load_int(const int* __restrict__ a, int s0, int o[4]) {
+	const int4 x = __ldg(reinterpret_cast<const int4*>(a + s0));
+	o[0] = x.x;
+	o[1] = x.y;
+	o[2] = x.z;
+	o[3] = x.w;
 }
 
 #define E3D_SLOTS(k, r) for (int k = 0; k < (NSL == 4 ? 4 : MAXSL); k++) if (NSL == 4 || k < r.n)
@@ -596,22 +575,22 @@ __device__ __forceinline__ void ausm_face_sides(const AusmSide<T>& L, const Ausm
 	}
 }
 
-// Pass 1 of a stage, one thread per real cell: gradient, limiter and MUSCL
+// Pass 1 of a stage, one thread per real tetrahedron: gradient, limiter and MUSCL
 // face states of the cell and of its ghost cells.
-template <class T, int GRAD, int LIM, int NSL>
+template <class T, int GRAD, int LIM>
 __device__ __forceinline__ void recon_cell(const FusedView<T>& v, const Physics& ph, int c) {
-	const SlotRange<T, NSL> sr(v, c);
+	const int s0 = 4 * c;
 	const Q5<T> q0 = ld5(v.Pin, v.NA, c);
-	int nb[MAXSL];
-	load_int<T, NSL>(v.slot_nbr, sr, nb);
-	T w[MAXSL][3];
-	if (GRAD == GRAD_GREEN_GAUSS) load3<T, NSL>(v.sS, sr, w);
-	else load3<T, NSL>(v.lsw, sr, w);
+	int nb[4];
+	load_int(v.slot_nbr, s0, nb);
+	T w[4][3];
+	if (GRAD == GRAD_GREEN_GAUSS) load3(v.sS, s0, w);
+	else load3(v.lsw, s0, w);
 	T gr[5][3];
 	for (int q = 0; q < 5; q++) gr[q][0] = gr[q][1] = gr[q][2] = T(0.0);
 	Q5<T> mx = q0, mn = q0;
 #pragma unroll
-	E3D_SLOTS(k, sr) {
+	for (int k = 0; k < 4; k++) {
 		const Q5<T> qn = ld5(v.Pin, v.NA, nb[k]);
 		for (int q = 0; q < 5; q++) {
 			if (GRAD == GRAD_GREEN_GAUSS) {
@@ -634,10 +613,10 @@ __device__ __forceinline__ void recon_cell(const FusedView<T>& v, const Physics&
 	if (GRAD == GRAD_GREEN_GAUSS)
 		for (int d = 0; d < 3; d++)
 			for (int q = 0; q < 5; q++) gr[q][d] /= V;
-	T rv[MAXSL][3];
-	load3<T, NSL>(v.srv, sr, rv);
+	T rv[4][3];
+	load3(v.srv, s0, rv);
 	const T eps2 = T(ph.k3) * V;
-	if constexpr (sizeof(T) == 4 && NSL == 4) {
+	if constexpr (sizeof(T) == 4) {
 		// FP32: the face value q + phi (g.r) reuses the limiter's d2 = g.r
 		Q5<T> fs[4];
 		for (int q = 0; q < 5; q++) {
@@ -656,15 +635,15 @@ __device__ __forceinline__ void recon_cell(const FusedView<T>& v, const Physics&
 			for (int k = 0; k < 4; k++) qv(fs[k], q) = qv(q0, q) + phi * d2[k];
 		}
 #pragma unroll
-		for (int k = 0; k < 4; k++) st5(v.FS, v.NS, sr.s0 + k, fs[k]);
+		for (int k = 0; k < 4; k++) st5(v.FS, v.NS, s0 + k, fs[k]);
 	} else {
-		// FP64 (and the generic slot path): the reference's accumulation order
+		// FP64: the reference's accumulation order
 		T phi[5];
 		for (int q = 0; q < 5; q++) {
 			const T dmax = qv(mx, q) - qv(q0, q), dmin = qv(mn, q) - qv(q0, q);
 			CellLimiter<T, LIM> lim;
 #pragma unroll
-			E3D_SLOTS(k, sr) {
+			for (int k = 0; k < 4; k++) {
 				T d2 = T(0.0);
 				d2 += gr[q][0] * rv[k][0];
 				d2 += gr[q][1] * rv[k][1];
@@ -674,27 +653,27 @@ __device__ __forceinline__ void recon_cell(const FusedView<T>& v, const Physics&
 			phi[q] = lim.value(dmax, dmin);
 		}
 #pragma unroll
-		E3D_SLOTS(k, sr) {
+		for (int k = 0; k < 4; k++) {
 			Q5<T> fs;
 			for (int q = 0; q < 5; q++)
 				qv(fs, q) = recon(qv(q0, q), phi[q], gr[q][0], gr[q][1], gr[q][2], rv[k][0], rv[k][1], rv[k][2]);
-			st5(v.FS, v.NS, sr.s0 + k, fs);
+			st5(v.FS, v.NS, s0 + k, fs);
 		}
 	}
 	// ghost cells of this cell's boundary faces: gradient (reflected or zero),
 	// limiter (the ghost's only neighbour is c) and face state.  The slot neighbours
 	// are read again (a cache hit) rather than held through the pass, which takes
 	// the FP32 pass from 32-68 bytes of spills to none.
-	load_int<T, NSL>(v.slot_nbr, sr, nb);
+	load_int(v.slot_nbr, s0, nb);
 #pragma unroll
-	E3D_SLOTS(k, sr) {
+	for (int k = 0; k < 4; k++) {
 		if (nb[k] >= v.NR) {
 			const int g = nb[k];
-			int ms = v.slot_mate[sr.s0 + k];
+			int ms = v.slot_mate[s0 + k];
 			ms = ms >= 0 ? ms : ~ms;
 			const Q5<T> qg = ld5(v.Pin, v.NA, g);
-			const T nx = v.sgeo[4 * (size_t)(sr.s0 + k)], ny = v.sgeo[4 * (size_t)(sr.s0 + k) + 1],
-			        nz = v.sgeo[4 * (size_t)(sr.s0 + k) + 2];
+			const T nx = v.sgeo[4 * (size_t)(s0 + k)], ny = v.sgeo[4 * (size_t)(s0 + k) + 1],
+			        nz = v.sgeo[4 * (size_t)(s0 + k) + 2];
 			const T g0 = v.srv[3 * (size_t)ms], g1 = v.srv[3 * (size_t)ms + 1], g2 = v.srv[3 * (size_t)ms + 2];
 			const bool refl = v.grefl[g - v.NR] != 0;
 			const T eps2g = T(ph.k3) * v.vol[g];
@@ -725,11 +704,11 @@ __device__ __forceinline__ void recon_cell(const FusedView<T>& v, const Physics&
 #ifndef E3D_RECON_MIN_BLOCKS
 #define E3D_RECON_MIN_BLOCKS 8
 #endif
-template <class T, int GRAD, int LIM, int NSL>
-__global__ void __launch_bounds__(128, E3D_RECON_MIN_BLOCKS) k_recon(FusedView<T> v, Physics ph) {
+template <int GRAD, int LIM>
+__global__ void __launch_bounds__(128, E3D_RECON_MIN_BLOCKS) k_recon(FusedView<float> v, Physics ph) {
 	start_after_previous();
 	const int c = blockIdx.x * blockDim.x + threadIdx.x;
-	if (c < v.NR) recon_cell<T, GRAD, LIM, NSL>(v, ph, c);
+	if (c < v.NR) recon_cell<float, GRAD, LIM>(v, ph, c);
 }
 
 // Reconstruction with one lane per (cell, variable): FP64, and both precisions on
@@ -763,7 +742,7 @@ __global__ void __launch_bounds__(5 * RV_CELLS, NSL == 4 ? 8 : 7) k_recon_var(Fu
 	const SlotRange<T, NSL> sr(v, c);
 	int nb[MAXSL];
 	if (NSL == 4) {
-		load_int<T, NSL>(v.slot_nbr, sr, nb);
+		load_int(v.slot_nbr, sr.s0, nb);
 	} else {
 #pragma unroll
 		E3D_SLOTS(k, sr) nb[k] = __ldg(v.slot_nbr + sr.s0 + k);
@@ -1421,7 +1400,7 @@ __global__ void __launch_bounds__(TPB, 512 / TPB) k_persistent(FusedView<T> v0, 
 			if (ORDER2) {
 				for (int w = blockIdx.x; w < a.n_work; w += gridDim.x) {
 					const int4 t = a.work[w];
-					for (int c = t.x + threadIdx.x; c < t.y; c += TPB) recon_cell<T, GRAD, LIM, 4>(v, ph, c);
+					for (int c = t.x + threadIdx.x; c < t.y; c += TPB) recon_cell<T, GRAD, LIM>(v, ph, c);
 				}
 				grid.sync();
 			}
@@ -1460,7 +1439,7 @@ __global__ void __launch_bounds__(128, sizeof(T) == 4 ? 8 : 4) k_recon_tiles(Fus
 	start_after_previous();
 	const int4 t = work[blockIdx.x];
 	const int c = t.x + threadIdx.x;
-	if (c < t.y) recon_cell<T, GRAD, LIM, 4>(v, ph, c);
+	if (c < t.y) recon_cell<T, GRAD, LIM>(v, ph, c);
 }
 
 template <class T, int SCHEME, bool ORDER1, int MODE>

@@ -33,7 +33,7 @@ void recon_pass(const FusedView<T>& v, const Physics& ph, cudaStream_t st) {
 	const int grid = (v.NR + 127) / 128, gv = (v.NR + RV_CELLS - 1) / RV_CELLS;
 	if (!v.tet4) launch_next(k_recon_var<T, GRAD, LIM, 0>, gv, 5 * RV_CELLS, 0, st, v, ph);
 	else if constexpr (sizeof(T) == 8) launch_next(k_recon_var<T, GRAD, LIM, 4>, gv, 5 * RV_CELLS, 0, st, v, ph);
-	else launch_next(k_recon<T, GRAD, LIM, 4>, grid, 128, 0, st, v, ph);
+	else launch_next(k_recon<GRAD, LIM>, grid, 128, 0, st, v, ph);
 }
 
 template <class T>

@@ -155,7 +155,6 @@ struct PersistArgs {
 	int carry;
 	int iters;             // outer iterations in this launch
 	int start_parity;      // 0: state in P0 (view v0 reads it), 1: state in P1
-	int tile_mult;         // a work item covers tile_mult * blockDim cells
 	// reductions
 	double* wpart;         // n_work*5 per-tile sums of (Rc-Rd)^2
 	const int* wall_off;
