@@ -836,9 +836,11 @@ __global__ void __launch_bounds__(5 * RV_CELLS, NSL == 4 ? 8 : 7) k_recon_var(Fu
 // registers and 23 % resident warps, with instruction-cache misses from four
 // copies of the flux; one copy needs 96.  Neighbours of a tetrahedron follow
 // from the mate slot (real slot 4c+k, ghost g's only slot 4 NR + g), so
-// slot_nbr is not read, and beta = 1 drops Rd unread.  B200, us a launch with /
-// without dissipation: 663k tets FP64 Roe 136 / 100 -> 121 / 88; 3.07M FP32
-// Roe 184 / 147 -> 175 / 144 (FP32 keeps the loop unrolled: 178 / 156 rolled).
+// slot_nbr is not read, and beta = 1 drops Rd unread (a value that is not finite
+// included: 0 * NaN does not reach the new Rd).  B200, us a launch with / without
+// dissipation: 663k tets FP64 Roe 136 / 100 -> 121 / 88, and 152 / 102 -> 126 / 74
+// with the 32-byte accesses (second pair on another box); 3.07M FP32 Roe 184 / 147 ->
+// 175 / 144 (FP32 keeps the loop unrolled: 178 / 156 rolled).
 // FIRST (the first stage): W0 (unless carried) and the local time step
 // (Timestep.cpp:26-148) are formed here from the state the stage starts from,
 // with the normals the fluxes read anyway, instead of in a pass of their own or
@@ -965,7 +967,7 @@ __device__ __forceinline__ void flux_update_cell(const FusedView<T>& v, const Ph
 }
 
 // resident blocks per SM the FP64 flux pass is compiled for (5: 96 registers;
-// 663k tets, Roe: 121 us at 5, 128 at 6, 138 at 7)
+// 663k tets, Roe: 126 us at 5, 131 at 6, 136 at 7)
 #ifndef E3D_FLUX64_MIN_BLOCKS
 #define E3D_FLUX64_MIN_BLOCKS 5
 #endif
@@ -1139,9 +1141,10 @@ __global__ void __launch_bounds__(128, 4)
 // The force sums keep the reference's wall-face order, a serial chain of FP64
 // adds (2.7k faces: 71 us per iteration as a kernel of its own); with up to
 // 32 iterations pending (tail_slots) the chains run side by side, and their time is
-// paid once per call instead of once per iteration.  Measured on B200 per
-// iteration, norms + forces + counter: 107 us before (304k cells, 2,738 wall
-// faces), 39 us at 1k cells.
+// paid once per call instead of once per iteration.  B200, tail and sums of one
+// iteration back to back, as six kernels / these two: 1.3k cells 23.5 / 13.3 us, 48k
+// 47 / 19, 304k (2,738 wall faces) 85 / 30; the sums, most of it, are now shared by
+// the iterations of the ring.
 
 // Sum of n values in ascending order by one warp (every lane returns it): the
 // next 128 are in flight while 128 are added from shared memory.

@@ -302,7 +302,8 @@ int e3d_shard_push_flow_data(e3d_solver* s, const double* all_blocks, int n_iter
  * of a solver; cells whose prediction is not physical keep the freestream
  * start (*n_fallback counts them).  Call it after one iteration from the
  * freestream start so the residual drop is measured from the same reference
- * norm as a plain start's. */
+ * norm as a plain start's.  It runs 2^20 cells at a time through two buffers that
+ * the surrogate keeps (64 bytes a cell, 64 MB at most). */
 int e3d_solver_set_precision(e3d_solver* s, int precision);
 int e3d_cell_features(e3d_solver* s, float* out, int64_t n_floats);
 
