@@ -1122,7 +1122,6 @@ void Engine::to_device(int b, std::vector<double>& a, int rows, int ld) const {
 // twice the solver time of ten iterations.
 void Engine::get(const std::string& name, int b, double* dst, size_t count) {
 	if (b < 0 || b >= nb_) throw Error(E3D_ERR_ARG, "block index out of range");
-	cuda_ok(cudaStreamSynchronize(st_), "sync");
 	const int nr = n_real_b_[b], na = n_all_b_[b], r0 = roff_[b], g0 = NR_ + goff_[b];
 	const bool f64 = opt_.precision == PREC_FP64;
 	const auto bring = [&](StateLayout layout, int rows, auto* dev) {
